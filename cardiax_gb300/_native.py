@@ -78,6 +78,11 @@ _SIGNATURES = {
     "fk_forward_euler_tracked": [Grid, _P, _P, _P, ctypes.POINTER(Params),
                                  ctypes.POINTER(Stimulus), _INT, _I64, _I64, _D, _D,
                                  ctypes.POINTER(Activation), _P],
+    "fk_forward_euler_resident": [Grid, _P, _P, _P, ctypes.POINTER(Params),
+                                  ctypes.POINTER(Stimulus), _INT, _I64, _I64, _D, _D,
+                                  ctypes.POINTER(Activation), _P, ctypes.c_size_t, _P],
+    "fk_forward_resident": [Grid, _P, _P, _P, ctypes.POINTER(Params), ctypes.POINTER(Stimulus),
+                            _INT, ctypes.POINTER(_I64), _INT, _D, _D, _P, _P, ctypes.c_size_t, _P],
     "fk_forward_euler_flow": [Grid, _P, _P, _P, _P, ctypes.POINTER(Params),
                               ctypes.POINTER(Stimulus), _INT, _I64, _I64, _D, _D,
                               ctypes.POINTER(Activation), _P, _I64, _P],
@@ -125,6 +130,8 @@ def lib(build: bool = True):
                 fn.argtypes = args
             L.fk_batch_workspace_bytes.restype = ctypes.c_size_t
             L.fk_batch_workspace_bytes.argtypes = [ctypes.POINTER(TissueDesc), _INT]
+            L.fk_resident_workspace_bytes.restype = ctypes.c_size_t
+            L.fk_resident_workspace_bytes.argtypes = [Grid]
             L.fk_flow_flag_words.restype = _I64
             L.fk_flow_flag_words.argtypes = [Grid]
             _lib = L
@@ -138,5 +145,6 @@ def call(name: str, *args) -> None:
 
 
 def exported_symbols():
-    return (["fk_status_string", "fk_batch_workspace_bytes", "fk_flow_flag_words"]
+    return (["fk_status_string", "fk_batch_workspace_bytes", "fk_flow_flag_words",
+             "fk_resident_workspace_bytes"]
             + list(_SIGNATURES))

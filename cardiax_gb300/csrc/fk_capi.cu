@@ -11,6 +11,8 @@
 //   fk_forward_heun   cardiax/solve.py:103-111 _forward_heun
 //   fk_forward_euler_flow, fk_forward_flow   _forward_euler / forward through the dataflow
 //                     kernel (one cooperative launch per call instead of one per step)
+//   fk_forward_euler_resident, fk_forward_resident   _forward_euler / forward with the state held
+//                     on chip over many steps of one launch (fk_resident.cu)
 //   fk_forward_euler_tb   _forward_euler with `depth` steps per launch (temporal blocking)
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -20,12 +22,14 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "../../include/cardiax_gb300.h"
 #include "fk_capi_internal.h"
 #include "fk_ptx.cuh"
 #include "fk_adjoint.cuh"
+#include "fk_resident.cuh"
 #include "fk_step.cuh"
 #include "fk_strip.cuh"
 #include "fk_tb.cuh"
@@ -426,6 +430,67 @@ int flow_run(const fk_grid &g, const float *src, float *dst, float *scratch, con
     return FK_OK;
 }
 
+// ---- resident stepping --------------------------------------------------------------------------
+// Calls of fewer steps take one launch per step.  The resident kernel's fixed cost (clearing the
+// strips, loading the state, the cooperative launch) is 13 us at 64^2 and 30 at 1200^2, against
+// 4.4 and 9.7 us per single-step launch: at 6 steps 26.7 against 33.9 us (64^2), 31.0 against 32.8
+// (512^2), 76.9 against 82.5 (1200^2).
+constexpr int64_t kResidentMinSteps = 6;
+
+// Steps t0 .. t0+n-1 of `n_exp` tissues from `in` through the resident kernel, states written to
+// `base` + offset after the steps listed in `outs` ((step, offset) pairs in step order, the last one
+// at step n), or with `every` after each step s to base + s * every.  `exps`: see launch_resident;
+// `tmp` (one state) holds the state between launches that end at no listed step (one tissue only).
+static int resident_run(const ResPlan &plan, const fk_grid &g, const float *in, float *base,
+                        const std::vector<std::pair<int64_t, int64_t>> &outs, int64_t every,
+                        float *tmp, const float *D, const Model &m, const Stim *st, int ns,
+                        int64_t t0, int64_t n, float dt, float rdx, const fk_activation *act,
+                        const StepArgs *exps, void *workspace, int *status, cudaStream_t s) {
+    StepArgs a;
+    ResidentArgs ra{};
+    ra.nr = plan.nr;
+    ra.nc = plan.nc;
+    ra.ng = plan.ng;
+    ra.nq = plan.nq;
+    ra.max_q = plan.max_q;
+    ra.max_g = plan.max_g;
+    ra.su_w = plan.su_w;
+    ra.su_h = plan.su_h;
+    ra.slot = plan.slot;
+    ra.xchg = static_cast<uint64_t *>(workspace);
+    ra.every = every;
+    size_t k = 0;
+    for (int64_t done = 0; done < n;) {
+        int64_t c = n - done < kResMaxSteps ? n - done : kResMaxSteps;
+        fill_args(a, g, in, D, m, st, ns, dt, rdx, status, act);
+        a.vo = base;
+        ra.t0 = t0 + done;
+        ra.n_out = 0;
+        if (!every) {
+            for (; k < outs.size() && outs[k].first <= done + c; ++k) {
+                if (ra.n_out == kResMaxOut - 1) {  // the rest in the next launch
+                    c = ra.out_step[ra.n_out - 1];
+                    break;
+                }
+                ra.out_step[ra.n_out] = (int)(outs[k].first - done);
+                ra.out_off[ra.n_out++] = outs[k].second;
+                in = base + outs[k].second;
+            }
+            if (ra.n_out == 0 || ra.out_step[ra.n_out - 1] != c) {
+                ra.out_step[ra.n_out] = (int)c;
+                ra.out_off[ra.n_out++] = tmp - base;
+                in = tmp;
+            }
+        }
+        ra.n = (int)c;
+        if (cudaMemsetAsync(workspace, 0, plan.workspace(), s) != cudaSuccess ||
+            launch_resident(plan, ra, a, exps, s) != cudaSuccess)
+            return FK_ERR_CUDA;
+        done += c;
+    }
+    return FK_OK;
+}
+
 __global__ void add_state_kernel(float *dst, const float *src, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -592,6 +657,48 @@ int fk_forward_euler_tracked(fk_grid g, float *state, float *scratch, const floa
             return FK_ERR_CUDA;
     }
     return FK_OK;
+}
+
+size_t fk_resident_workspace_bytes(fk_grid g) {
+    if (check_grid(g)) return 0;
+    const ResPlan plan = resident_plan(g.H, g.W, 1);
+    return plan.ok() ? plan.workspace() : 0;
+}
+
+// Whether a call of n steps takes the resident kernel; `plan` is filled in then.
+static bool takes_resident(const fk_grid &g, int64_t n, int n_stimuli, const void *workspace,
+                           size_t bytes, ResPlan &plan) {
+    if (!workspace || n < kResidentMinSteps || n_stimuli > kMaxStim || g_step_kernel != 0 ||
+        !aligned16(workspace))
+        return false;
+    plan = resident_plan(g.H, g.W, 1);
+    return plan.ok() && bytes >= plan.workspace();
+}
+
+int fk_forward_euler_resident(fk_grid g, float *state, float *scratch, const float *D,
+                              const fk_params *p, const fk_stimulus *stimuli, int n_stimuli,
+                              int64_t t0, int64_t t1, double dt, double dx,
+                              const fk_activation *act, void *workspace, size_t workspace_bytes,
+                              void *stream) {
+    int rc = common_checks(g, state, scratch, D, p, dx);
+    if (rc) return rc;
+    if (t1 < t0 || !std::isfinite(dt)) return FK_ERR_ARGUMENT;
+    ResPlan plan;
+    if (!takes_resident(g, t1 - t0, n_stimuli, workspace, workspace_bytes, plan))
+        return fk_forward_euler_tracked(g, state, scratch, D, p, stimuli, n_stimuli, t0, t1, dt, dx,
+                                        act, stream);
+    if (act) {
+        if (!act->first || !act->last || !act->count) return FK_ERR_NULL;
+        if (!std::isfinite(act->threshold)) return FK_ERR_ARGUMENT;
+    }
+    Stim st[kMaxStim];
+    if ((rc = make_stims(stimuli, n_stimuli, g, st))) return rc;
+    int *status = status_ptr();
+    if (!status) return FK_ERR_CUDA;
+    const int64_t n = t1 - t0;
+    return resident_run(plan, g, state, state, {{n, 0}}, 0, scratch, D, make_model(*p), st,
+                        n_stimuli, t0, n, (float)dt, 1.0f / (float)dx, act, nullptr, workspace,
+                        status, (cudaStream_t)stream);
 }
 
 int64_t fk_flow_flag_words(fk_grid g) {
@@ -847,6 +954,48 @@ int fk_forward(fk_grid g, const float *state0, float *scratch, const float *D,
             if (rc) return rc;
             cur = o;
         }
+        cur = dst;
+    }
+    return FK_OK;
+}
+
+int fk_forward_resident(fk_grid g, const float *state0, float *scratch, const float *D,
+                        const fk_params *p, const fk_stimulus *stimuli, int n_stimuli,
+                        const int64_t *checkpoints, int n_checkpoints, double dt, double dx,
+                        float *out, void *workspace, size_t workspace_bytes, void *stream) {
+    int rc = common_checks(g, state0, scratch, D, p, dx);
+    if (rc) return rc;
+    if (!out || !checkpoints) return FK_ERR_NULL;
+    if (!aligned16(out)) return FK_ERR_ALIGN;
+    if (n_checkpoints < 1 || !std::isfinite(dt)) return FK_ERR_ARGUMENT;
+    for (int i = 0; i + 1 < n_checkpoints; ++i)
+        if (checkpoints[i + 1] < checkpoints[i]) return FK_ERR_ARGUMENT;
+    const int64_t t0 = checkpoints[0], n = checkpoints[n_checkpoints - 1] - t0;
+    ResPlan plan;
+    if (!takes_resident(g, n, n_stimuli, workspace, workspace_bytes, plan))
+        return fk_forward(g, state0, scratch, D, p, stimuli, n_stimuli, checkpoints, n_checkpoints,
+                          dt, dx, out, stream);
+    Stim st[kMaxStim];
+    if ((rc = make_stims(stimuli, n_stimuli, g, st))) return rc;
+    int *status = status_ptr();
+    if (!status) return FK_ERR_CUDA;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int64_t n_state = 3 * g.H * g.pitch;
+    std::vector<std::pair<int64_t, int64_t>> outs;
+    for (int i = 0; i + 1 < n_checkpoints; ++i)
+        if (checkpoints[i + 1] > checkpoints[i])
+            outs.push_back({checkpoints[i + 1] - t0, i * n_state});
+    if ((rc = resident_run(plan, g, state0, out, outs, 0, scratch, D, make_model(*p), st, n_stimuli,
+                           t0, n, (float)dt, 1.0f / (float)dx, nullptr, nullptr, workspace, status,
+                           s)))
+        return rc;
+    const float *cur = state0;
+    for (int i = 0; i + 1 < n_checkpoints; ++i) {  // intervals of no steps repeat the state before
+        float *dst = out + i * n_state;
+        if (checkpoints[i + 1] == checkpoints[i] &&
+            cudaMemcpyAsync(dst, cur, sizeof(float) * n_state, cudaMemcpyDeviceToDevice, s) !=
+                cudaSuccess)
+            return FK_ERR_CUDA;
         cur = dst;
     }
     return FK_OK;

@@ -136,6 +136,7 @@ class Tissue:
             self.state = torch.empty((3, H, self.pitch), dtype=torch.float32, device=self.device)
             self.scratch = torch.empty_like(self.state)
         self.activation = None
+        self._resident = None  # the resident stepper's exchange buffer
         self._batches = {}  # one-tissue batch plans by tile rows (schedule="batch")
         self.init()
 
@@ -188,6 +189,15 @@ class Tissue:
             self._flags = torch.zeros(n, dtype=torch.int32, device=self.device)
         return self._flags
 
+    def _resident_workspace(self):
+        """(pointer, bytes) of the resident stepper's exchange buffer, (None, 0) on a grid that it
+        does not take (owned by this tissue; its calls are ordered on one stream)."""
+        if self._resident is None:
+            n = int(N.lib().fk_resident_workspace_bytes(self.grid))
+            self._resident = torch.empty(n, dtype=torch.uint8, device=self.device)
+        n = self._resident.numel()
+        return (self._resident.data_ptr() if n else None), n
+
     def _one_batch(self, tile_rows: int):
         """A batch plan holding this tissue alone, with ``tile_rows`` x 64 work items (kept
         until activation tracking changes)."""
@@ -200,9 +210,11 @@ class Tissue:
 
     def advance(self, t0: int, t1: int, schedule: str = "step", depth: int = 1,
                 tile_rows: int = 16) -> "Tissue":
-        """Steps t0 .. t1-1 in place (cardiax/solve.py:92-100).  ``schedule="step"``: one launch
-        per step (chained with programmatic dependent launch), or with ``depth`` 2, 4 or 8 that
-        many steps per launch (temporal blocking); ``"flow"``: one cooperative dataflow launch
+        """Steps t0 .. t1-1 in place (cardiax/solve.py:92-100).  ``schedule="step"``: grids that
+        fit on chip (16 x 16 up to about 1240 x 1240) run in one launch with the state held there
+        (calls of a few steps excepted), others one launch per step (chained with programmatic
+        dependent launch); with ``depth`` 2, 4 or 8 that many steps per launch (temporal
+        blocking); ``"flow"``: one cooperative dataflow launch
         for the whole range; ``"batch"``: the batched kernel on this tissue alone, with
         ``tile_rows`` x 64 work items (16-row items put twice the CTAs on a small grid and
         shorten each step's critical path) and CUDA-graph replay; ``"auto"``: whichever of these
@@ -229,9 +241,10 @@ class Tissue:
                    stream_handle())
             return self
         if schedule == "step":
-            N.call("fk_forward_euler_tracked", self.grid, self.state.data_ptr(),
+            ws, ws_bytes = self._resident_workspace()
+            N.call("fk_forward_euler_resident", self.grid, self.state.data_ptr(),
                    self.scratch.data_ptr(), self.D.data_ptr(), ctypes.byref(self.params),
-                   self.stim, self.n_stim, int(t0), int(t1), self.dt, self.dx, act,
+                   self.stim, self.n_stim, int(t0), int(t1), self.dt, self.dx, act, ws, ws_bytes,
                    stream_handle())
             return self
         if schedule != "flow":
@@ -267,9 +280,11 @@ class Tissue:
             return out
         arr = (ctypes.c_int64 * len(ck))(*ck)
         if schedule == "step" or self.n_stim > N.FK_MAX_ACTIVE_STIMULI:
-            N.call("fk_forward", self.grid, self.state.data_ptr(), self.scratch.data_ptr(),
-                   self.D.data_ptr(), ctypes.byref(self.params), self.stim, self.n_stim, arr,
-                   len(ck), self.dt, self.dx, out.data_ptr(), stream_handle())
+            ws, ws_bytes = self._resident_workspace()
+            N.call("fk_forward_resident", self.grid, self.state.data_ptr(),
+                   self.scratch.data_ptr(), self.D.data_ptr(), ctypes.byref(self.params),
+                   self.stim, self.n_stim, arr, len(ck), self.dt, self.dx, out.data_ptr(), ws,
+                   ws_bytes, stream_handle())
             return out
         if schedule != "flow":
             raise ValueError(f"unknown schedule {schedule!r}")

@@ -169,6 +169,24 @@ int fk_forward_euler_tracked(fk_grid g, float *state, float *scratch, const floa
                              int64_t t0, int64_t t1, double dt, double dx,
                              const fk_activation *act, void *stream);
 
+/* Resident stepping: fk_forward_euler_tracked and fk_forward with the whole state held on chip
+ * over many steps of one cooperative launch (no reference counterpart; same results bit for bit).
+ * `workspace` is a 16-byte aligned device buffer of fk_resident_workspace_bytes(g) bytes owned by
+ * the call (cleared by the call on `stream`; calls that overlap on the GPU need separate buffers).
+ * A grid too large or too small for the current device (workspace size 0), a call of few steps or
+ * with more than FK_MAX_ACTIVE_STIMULI stimuli, and a NULL or smaller workspace run one step per
+ * launch as the plain entry points do. */
+size_t fk_resident_workspace_bytes(fk_grid g);
+int fk_forward_euler_resident(fk_grid g, float *state, float *scratch, const float *D,
+                              const fk_params *p, const fk_stimulus *stimuli, int n_stimuli,
+                              int64_t t0, int64_t t1, double dt, double dx,
+                              const fk_activation *act, void *workspace, size_t workspace_bytes,
+                              void *stream);
+int fk_forward_resident(fk_grid g, const float *state0, float *scratch, const float *D,
+                        const fk_params *p, const fk_stimulus *stimuli, int n_stimuli,
+                        const int64_t *checkpoints, int n_checkpoints, double dt, double dx,
+                        float *out, void *workspace, size_t workspace_bytes, void *stream);
+
 /* Temporal blocking (no reference counterpart; same results bit for bit): fk_forward_euler with
  * `depth` steps (1, 2, 4 or 8) per launch.  Each tile is loaded once with a 4*depth-cell halo,
  * advanced `depth` times in shared memory (recomputing the halo ring) and stored once; the last
