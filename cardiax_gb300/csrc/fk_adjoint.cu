@@ -24,6 +24,7 @@
 
 #include "fk_adjoint.cuh"
 #include "fk_math.cuh"
+#include "fk_ptx.cuh"
 
 namespace fk {
 
@@ -529,16 +530,513 @@ __global__ void __launch_bounds__(ANT, 4) fk_adjoint_kernel(const __grid_constan
     adjoint_tile(a, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
-// One reverse step of many experiments (blockIdx.z): exps[e] describes step 0 of experiment e's
-// segment with the cotangent ping-pong buffers (lu.. = buffer A, olu.. = buffer B); step k reads
-// the state k * k_stride further on, and parity 1 swaps the two cotangent buffers.
-__global__ void __launch_bounds__(ANT, 4) fk_adjoint_batch_kernel(const AdjointArgs *__restrict__ exps,
-                                                               int64_t k_stride, int k, int parity,
-                                                               float t) {
-    __shared__ __align__(16) AdjointArgs sa;
+// ---- lines of at least kLineMin cells: two threads per unit of two rows of a quad, one stage -------
+// What bounds it: the tile kernel above stages six derivative planes, reads ten-cell products for
+// each cell of the 6-cell edge band, tests every stimulus's protocol in every cell and reduces 13
+// parameter sums over a warp for every two cells (us per step: 39.5 for 16 experiments of 256^2,
+// 10.9 for one 151 x 203 grid, 10.5 for 16 of 64^2).  Here everything comes from one staged tile of
+// u, D and lambda_u and stays in registers: 28.6, 7.1 and 7.9 us.  At 16 x 256^2 a step executes 400
+// instructions per cell at 42 % of the issue slots; one small grid waits for its loads (0.5 us),
+// then for the longest chain of a unit, 2500 cycles for each half of it.  The operations are fewer
+// because they are regrouped:
+//   * both transposed products of an axis share their second operator,
+//       A^T (D mu) + B^T ((B D) mu) = (E^T G^T / dx) (G^T C^T (D mu) / dx + C^T (B D) mu),
+//   * G^T on central rows is -G; the one-sided rows 0 and N-1 (and the pad rows -1 and N in the
+//     second operator) are taken out of the central sum and added as rank-one terms to the four
+//     cells they reach, only by the warps that hold such cells,
+//   * 1/dx^2, dt and the constant factors of the parameter sums are applied once, to the sums, and a
+//     parameter sum is reduced over a warp once per 8 cells.
+constexpr int kLineMin = 20;  // shorter lines (fewer than three quads or nine rows in a last tile)
+                              // take the tile kernel above
+constexpr int LR = 2;         // rows per thread
+constexpr int LG = 8, LQ = 16;                   // most row groups and quads of a tile
+constexpr int LU = LG * LQ;                      // units of a tile; two threads share one
+constexpr int LNT = 2 * LU;
+constexpr int LSW = 4 * LQ + 12;                 // staged row: 4 cells on either side, and 4 more so
+                                                 // that 8 lanes (2 quads of 4 groups) read from 8
+                                                 // different 16-byte banks
+constexpr int LSH = LG * LR + 8 + 1;             // 4 rows above and below; the first group of the
+                                                 // last tile row may reach one row further up
+
+__constant__ float kHeadC[4] = {C_HEAD0, C_THREE, -C_3_2, C_1_3};
+__constant__ float kTailC[4] = {C_TAIL0, C_3_2, -C_THREE, C_TAIL3};
+
+struct V4 {
+    float x, y, z, w;
+};
+__device__ __forceinline__ V4 ld_v4(const float *p) {
+    const float4 v = *reinterpret_cast<const float4 *>(p);
+    return V4{v.x, v.y, v.z, v.w};
+}
+__device__ __forceinline__ V4 vmul(V4 a, V4 b) { return V4{a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w}; }
+__device__ __forceinline__ V4 vscale(float c, V4 a) { return V4{c * a.x, c * a.y, c * a.z, c * a.w}; }
+__device__ __forceinline__ V4 vfma(V4 a, V4 b, V4 c) {
+    return V4{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z), fmaf(a.w, b.w, c.w)};
+}
+__device__ __forceinline__ V4 vaxpy(float c, V4 a, V4 b) {  // c a + b
+    return V4{fmaf(c, a.x, b.x), fmaf(c, a.y, b.y), fmaf(c, a.z, b.z), fmaf(c, a.w, b.w)};
+}
+__device__ __forceinline__ float vmul(float a, float b) { return a * b; }
+__device__ __forceinline__ float vscale(float c, float a) { return c * a; }
+__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float vaxpy(float c, float a, float b) { return fmaf(c, a, b); }
+
+template <class T>
+__device__ __forceinline__ T v_central(T m2, T m1, T p1, T p2) {
+    return vaxpy(-C_1_12, p2, vaxpy(C_2_3, p1, vaxpy(-C_2_3, m1, vscale(C_1_12, m2))));
+}
+template <class T>
+__device__ __forceinline__ T v_head(T a, T b, T c, T d) {
+    return vaxpy(C_1_3, d, vaxpy(-C_3_2, c, vaxpy(C_THREE, b, vscale(C_HEAD0, a))));
+}
+template <class T>
+__device__ __forceinline__ T v_tail(T a, T b, T c, T d) {
+    return vaxpy(C_TAIL3, d, vaxpy(-C_THREE, c, vaxpy(C_3_2, b, vscale(C_TAIL0, a))));
+}
+
+// One axis at R neighbouring cells x0 .. x0+R-1 of a line of N cells, in two halves so that few
+// values are live at a time; derivatives unscaled (results times 1/dx^2).  EDGE: a cell of the warp
+// lies within reach of one of the line's ends.  cell(f, d) is cell x0 + d of field f (0: u, 1: D, both
+// edge-padded; 2: lambda_u, zero outside the grid); of(f, t) the same at d = t - 4 for the t known at
+// compile time.  v_central with its arguments reversed is -G.
+//
+// gd: lambda u'' + B^T (lambda u').
+template <int R, bool EDGE, class T, class Of, class At>
+__device__ __forceinline__ void axis_gd(int x0, int N, Of of, At cell, T (&gd)[R]) {
+    T U[R + 8], ux[R + 4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) U[t] = of(0, t);
+#pragma unroll
+    for (int t = 0; t < R + 4; ++t) {
+        U[t + 4] = of(0, t + 4);
+        ux[t] = v_central(U[t], U[t + 1], U[t + 3], U[t + 4]);
+        if (EDGE) {
+            const int x = x0 - 2 + t;
+            if (t <= 2 && x <= 0) ux[t] = v_head(cell(0, t - 2), cell(0, t - 1), cell(0, t), cell(0, t + 1));
+            if (t >= 1 && x >= N - 1) ux[t] = v_tail(cell(0, t - 5), cell(0, t - 4), cell(0, t - 3), cell(0, t - 2));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        T d = v_central(ux[k], ux[k + 1], ux[k + 3], ux[k + 4]);
+        if (EDGE) {
+            const int x = x0 + k;
+            if (k == 0 && x == 0) d = v_head(ux[2], ux[3], ux[4], ux[5]);
+            if (x == N - 1) {
+                T far = ux[k >= 1 ? k - 1 : 0];
+                if (k == 0) far = v_central(cell(0, -5), cell(0, -4), cell(0, -2), cell(0, -1));
+                d = v_tail(far, ux[k], ux[k + 1], ux[k + 2]);
+            }
+        }
+        gd[k] = vmul(of(2, k + 4), d);
+    }
+    // lambda u', with the one-sided rows 0 and N-1 taken out of the central sums
+    T (&m)[R + 4] = ux;
+#pragma unroll
+    for (int t = 0; t < R + 4; ++t) m[t] = vmul(of(2, t + 2), ux[t]);
+    if (EDGE) {
+        const T zero = vscale(0.0f, T{}), m1 = m[3];
+        const int dn = N - 1 - x0;
+        T m0 = zero, mn = zero;
+        if (x0 <= 4) m0 = vmul(cell(2, -x0), v_head(cell(0, -x0), cell(0, 1 - x0), cell(0, 2 - x0), cell(0, 3 - x0)));
+        if (dn <= R + 4) mn = vmul(cell(2, dn), v_tail(cell(0, dn - 3), cell(0, dn - 2), cell(0, dn - 1), cell(0, dn)));
+#pragma unroll
+        for (int t = 0; t < R + 4; ++t) {
+            if (t < 3 && x0 - 2 + t <= 0) m[t] = zero;
+            if (t >= 2 && x0 - 2 + t >= N - 1) m[t] = zero;
+        }
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int x = x0 + k;
+            gd[k] = vaxpy((unsigned)x < 4u ? kHeadC[x & 3] : 0.0f, m0, gd[k]);
+            gd[k] = vaxpy(x >= N - 4 && x < N ? kTailC[(x - N) & 3] : 0.0f, mn, gd[k]);
+            // the pad rows fold onto the first and the last cell
+            if (k == 0 && x == 0) gd[k] = vaxpy(C_1_12, m1, gd[k]);
+            if (x == N - 1) gd[k] = vaxpy(-C_1_12, m[k + 1], gd[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) gd[k] = vaxpy(1.0f, v_central(m[k + 4], m[k + 3], m[k + 1], m[k]), gd[k]);
+}
+
+// at: A^T (D lambda) + B^T ((B D) lambda).
+template <int R, bool EDGE, class T, class Of, class At>
+__device__ __forceinline__ void axis_at(int x0, int N, Of of, At cell, T (&at)[R]) {
+    const T zero = vscale(0.0f, T{});
+    // D lambda at the one-sided rows (q0, qn), and what these rows and the pad rows carry into the
+    // second operator (b0, bm and bn, bp)
+    T q0 = zero, b0 = zero, bm = zero, qn = zero, bn = zero, bp = zero;
+    if (EDGE) {
+        if (x0 <= 4) {
+            const int d = -x0;
+            auto Q = [&](int k) { return vmul(cell(1, d + k), cell(2, d + k)); };
+            q0 = Q(0);
+            const T q1 = Q(1);
+            bm = vscale(C_1_12, q1);
+            const T g = v_head(cell(1, d), cell(1, d + 1), cell(1, d + 2), cell(1, d + 3));
+            b0 = vfma(g, cell(2, d), vaxpy(C_HEAD0, q0, vaxpy(-C_2_3, q1, vscale(C_1_12, Q(2)))));
+        }
+        if (N - 1 - x0 <= R + 4) {
+            const int d = N - 1 - x0;
+            auto Q = [&](int k) { return vmul(cell(1, d - k), cell(2, d - k)); };
+            qn = Q(0);
+            const T q1 = Q(1);
+            bp = vscale(-C_1_12, q1);
+            const T g = v_tail(cell(1, d - 3), cell(1, d - 2), cell(1, d - 1), cell(1, d));
+            bn = vfma(g, cell(2, d), vaxpy(C_TAIL3, qn, vaxpy(C_2_3, q1, vscale(-C_1_12, Q(2)))));
+        }
+    }
+    T D[R + 8], q[R + 8], s[R + 4];
+    auto take = [&](int t) {
+        D[t] = of(1, t);
+        q[t] = vmul(D[t], of(2, t));
+        if (EDGE) {
+            const int x = x0 - 4 + t;
+            if ((t <= 4 && x == 0) || (t >= 4 && x == N - 1)) q[t] = zero;
+        }
+    };
+#pragma unroll
+    for (int t = 0; t < 4; ++t) take(t);
+#pragma unroll
+    for (int t = 0; t < R + 4; ++t) {
+        take(t + 4);
+        T g = v_central(D[t], D[t + 1], D[t + 3], D[t + 4]);
+        T y = v_central(q[t + 4], q[t + 3], q[t + 1], q[t]);
+        if (EDGE) {
+            const int x = x0 - 2 + t;
+            if (t <= 2 && x == 0) g = v_head(cell(1, t - 2), cell(1, t - 1), cell(1, t), cell(1, t + 1));
+            if (t >= 1 && x == N - 1) g = v_tail(cell(1, t - 5), cell(1, t - 4), cell(1, t - 3), cell(1, t - 2));
+            y = vaxpy((unsigned)x < 4u ? kHeadC[x & 3] : 0.0f, q0, y);
+            y = vaxpy((unsigned)(x - N + 4) < 4u ? kTailC[(x - N) & 3] : 0.0f, qn, y);
+        }
+        s[t] = vfma(g, of(2, t + 2), y);
+    }
+    const T s1 = s[3];
+    if (EDGE)  // rows -1, 0 and N-1, N leave the central sums of the second operator
+#pragma unroll
+        for (int t = 0; t < R + 4; ++t) {
+            if (t < 3 && x0 - 2 + t <= 0) s[t] = zero;
+            if (t >= 2 && x0 - 2 + t >= N - 1) s[t] = zero;
+        }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        T a = v_central(s[k + 4], s[k + 3], s[k + 1], s[k]);
+        if (EDGE) {
+            const int x = x0 + k;
+            a = vaxpy((unsigned)x < 4u ? kHeadC[x & 3] : 0.0f, b0, a);
+            a = vaxpy((unsigned)x < 3u ? kHeadC[(x + 1) & 3] : 0.0f, bm, a);
+            a = vaxpy(x >= N - 4 && x < N ? kTailC[(x - N) & 3] : 0.0f, bn, a);
+            a = vaxpy(x >= N - 3 && x < N ? kTailC[(x - N - 1) & 3] : 0.0f, bp, a);
+            if (k == 0 && x == 0) a = vaxpy(C_HEAD0, bm, vaxpy(C_1_12, s1, a));  // the pad rows fold
+            if (x == N - 1) a = vaxpy(C_TAIL3, bp, vaxpy(-C_1_12, s[k + 1], a));
+        }
+        at[k] = a;
+    }
+}
+
+// Sums 16 values over a warp: lane i < 16 returns the sum of v[i] (lanes 16..31 the same).  Each
+// exchange halves the values a lane still carries: 16 exchanges instead of 5 per value.
+__device__ __forceinline__ float warp_sum16(float (&v)[16]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1) {
+        const bool up = (lane & h) != 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k >= h) break;
+            const float keep = up ? v[k + h] : v[k], give = up ? v[k] : v[k + h];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+
+__device__ __forceinline__ void cp_async16(float *dst, const float *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+// Tile (bx, by) of an nbx x nby cut of the grid (rows in groups of LR, columns in quads, dealt out
+// evenly; the last tile row's groups are aligned to the bottom, so that rows 0 and H-1 are the first
+// and the last row of a thread).  Its dL/dtheta sums go to slot by * nbx + bx of a.gtheta.
+__device__ __forceinline__ void adjoint_line_tile(const AdjointArgs &a, int bx, int by, int nbx,
+                                                  int nby) {
+    __shared__ __align__(16) float su[LSH * LSW];
+    __shared__ __align__(16) float sd[LSH * LSW];
+    __shared__ __align__(16) float sl[LSH * LSW];
+    __shared__ float4 sp[4][LR][LU];  // a unit's own v, w, lambda_v, lambda_w; the first then its
+                                      // lambda_u through the currents
+    __shared__ float4 sr[2][LR][LU];  // the x direction's part of lambda_u and of dL/dD
+    __shared__ float red[LU / 32][16];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int role = tid / LU, unit = tid % LU;
+    const int H = a.H, W = a.W, pitch = a.pitch;
+    const float dt = a.dt, rdx = a.rdx;
+    const int ng = (H + LR - 1) / LR, nq = (W + 3) / 4;
+    const int g0 = by * ng / nby, g1 = (by + 1) * ng / nby;
+    const int c0 = bx * nq / nbx, c1 = (bx + 1) * nq / nbx;
+    const int shift = by == nby - 1 ? ng * LR - H : 0;
+    const int row0 = g0 * LR - shift, j0 = 4 * c0;   // the tile's first group's first row
+    const int rows = (g1 - g0) * LR, tq = c1 - c0;
+    // units by pairs of quad columns: those near the left and right sides then lie in few warps
+    const int G = g1 - g0, pair = (unit >> 1) / G;
+    const bool mine = 2 * pair + (unit & 1) < tq;
+    const int lq = mine ? 2 * pair + (unit & 1) : 0, lg = mine ? (unit >> 1) - pair * G : 0;
+    const int i0 = row0 + lg * LR, j = j0 + 4 * lq;
+    const int k_lo = by == nby - 1 && lg == 0 ? shift : 0;  // rows before it belong to the tile above
+    const int64_t off0 = (int64_t)i0 * pitch + j;
+
+    // All reads go through L2: with programmatic dependent launch this block may have started before
+    // the step that wrote lambda and dL/dD ended, and L1 is not coherent with the other SMs.
+    // ---- stage u, D, lambda_u with 4 cells around: clamped copies outside the grid, lambda 0 ------
+    constexpr int N4 = LSW / 4, RPP = LNT / N4;  // quads of a staged row, rows per pass
+    if (tid < RPP * N4 && tid % N4 < tq + 2) {
+        const int c = 4 * (tid % N4), jc = j0 - 4 + c;
+        const bool quad_in = jc >= 0 && jc + 3 < W;
+        for (int r = tid / N4; r < rows + 8; r += RPP) {
+            const int i = row0 - 4 + r;
+            const int64_t g = (int64_t)clampi(i, 0, H - 1) * pitch;
+            const int o = r * LSW + c;
+            const bool row_in = i >= 0 && i < H;
+            if (quad_in) {
+                cp_async16(su + o, a.u + g + jc);
+                cp_async16(sd + o, a.D + g + jc);
+                if (row_in) cp_async16(sl + o, a.lu + g + jc);
+                else *reinterpret_cast<float4 *>(sl + o) = make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+                // a quad across or beyond the grid's side: the nearest cell in place of those outside
+                const int jn = clampi(jc, 0, 4 * (nq - 1));  // the quad of the row that has it
+                float4 x = __ldcg(reinterpret_cast<const float4 *>(a.u + g + jn));
+                float4 y = __ldcg(reinterpret_cast<const float4 *>(a.D + g + jn));
+                float4 z = __ldcg(reinterpret_cast<const float4 *>(a.lu + g + jn));
+                if (jc < 0) {
+                    x.y = x.z = x.w = x.x;
+                    y.y = y.z = y.w = y.x;
+                }
+                const int n = W - 1 - jn;  // the last cell's place in the quad
+                if (n < 1) x.y = x.x, y.y = y.x;
+                if (n < 2) x.z = x.y, y.z = y.y;
+                if (n < 3) x.w = x.z, y.w = y.z;
+                if (jc > jn) {
+                    x.x = x.y = x.z = x.w;
+                    y.x = y.y = y.z = y.w;
+                }
+                const bool l_in = row_in && jc == jn;
+                z.x = l_in ? z.x : 0.0f;
+                z.y = l_in && n >= 1 ? z.y : 0.0f;
+                z.z = l_in && n >= 2 ? z.z : 0.0f;
+                z.w = l_in && n >= 3 ? z.w : 0.0f;
+                *reinterpret_cast<float4 *>(su + o) = x;
+                *reinterpret_cast<float4 *>(sd + o) = y;
+                *reinterpret_cast<float4 *>(sl + o) = z;
+            }
+        }
+    }
+    if (role == 0)
+#pragma unroll
+        for (int k = 0; k < LR; ++k)
+            if (mine && k >= k_lo) {
+                const int64_t o = off0 + (int64_t)k * pitch;  // j < W: the quad lies in the pitched row
+                cp_async16(reinterpret_cast<float *>(&sp[0][k][unit]), a.v + o);
+                cp_async16(reinterpret_cast<float *>(&sp[1][k][unit]), a.w + o);
+                cp_async16(reinterpret_cast<float *>(&sp[2][k][unit]), a.lv + o);
+                cp_async16(reinterpret_cast<float *>(&sp[3][k][unit]), a.lw + o);
+            } else {
+#pragma unroll
+                for (int f = 0; f < 4; ++f) sp[f][k][unit] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+    const unsigned active = __ballot_sync(0xffffffffu, lane < a.n_stim && stim_active(a.stim[lane < kMaxStim ? lane : 0], a.t));
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+
+    double *const slot = a.gtheta + (int64_t)(by * nbx + bx) * kAdjParamStride + (tid < 12 ? tid : 0);
+    const double slot_was = a.gtheta && tid < 12 ? __ldcg(slot) : 0.0;  // early: its trip overlaps the work
+
+    // Role 0 takes the pointwise part, role 1 the x direction (along rows), of the unit's two rows;
+    // then the y direction of row 0 and of row 1: the chain of one thread is half as long.
+    const int base = (lg * LR + 4) * LSW + 4 * lq + 4;  // the unit's first cell
+    if (role == 0) {
+        const Model &md = a.m;
+        float gth[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) gth[k] = 0.0f;
+#pragma unroll 1
+        for (int k = 0; k < LR; ++k) {
+            const float4 v4 = sp[0][k][unit], w4 = sp[1][k][unit];
+            float4 lv4 = sp[2][k][unit], lw4 = sp[3][k][unit];
+            const float4 u4 = *reinterpret_cast<const float4 *>(su + base + k * LSW);
+            const float4 l4 = *reinterpret_cast<const float4 *>(sl + base + k * LSW);
+            float4 lj4 = l4;  // lambda_u where the current is the model's
+            const int i = i0 + k;
+            const int64_t o = off0 + (int64_t)k * pitch;
+            const bool row_ok = mine && k >= k_lo;
+            if (!row_ok) lj4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j + 3 >= W) {  // columns beyond W (lambda_u is zero there)
+                if (j + 1 >= W) lv4.y = lw4.y = 0.f;
+                if (j + 2 >= W) lv4.z = lw4.z = 0.f;
+                lv4.w = j + 3 >= W ? 0.f : lv4.w;
+                lw4.w = j + 3 >= W ? 0.f : lw4.w;
+            }
+            if (active && row_ok)  // cells whose current a stimulus replaces
+                for (unsigned x = active; x; x &= x - 1) {
+                    const Stim &st = a.stim[__ffs(x) - 1];
+                    float4 f;
+                    if (st.field) {
+                        f = __ldg(reinterpret_cast<const float4 *>(st.field + o));
+                    } else {
+                        const bool in = i >= st.r0 && i < st.r1;
+                        f.x = in && j >= st.c0 && j < st.c1 ? st.amplitude : 0.0f;
+                        f.y = in && j + 1 >= st.c0 && j + 1 < st.c1 ? st.amplitude : 0.0f;
+                        f.z = in && j + 2 >= st.c0 && j + 2 < st.c1 ? st.amplitude : 0.0f;
+                        f.w = in && j + 3 >= st.c0 && j + 3 < st.c1 ? st.amplitude : 0.0f;
+                    }
+                    if (f.x != 0.0f) lj4.x = 0.0f;
+                    if (f.y != 0.0f) lj4.y = 0.0f;
+                    if (f.z != 0.0f) lj4.z = 0.0f;
+                    if (f.w != 0.0f) lj4.w = 0.0f;
+                }
+            const float uu[4] = {u4.x, u4.y, u4.z, u4.w}, ll[4] = {l4.x, l4.y, l4.z, l4.w};
+            const float vv[4] = {v4.x, v4.y, v4.z, v4.w}, ww[4] = {w4.x, w4.y, w4.z, w4.w};
+            const float lvv[4] = {lv4.x, lv4.y, lv4.z, lv4.w}, lww[4] = {lw4.x, lw4.y, lw4.z, lw4.w};
+            const float ljj[4] = {lj4.x, lj4.y, lj4.z, lj4.w};
+            float ov[4], ow[4], pu[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float u = uu[c], v = vv[c], w = ww[c], lv = lvv[c], lw = lww[c], lj = ljj[c];
+                const bool p = u >= md.V_c, q = u >= md.V_v;
+                const float uk = u - md.V_csi;
+                const float S = one_plus_tanh(md.k * uk);  // 1 + tanh
+                const float sech2 = S * (2.0f - S);        // 1 - tanh^2
+                const float uc = u - md.V_c, u1 = 1.0f - u;
+                ov[c] = lv * (1.0f + dt * (p ? -md.r_tau_vp : (q ? -md.r_tau_v2m : -md.r_tau_v1m)));
+                ow[c] = lw * (1.0f + dt * (p ? -md.r_tau_wp : -md.r_tau_wm));
+                const float dfi = p ? -v * (1.0f + md.V_c - 2.0f * u) * md.r_tau_d : 0.0f;
+                const float dso = p ? 0.0f : md.r_tau_0;
+                const float dsi = -w * md.k * sech2 * md.r_2tau_si;
+                const float mu = dt * lj;
+                ov[c] = fmaf(mu, p ? uc * u1 * md.r_tau_d * md.r_Cm : 0.0f, ov[c]);
+                ow[c] = fmaf(mu, S * md.r_2tau_si * md.r_Cm, ow[c]);
+                pu[c] = fmaf(mu, -(dfi + dso + dsi) * md.r_Cm, ll[c]);
+                // parameter sums without their constant factors (cardiax/params.py fields 0..11)
+                const float lvp = p ? lv : 0.0f, lvo = (lv - lvp) * (1.0f - v), lvq = q ? lvo : 0.0f;
+                const float lwp = p ? lw : 0.0f;
+                gth[0] = fmaf(lvp, v, gth[0]);
+                gth[1] += lvo - lvq;
+                gth[2] += lvq;
+                gth[3] = fmaf(lwp, w, gth[3]);
+                gth[4] = fmaf(lw - lwp, 1.0f - w, gth[4]);
+                const float jp = p ? lj : 0.0f, jv = jp * v * u1, jw = lj * w, js = jw * sech2;
+                gth[5] = fmaf(jv, uc, gth[5]);
+                gth[6] = fmaf(lj - jp, u, gth[6]);
+                gth[7] += jp;
+                gth[8] = fmaf(jw, S, gth[8]);
+                gth[9] = fmaf(js, uk, gth[9]);
+                gth[10] += js;
+                gth[11] += jv;
+            }
+            sp[0][k][unit] = make_float4(pu[0], pu[1], pu[2], pu[3]);
+            if (row_ok) {
+                if (j + 3 < W) {
+                    *reinterpret_cast<float4 *>(a.olv + o) = make_float4(ov[0], ov[1], ov[2], ov[3]);
+                    *reinterpret_cast<float4 *>(a.olw + o) = make_float4(ow[0], ow[1], ow[2], ow[3]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (j + c < W) {
+                            a.olv[o + c] = ov[c];
+                            a.olw[o + c] = ow[c];
+                        }
+                }
+            }
+        }
+        if (a.gtheta) {
+            const float x = warp_sum16(gth);
+            if (lane < 16) red[unit / 32][lane] = x;
+        }
+    } else {
+        V4 x[LR];
+        auto cell = [&](int f, int d) {
+            return ld_v4((f == 0 ? su : f == 1 ? sd : sl) + base + d * LSW);
+        };
+        auto of = [&](int f, int t) { return cell(f, t - 4); };
+        const bool edge = __any_sync(0xffffffffu, mine && (i0 <= 5 || i0 + LR + 1 >= H - 4)) != 0;
+        if (edge) axis_gd<LR, true, V4>(i0, H, of, cell, x);
+        else axis_gd<LR, false, V4>(i0, H, of, cell, x);
+#pragma unroll
+        for (int k = 0; k < LR; ++k) sr[1][k][unit] = make_float4(x[k].x, x[k].y, x[k].z, x[k].w);
+        if (edge) axis_at<LR, true, V4>(i0, H, of, cell, x);
+        else axis_at<LR, false, V4>(i0, H, of, cell, x);
+#pragma unroll
+        for (int k = 0; k < LR; ++k) sr[0][k][unit] = make_float4(x[k].x, x[k].y, x[k].z, x[k].w);
+    }
+    const int k = role;  // LR == 2
+    const bool stored = mine && k >= k_lo;
+    const int64_t g = off0 + (int64_t)k * pitch;
+    float4 gd4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (a.gD && stored) gd4 = __ldcg(reinterpret_cast<const float4 *>(a.gD + g));
+    float ay[4], gy[4];
+    {
+        const int o = base + k * LSW;
+        auto cell = [&](int f, int d) { return (f == 0 ? su : f == 1 ? sd : sl)[o + d]; };
+        float L[12], F[12];
+        auto row = [&](const float *p, float (&x)[12]) {
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                const float4 y = *reinterpret_cast<const float4 *>(p + o + 4 * t - 4);
+                x[4 * t] = y.x, x[4 * t + 1] = y.y, x[4 * t + 2] = y.z, x[4 * t + 3] = y.w;
+            }
+        };
+        row(sl, L);
+        row(su, F);
+        auto of = [&](int f, int t) { return f == 2 ? L[t] : F[t]; };
+        const bool edge = __any_sync(0xffffffffu, mine && (j <= 5 || j + 5 >= W - 4)) != 0;
+        if (edge) axis_gd<4, true, float>(j, W, of, cell, gy);
+        else axis_gd<4, false, float>(j, W, of, cell, gy);
+        row(sd, F);
+        if (edge) axis_at<4, true, float>(j, W, of, cell, ay);
+        else axis_at<4, false, float>(j, W, of, cell, ay);
+    }
+    __syncthreads();
+    if (stored) {
+        const float c2 = rdx * rdx * dt;
+        const float4 pu = sp[0][k][unit], ax = sr[0][k][unit], gx = sr[1][k][unit];
+        const float4 r = make_float4(fmaf(c2, ax.x + ay[0], pu.x), fmaf(c2, ax.y + ay[1], pu.y),
+                                     fmaf(c2, ax.z + ay[2], pu.z), fmaf(c2, ax.w + ay[3], pu.w));
+        gd4 = make_float4(fmaf(c2, gx.x + gy[0], gd4.x), fmaf(c2, gx.y + gy[1], gd4.y),
+                          fmaf(c2, gx.z + gy[2], gd4.z), fmaf(c2, gx.w + gy[3], gd4.w));
+        if (j + 3 < W) {
+            *reinterpret_cast<float4 *>(a.olu + g) = r;
+            if (a.gD) __stcg(reinterpret_cast<float4 *>(a.gD + g), gd4);
+        } else {
+            const float rr[4] = {r.x, r.y, r.z, r.w}, ee[4] = {gd4.x, gd4.y, gd4.z, gd4.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (j + c < W) {
+                    a.olu[g + c] = rr[c];
+                    if (a.gD) __stcg(a.gD + g + c, ee[c]);
+                }
+        }
+    }
+    if (a.gtheta && tid < 12) {
+        double x = 0.0;
+#pragma unroll
+        for (int w = 0; w < LU / 32; ++w) x += (double)red[w][tid];
+        __stcg(slot, fma(a.theta_factor[tid], x, slot_was));
+    }
+}
+
+__global__ void __launch_bounds__(LNT, 2) fk_adjoint_line_kernel(const __grid_constant__ AdjointArgs a) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+    adjoint_line_tile(a, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
+}
+
+// The device copy of an experiment's arguments, moved to step k of its segment (see
+// fk_adjoint_batch_kernel); all threads, two barriers.
+__device__ __forceinline__ void stage_experiment(AdjointArgs &sa, const AdjointArgs *exps, int64_t k_stride,
+                                                 int k, int parity, float t) {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(exps + blockIdx.z);
     uint32_t *dst = reinterpret_cast<uint32_t *>(&sa);
-    for (int w = threadIdx.x; w < (int)(sizeof(AdjointArgs) / 4); w += ANT) dst[w] = __ldg(src + w);
+    for (int w = threadIdx.x; w < (int)(sizeof(AdjointArgs) / 4); w += blockDim.x) dst[w] = __ldg(src + w);
     __syncthreads();
     if (threadIdx.x == 0) {
         const int64_t o = (int64_t)k * k_stride;
@@ -557,17 +1055,80 @@ __global__ void __launch_bounds__(ANT, 4) fk_adjoint_batch_kernel(const AdjointA
         }
     }
     __syncthreads();
+}
+
+// One reverse step of many experiments (blockIdx.z): exps[e] describes step 0 of experiment e's
+// segment with the cotangent ping-pong buffers (lu.. = buffer A, olu.. = buffer B); step k reads
+// the state k * k_stride further on, and parity 1 swaps the two cotangent buffers.
+__global__ void __launch_bounds__(ANT, 4) fk_adjoint_batch_kernel(const AdjointArgs *__restrict__ exps,
+                                                               int64_t k_stride, int k, int parity,
+                                                               float t) {
+    __shared__ __align__(16) AdjointArgs sa;
+    stage_experiment(sa, exps, k_stride, k, parity, t);
     adjoint_tile(sa, blockIdx.x, blockIdx.y, gridDim.x);
+}
+
+__global__ void __launch_bounds__(LNT, 2)
+    fk_adjoint_line_batch_kernel(const AdjointArgs *__restrict__ exps, int64_t k_stride, int k,
+                                 int parity, float t) {
+    __shared__ __align__(16) AdjointArgs sa;
+    grid_dependency_wait();
+    grid_launch_dependents();
+    stage_experiment(sa, exps, k_stride, k, parity, t);
+    adjoint_line_tile(sa, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
+}
+
+// Which kernel takes a grid, and its blocks.
+bool long_lines(int H, int W) { return H >= kLineMin && W >= kLineMin; }
+dim3 adjoint_grid(int H, int W, int n_exp) {
+    if (!long_lines(H, W)) return dim3((W + ATX - 1) / ATX, (H + ATY - 1) / ATY, n_exp);
+    return dim3(((W + 3) / 4 + LQ - 1) / LQ, ((H + LR - 1) / LR + LG - 1) / LG, n_exp);
+}
+
+template <class K, class... A>
+cudaError_t launch_line(K kernel, dim3 grid, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(LNT);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace
 
+void set_theta_factors(AdjointArgs &a) {
+    const Model &m = a.m;
+    const double d = a.dt, cm = m.r_Cm, si = m.r_2tau_si;
+    const double f[12] = {
+        d * m.r_tau_vp * m.r_tau_vp,      // tau_v_plus
+        -d * m.r_tau_v1m * m.r_tau_v1m,   // tau_v1_minus
+        -d * m.r_tau_v2m * m.r_tau_v2m,   // tau_v2_minus
+        d * m.r_tau_wp * m.r_tau_wp,      // tau_w_plus
+        -d * m.r_tau_wm * m.r_tau_wm,     // tau_w_minus
+        -d * m.r_tau_d * m.r_tau_d * cm,  // tau_d
+        d * m.r_tau_0 * m.r_tau_0 * cm,   // tau_0
+        d * m.inv_tau_r * m.inv_tau_r * cm,  // tau_r
+        -d * 2.0 * si * si * cm,          // tau_si
+        d * si * cm,                      // k
+        -d * m.k * si * cm,               // V_csi
+        -d * m.r_tau_d * cm,              // V_c
+    };
+    for (int k = 0; k < 12; ++k) a.theta_factor[k] = f[k];
+}
+
 int64_t adjoint_slots(int H, int W) {
-    return (int64_t)((W + ATX - 1) / ATX) * ((H + ATY - 1) / ATY);
+    const dim3 g = adjoint_grid(H, W, 1);
+    return (int64_t)g.x * g.y;
 }
 
 cudaError_t launch_adjoint(const AdjointArgs &a, cudaStream_t stream) {
-    dim3 grid((a.W + ATX - 1) / ATX, (a.H + ATY - 1) / ATY);
+    const dim3 grid = adjoint_grid(a.H, a.W, 1);
+    if (long_lines(a.H, a.W)) return launch_line(fk_adjoint_line_kernel, grid, stream, a);
     fk_adjoint_kernel<<<grid, ANT, 0, stream>>>(a);
     return cudaGetLastError();
 }
@@ -575,7 +1136,9 @@ cudaError_t launch_adjoint(const AdjointArgs &a, cudaStream_t stream) {
 cudaError_t launch_adjoint_batch(const AdjointArgs *exps, int n_exp, int H, int W, int64_t k_stride,
                                  int k, int parity, float t, cudaStream_t stream) {
     if (n_exp < 1) return cudaSuccess;
-    dim3 grid((W + ATX - 1) / ATX, (H + ATY - 1) / ATY, n_exp);
+    const dim3 grid = adjoint_grid(H, W, n_exp);
+    if (long_lines(H, W))
+        return launch_line(fk_adjoint_line_batch_kernel, grid, stream, exps, k_stride, k, parity, t);
     fk_adjoint_batch_kernel<<<grid, ANT, 0, stream>>>(exps, k_stride, k, parity, t);
     return cudaGetLastError();
 }

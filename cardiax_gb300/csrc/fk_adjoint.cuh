@@ -23,7 +23,12 @@ struct AdjointArgs {
     int n_stim;
     Model m;
     Stim stim[kMaxStim];
+    double theta_factor[12];           // constant factors of the parameter sums (set_theta_factors)
 };
+
+// dt and the model's constants in dL/dtheta, fields 0..11 of cardiax/params.py (field 12, V_v, enters
+// only through a Heaviside gate: zero); from a.m and a.dt.
+void set_theta_factors(AdjointArgs &a);
 
 // Number of dL/dtheta slots (kAdjParamStride doubles each) written by launch_adjoint.
 int64_t adjoint_slots(int H, int W);

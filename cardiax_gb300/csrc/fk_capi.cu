@@ -1038,6 +1038,7 @@ int fk_adjoint_step(fk_grid g, const float *state, const float *D, const fk_para
     a.rdx = 1.0f / (float)dx;
     a.n_stim = n_stimuli;
     a.m = make_model(*p);
+    set_theta_factors(a);
     return launch_adjoint(a, (cudaStream_t)stream) == cudaSuccess ? FK_OK : FK_ERR_CUDA;
 }
 
@@ -1093,6 +1094,7 @@ int fk_adjoint_batch_range(int n_exp, fk_grid g, const float *bufs, int64_t exp_
         a.rdx = 1.0f / (float)dx;
         a.n_stim = n_stimuli[e];
         a.m = m;
+        set_theta_factors(a);
     }
     cudaStream_t cs = (cudaStream_t)stream;
     AdjointArgs *dexp = static_cast<AdjointArgs *>(workspace);
