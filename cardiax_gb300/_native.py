@@ -47,6 +47,12 @@ class Activation(ctypes.Structure):
                 ("threshold", ctypes.c_float)]
 
 
+class FieldKind(ctypes.Structure):
+    """fk_field_kind: 0 empty, 1 rectangle, 2 dense."""
+    _fields_ = [("kind", ctypes.c_int32), ("r0", ctypes.c_int32), ("r1", ctypes.c_int32),
+                ("c0", ctypes.c_int32), ("c1", ctypes.c_int32), ("amplitude", ctypes.c_float)]
+
+
 class TissueDesc(ctypes.Structure):
     _fields_ = [("g", Grid), ("state", ctypes.c_void_p), ("scratch", ctypes.c_void_p),
                 ("D", ctypes.c_void_p), ("params", Params),
@@ -94,6 +100,8 @@ _SIGNATURES = {
                      _D, _D, _P, _P, _P],
     "fk_forward_heun": [Grid, _P, _P, _P, ctypes.POINTER(Params), ctypes.POINTER(Stimulus), _INT,
                         _I64, _I64, _D, _D, _P],
+    "fk_analyse_fields": [ctypes.POINTER(_P), _INT, _I64, _I64, _I64, _P, ctypes.c_size_t,
+                          ctypes.POINTER(FieldKind), _P],
     "fk_resize_bilinear": [_P, _I64, _I64, _I64, _I64, _P, _I64, _I64, _I64, _INT, _P],
     "fk_rotate_field": [_P, _I64, _I64, _I64, _P, _I64, _D, _P],
     "fk_scar_raster": [_P, _P, _P, _I64, _I64, _I64, _P, _I64, _P, _P],
@@ -130,6 +138,8 @@ def lib(build: bool = True):
                 fn.argtypes = args
             L.fk_batch_workspace_bytes.restype = ctypes.c_size_t
             L.fk_batch_workspace_bytes.argtypes = [ctypes.POINTER(TissueDesc), _INT]
+            L.fk_analyse_workspace_bytes.restype = ctypes.c_size_t
+            L.fk_analyse_workspace_bytes.argtypes = [_INT]
             L.fk_resident_workspace_bytes.restype = ctypes.c_size_t
             L.fk_resident_workspace_bytes.argtypes = [Grid]
             L.fk_flow_flag_words.restype = _I64
@@ -146,5 +156,5 @@ def call(name: str, *args) -> None:
 
 def exported_symbols():
     return (["fk_status_string", "fk_batch_workspace_bytes", "fk_flow_flag_words",
-             "fk_resident_workspace_bytes"]
+             "fk_resident_workspace_bytes", "fk_analyse_workspace_bytes"]
             + list(_SIGNATURES))

@@ -19,7 +19,7 @@ from typing import Sequence
 import torch
 
 from . import _native as N
-from .tissue import (Tissue, as_cuda_f32, params_struct, pitch_of, stimulus_table, stream_handle,
+from .tissue import (Tissue, as_cuda_f32, params_struct, pitch_of, stimulus_tables, stream_handle,
                      to_pitched)
 
 N_THETA = 13
@@ -236,8 +236,8 @@ class _BatchPlan:
         self.stims, self.keep = [], []
         descs = (N.TissueDesc * B)()
         none = N.Activation(None, None, None, 0.0)
-        for b in range(B):
-            arr, n, keep = stimulus_table(stimuli[b], H, W, self.pitch, dev)
+        tables = stimulus_tables([stimuli[b] for b in range(B)], H, W, self.pitch, dev)
+        for b, (arr, n, keep) in enumerate(tables):
             self.stims.append((arr, n))
             self.keep.append(keep)
             descs[b] = N.TissueDesc(self.grid, self.S[b].data_ptr(), self.scratch[b].data_ptr(),

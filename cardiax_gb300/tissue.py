@@ -67,49 +67,71 @@ def params_struct(params) -> N.Params:
     return N.Params(*vals)
 
 
+def analyse_fields(fields: Sequence[torch.Tensor]) -> list:
+    """Classifies stimulus fields of one (H, W) shape on one CUDA device: ``("empty",)`` (all
+    zero), ``("rect", r0, r1, c0, c1, a)`` (a constant ``a`` on a rectangle, zero elsewhere) or
+    ``("dense",)``.  One launch and one synchronisation for all of them (set-up cost, once per
+    tissue or batch)."""
+    if not fields:
+        return []
+    H, W = (int(x) for x in fields[0].shape)
+    rows = [f if f.stride(-1) == 1 and f.stride(0) == W else f.contiguous() for f in fields]
+    n, dev = len(rows), rows[0].device
+    with torch.cuda.device(dev):
+        nbytes = int(N.lib().fk_analyse_workspace_bytes(n))
+        work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        out = (N.FieldKind * n)()
+        N.call("fk_analyse_fields", (ctypes.c_void_p * n)(*[f.data_ptr() for f in rows]), n, H, W,
+               W, work.data_ptr(), nbytes, out, stream_handle())
+    return [("empty",) if k.kind == 0 else ("dense",) if k.kind == 2 else
+            ("rect", k.r0, k.r1, k.c0, k.c1, float(k.amplitude)) for k in out]
+
+
 def analyse_field(field: torch.Tensor):
-    """Classifies a stimulus field: ``("empty",)`` (all zero), ``("rect", r0, r1, c0, c1, a)``
-    (a constant ``a`` on a rectangle, zero elsewhere) or ``("dense",)``.  Runs a few reductions
-    on the device and one synchronisation (set-up cost, once per tissue)."""
-    nz = field != 0
-    rows = torch.nonzero(nz.any(1)).flatten()
-    if rows.numel() == 0:
-        return ("empty",)
-    cols = torch.nonzero(nz.any(0)).flatten()
-    r0, r1 = int(rows[0]), int(rows[-1]) + 1
-    c0, c1 = int(cols[0]), int(cols[-1]) + 1
-    box = field[r0:r1, c0:c1]
-    a = box[0, 0]
-    if bool((box == a).all()):
-        return ("rect", r0, r1, c0, c1, float(a))
-    return ("dense",)
+    """:func:`analyse_fields` of one field."""
+    return analyse_fields([field])[0]
+
+
+def stimulus_tables(lists: Sequence[Sequence], H: int, W: int, pitch: int, device) -> list:
+    """The C stimulus table of each list of cardiax-style Stimulus on one grid, with its length and
+    the device buffers it points to (kept alive by the caller)."""
+    protos, fields = [], []
+    for stimuli in lists:
+        for s in stimuli:
+            proto, field = s[0], s[1]
+            protos.append((_scalar(proto[0]), _scalar(proto[1]), _scalar(proto[2])))
+            f = as_cuda_f32(field, device)
+            if tuple(f.shape) != (H, W):
+                raise ValueError(f"stimulus field shape {tuple(f.shape)} != grid {(H, W)}")
+            fields.append(f)
+    kinds = analyse_fields(fields)
+    tables, at = [], 0
+    for stimuli in lists:
+        entries, keep = [], []
+        for (start, duration, period), f, kind in zip(protos[at:at + len(stimuli)],
+                                                      fields[at:at + len(stimuli)],
+                                                      kinds[at:at + len(stimuli)]):
+            if kind[0] == "empty":
+                continue  # a zero field never replaces the current
+            if kind[0] == "rect":
+                _, r0, r1, c0, c1, a = kind
+                entries.append(N.Stimulus(start, duration, period, None, r0, r1, c0, c1, a))
+            else:
+                p = to_pitched(f, H, W, pitch, device)
+                keep.append(p)
+                entries.append(N.Stimulus(start, duration, period, p.data_ptr(), 0, 0, 0, 0, 0.0))
+        at += len(stimuli)
+        if len(entries) > N.FK_MAX_STIMULI:
+            raise ValueError(f"at most {N.FK_MAX_STIMULI} non-zero stimuli are supported per tissue "
+                             f"(of which at most {N.FK_MAX_ACTIVE_STIMULI} active at one step)")
+        arr = (N.Stimulus * max(1, len(entries)))(*entries)
+        tables.append((arr, len(entries), keep))
+    return tables
 
 
 def stimulus_table(stimuli: Sequence, H: int, W: int, pitch: int, device):
-    """The C stimulus table for ``stimuli`` (sequence of cardiax-style Stimulus), plus the
-    device buffers it points to (kept alive by the caller)."""
-    entries, keep = [], []
-    for s in stimuli:
-        proto, field = s[0], s[1]
-        start, duration, period = (_scalar(proto[0]), _scalar(proto[1]), _scalar(proto[2]))
-        f = as_cuda_f32(field, device)
-        if tuple(f.shape) != (H, W):
-            raise ValueError(f"stimulus field shape {tuple(f.shape)} != grid {(H, W)}")
-        kind = analyse_field(f)
-        if kind[0] == "empty":
-            continue  # a zero field never replaces the current
-        if kind[0] == "rect":
-            _, r0, r1, c0, c1, a = kind
-            entries.append(N.Stimulus(start, duration, period, None, r0, r1, c0, c1, a))
-        else:
-            p = to_pitched(f, H, W, pitch, device)
-            keep.append(p)
-            entries.append(N.Stimulus(start, duration, period, p.data_ptr(), 0, 0, 0, 0, 0.0))
-    if len(entries) > N.FK_MAX_STIMULI:
-        raise ValueError(f"at most {N.FK_MAX_STIMULI} non-zero stimuli are supported per tissue "
-                         f"(of which at most {N.FK_MAX_ACTIVE_STIMULI} active at one step)")
-    arr = (N.Stimulus * max(1, len(entries)))(*entries)
-    return arr, len(entries), keep
+    """:func:`stimulus_tables` of one list."""
+    return stimulus_tables([list(stimuli)], H, W, pitch, device)[0]
 
 
 def stream_handle() -> int:

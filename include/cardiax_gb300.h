@@ -217,6 +217,19 @@ int fk_forward_flow(fk_grid g, const float *state0, float *scratch, const float 
                     const int64_t *checkpoints, int n_checkpoints, double dt, double dx,
                     float *out, int32_t *flags, int64_t n_flags, void *stream);
 
+/* ---- stimulus fields ----------------------------------------------------------------------------
+ * What each of the n H x W fields (row pitch `pitch`, host array of device pointers) is: 0 empty
+ * (all zero), 1 the constant `amplitude` on the rectangle [r0, r1) x [c0, c1) and zero elsewhere,
+ * 2 anything else.  `workspace`: fk_analyse_workspace_bytes(n) bytes of device memory, 8-byte
+ * aligned; `out`: n host entries, filled when the call returns (it waits for `stream`). */
+typedef struct {
+    int32_t kind, r0, r1, c0, c1;
+    float amplitude;
+} fk_field_kind;
+size_t fk_analyse_workspace_bytes(int n);
+int fk_analyse_fields(const float *const *fields, int n, int64_t H, int64_t W, int64_t pitch,
+                      void *workspace, size_t workspace_bytes, fk_field_kind *out, void *stream);
+
 /* ---- checkpoint emission ----------------------------------------------------------------------
  * io.imresize (cardiax/io.py:118-124), which the data-generation caller applies to every
  * checkpoint (deepx/generate.py:187-199): `planes` float32 planes of H x W (row pitch in_pitch,
