@@ -323,6 +323,12 @@ int step_once(const fk_grid &g, const float *in, float *out, const float *D, con
         a.act_count = act->count;
         a.act_threshold = act->threshold;
     }
+    if (heun == 2) {
+        a.v = x0;
+        a.w = x0 + plane;
+    }
+    // stage 1's input is read again by stage 2
+    if (heun == 1) a.l2_hints = 0;
     a.dso = dso;
     a.x0 = x0;
     a.d1 = d1;
@@ -842,9 +848,10 @@ int fk_forward_euler(fk_grid g, float *state, float *scratch, const float *D, co
 }
 
 // One Heun step from `in` to `out` with work = [d1, x1, ...]: two launches of the step kernel.
-// Stage 1 is the Euler step x1 = x + dt d1 that also stores d1 = f(x, t); stage 2 evaluates
-// f(x1, t) and writes x + (d1 + f(x1, t)) dt/2 -- per cell the operations of the derivative,
-// x1 = fmaf(d1, dt, x) and fmaf(d1 + d2, dt/2, x) of cardiax/solve.py:73-85.
+// Stage 1 is the Euler step of u, x1.u = x.u + dt d1.u, that also stores d1.u; stage 2 forms the rest
+// of x1 and d1 again from the gates at x, evaluates f(x1, t) and writes x + (d1 + f(x1, t)) dt/2 --
+// per cell the operations of the derivative, x1 = fmaf(d1, dt, x) and fmaf(d1 + d2, dt/2, x) of
+// cardiax/solve.py:73-85.
 static int heun_once(const fk_grid &g, const float *in, float *out, float *work, const float *D,
                      const Model &m, const Stim *st, int ns, int64_t t, float dt, float rdx,
                      const CUtensorMap &tm_d, MapCache &maps, int *status, cudaStream_t s) {

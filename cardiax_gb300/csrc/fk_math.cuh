@@ -127,6 +127,18 @@ __device__ __forceinline__ Reaction reaction(float u, float v, float w, const Mo
     return r;
 }
 
+// The gates' derivatives alone, by the operations of reaction().
+struct Gates {
+    float dv, dw;
+};
+__device__ __forceinline__ Gates gates(float u, float v, float w, const Model &m) {
+    const bool p = u >= m.V_c;
+    const float r_tvm = u >= m.V_v ? m.r_tau_v2m : m.r_tau_v1m;
+    const float dv_on = -(v * m.r_tau_vp), dv_off = (1.0f - v) * r_tvm;
+    const float dw_on = -(w * m.r_tau_wp), dw_off = (1.0f - w) * m.r_tau_wm;
+    return Gates{p ? dv_on : dv_off, p ? dw_on : dw_off};
+}
+
 // del(u) = D (u_xx + u_yy) + D_x u_x + D_y u_y  (cardiax/solve.py:55)
 __device__ __forceinline__ float diffusion(float d, float dx_, float dy_, float ux, float uy,
                                            float uxx, float uyy) {

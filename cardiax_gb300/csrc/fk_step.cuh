@@ -90,9 +90,11 @@ struct StepArgs {
     // nonzero: the step's live data (the new state and D) fits in L2, so the step kernel marks
     // the input state's reads evict-first and D's evict-last (set by the host per device)
     int l2_hints;
-    // Heun stages (cardiax/solve.py:73-85; fk_step_kernel only).  Stage 1 is the Euler step
-    // x1 = x + dt d1 that also stores d1 = f(x, t) to `dso`; stage 2 reads x1 (the input state),
-    // x0 = x and d1, and writes x0 + (d1 + f(x1, t)) h with h = dt / 2.  Three planes each.
+    // Heun stages (cardiax/solve.py:73-85; fk_step_kernel only).  Stage 1 is the Euler step of u
+    // alone, x1.u = x.u + dt d1.u, that also stores d1.u (one plane) to `dso`.  Stage 2 reads u of x1
+    // as its input state and v, w of x0 = x (a.v, a.w), forms v and w of x1 and of d1 again from the
+    // gates at x0 -- some twenty operations instead of eight planes written and read -- and writes
+    // x0 + (d1 + f(x1, t)) h with h = dt / 2.  `d1`: the plane stage 1 stored.
     float *dso;
     const float *x0, *d1;
     float h;

@@ -99,8 +99,17 @@ __device__ __noinline__ void boundary_cell(const StepArgs &a, float t, unsigned 
     dxD *= rdx;
     dyD *= rdx;
     const int64_t off = (int64_t)i * a.pitch + j;
-    const float u = __ldcg(a.u + off), v = __ldcg(a.v + off), w = __ldcg(a.w + off),
-                d = __ldg(a.D + off);
+    const int64_t plane = (int64_t)a.H * a.pitch;
+    const float u = __ldcg(a.u + off), d = __ldg(a.D + off);
+    float v = __ldcg(a.v + off), w = __ldcg(a.w + off);
+    // Heun stage 2: v, w are those of x0; x1's follow from the gates at x0 as in stage 1
+    const float v0 = v, w0 = w, u0 = heun == 2 ? __ldcg(a.x0 + 2 * plane + off) : 0.0f;
+    Gates g0{0.0f, 0.0f};
+    if (heun == 2) {
+        g0 = gates(u0, v0, w0, a.m);
+        v = fmaf(g0.dv, a.dt, v0);
+        w = fmaf(g0.dw, a.dt, w0);
+    }
     Reaction r = reaction(u, v, w, a.m);
     if (active) {
         float acc = 0.0f;
@@ -115,25 +124,20 @@ __device__ __noinline__ void boundary_cell(const StepArgs &a, float t, unsigned 
     }
     const float du = diffusion(d, dxD, dyD, UX(i), UY(j), uxx, uyy) + r.j_ion;
     float ov, ow, ou;
-    const int64_t plane = (int64_t)a.H * a.pitch;
     if (deriv) {
         ov = r.dv;
         ow = r.dw;
         ou = du;
     } else if (heun == 2) {  // x0 + (d1 + d2) h, d2 = this cell's derivative at x1
-        ov = fmaf(__ldcg(a.d1 + off) + r.dv, a.h, __ldcg(a.x0 + off));
-        ow = fmaf(__ldcg(a.d1 + plane + off) + r.dw, a.h, __ldcg(a.x0 + plane + off));
-        ou = fmaf(__ldcg(a.d1 + 2 * plane + off) + du, a.h, __ldcg(a.x0 + 2 * plane + off));
+        ov = fmaf(g0.dv + r.dv, a.h, v0);
+        ow = fmaf(g0.dw + r.dw, a.h, w0);
+        ou = fmaf(__ldcg(a.d1 + off) + du, a.h, u0);
     } else {
         ov = fmaf(r.dv, a.dt, v);
         ow = fmaf(r.dw, a.dt, w);
         ou = fmaf(du, a.dt, u);
         if (ACT) record_activation(a, t, off, u, ou);
-        if (heun == 1) {
-            __stcg(a.dso + off, r.dv);
-            __stcg(a.dso + plane + off, r.dw);
-            __stcg(a.dso + 2 * plane + off, du);
-        }
+        if (heun == 1) __stcg(a.dso + off, du);
     }
     if (o.v) {
         const int lo = (i - o.i0) * TX + (j - o.j0);
@@ -141,8 +145,10 @@ __device__ __noinline__ void boundary_cell(const StepArgs &a, float t, unsigned 
         o.w[lo] = ow;
         o.u[lo] = ou;
     } else {
-        __stcg(a.vo + off, ov);
-        __stcg(a.wo + off, ow);
+        if (heun != 1) {
+            __stcg(a.vo + off, ov);
+            __stcg(a.wo + off, ow);
+        }
         __stcg(a.uo + off, ou);
     }
 }
@@ -533,7 +539,22 @@ __device__ __forceinline__ bool compute_tile(const StepArgs &a, const PackConsts
             const float4 y0 = ld4(yb), y1 = ld4(yb + 4), y2 = ld4(yb + 8);
             const float4 dl = ld4(db - 4), dr = ld4(db + 4);
             const float4 uc = ld4(su + (r + HALO_U) * SW + HALO_U + 4 * tx);
-            const float4 vc = io.v[k], wc = io.w[k];
+            float4 vc = io.v[k], wc = io.w[k];
+            // Heun stage 2: io holds v, w of x0; x1's follow from the gates at x0, as in stage 1
+            float4 x0u = make_float4(0.f, 0.f, 0.f, 0.f);
+            Gates h0{0.f, 0.f}, h1{0.f, 0.f}, h2{0.f, 0.f}, h3{0.f, 0.f};
+            if (HEUN == 2) {
+                if (whole || (i < H && j < W))
+                    x0u = __ldcg(reinterpret_cast<const float4 *>(a.x0 + 2 * (int64_t)H * pitch + goff));
+                h0 = gates(x0u.x, vc.x, wc.x, a.m);
+                h1 = gates(x0u.y, vc.y, wc.y, a.m);
+                h2 = gates(x0u.z, vc.z, wc.z, a.m);
+                h3 = gates(x0u.w, vc.w, wc.w, a.m);
+                vc = make_float4(fmaf(h0.dv, a.dt, vc.x), fmaf(h1.dv, a.dt, vc.y), fmaf(h2.dv, a.dt, vc.z),
+                                 fmaf(h3.dv, a.dt, vc.w));
+                wc = make_float4(fmaf(h0.dw, a.dt, wc.x), fmaf(h1.dw, a.dt, wc.y), fmaf(h2.dw, a.dt, wc.z),
+                                 fmaf(h3.dw, a.dt, wc.w));
+            }
             const float f[12] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w,
                                  y2.x, y2.y, y2.z, y2.w};  // u_y at columns j-4 .. j+7
             const float g[12] = {dl.x, dl.y, dl.z, dl.w, dcq.lo.x, dcq.lo.y, dcq.hi.x, dcq.hi.y,
@@ -607,25 +628,17 @@ __device__ __forceinline__ bool compute_tile(const StepArgs &a, const PackConsts
                 nw_hi = rh.dw;
                 nu_lo = du_lo;
                 nu_hi = du_hi;
-            } else if (HEUN == 2) {  // x0 + (d1 + d2) h; the input state is x1
-                const int64_t pl = (int64_t)H * pitch;
-                const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 xv = z, xw = z, xu = z, dv1 = z, dw1 = z, du1 = z;
-                if (whole || (i < H && j < W)) {
-                    xv = __ldcg(reinterpret_cast<const float4 *>(a.x0 + goff));
-                    xw = __ldcg(reinterpret_cast<const float4 *>(a.x0 + pl + goff));
-                    xu = __ldcg(reinterpret_cast<const float4 *>(a.x0 + 2 * pl + goff));
-                    dv1 = __ldcg(reinterpret_cast<const float4 *>(a.d1 + goff));
-                    dw1 = __ldcg(reinterpret_cast<const float4 *>(a.d1 + pl + goff));
-                    du1 = __ldcg(reinterpret_cast<const float4 *>(a.d1 + 2 * pl + goff));
-                }
+            } else if (HEUN == 2) {  // x0 + (d1 + d2) h, d2 the derivative at x1
+                float4 du1 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (whole || (i < H && j < W)) du1 = __ldcg(reinterpret_cast<const float4 *>(a.d1 + goff));
+                const float4 xv = io.v[k], xw = io.w[k];
                 const float2 hh = mk2(a.h, a.h);
-                nv_lo = p_fma(p_add(mk2(dv1.x, dv1.y), rl.dv), hh, mk2(xv.x, xv.y));
-                nv_hi = p_fma(p_add(mk2(dv1.z, dv1.w), rh.dv), hh, mk2(xv.z, xv.w));
-                nw_lo = p_fma(p_add(mk2(dw1.x, dw1.y), rl.dw), hh, mk2(xw.x, xw.y));
-                nw_hi = p_fma(p_add(mk2(dw1.z, dw1.w), rh.dw), hh, mk2(xw.z, xw.w));
-                nu_lo = p_fma(p_add(mk2(du1.x, du1.y), du_lo), hh, mk2(xu.x, xu.y));
-                nu_hi = p_fma(p_add(mk2(du1.z, du1.w), du_hi), hh, mk2(xu.z, xu.w));
+                nv_lo = p_fma(p_add(mk2(h0.dv, h1.dv), rl.dv), hh, mk2(xv.x, xv.y));
+                nv_hi = p_fma(p_add(mk2(h2.dv, h3.dv), rh.dv), hh, mk2(xv.z, xv.w));
+                nw_lo = p_fma(p_add(mk2(h0.dw, h1.dw), rl.dw), hh, mk2(xw.x, xw.y));
+                nw_hi = p_fma(p_add(mk2(h2.dw, h3.dw), rh.dw), hh, mk2(xw.z, xw.w));
+                nu_lo = p_fma(p_add(mk2(du1.x, du1.y), du_lo), hh, mk2(x0u.x, x0u.y));
+                nu_hi = p_fma(p_add(mk2(du1.z, du1.w), du_hi), hh, mk2(x0u.z, x0u.w));
             } else {
                 nv_lo = p_fma(rl.dv, ps.dt, v_lo);
                 nv_hi = p_fma(rh.dv, ps.dt, v_hi);
@@ -644,38 +657,30 @@ __device__ __forceinline__ bool compute_tile(const StepArgs &a, const PackConsts
             };
             if constexpr (DIRECT) {
                 if (whole || (i < H && j < W)) {
-                    const int64_t pl = (int64_t)H * pitch;
-                    // Heun stage 1 also stores d1 (the derivative at the input state)
-                    const float4 d4v = make_float4(rl.dv.x, rl.dv.y, rh.dv.x, rh.dv.y);
-                    const float4 d4w = make_float4(rl.dw.x, rl.dw.y, rh.dw.x, rh.dw.y);
+                    // Heun stage 1 stores u of x1 and the derivative of u alone (stage 2 forms the
+                    // rest again from the gates at x0)
                     const float4 d4u = make_float4(du_lo.x, du_lo.y, du_hi.x, du_hi.y);
                     if (whole || (!band_mask && j + 3 < W)) {
-                        __stcg(reinterpret_cast<float4 *>(a.vo + goff), ov4);
-                        __stcg(reinterpret_cast<float4 *>(a.wo + goff), ow4);
-                        __stcg(reinterpret_cast<float4 *>(a.uo + goff), ou4);
-                        if (HEUN == 1) {
-                            __stcg(reinterpret_cast<float4 *>(a.dso + goff), d4v);
-                            __stcg(reinterpret_cast<float4 *>(a.dso + pl + goff), d4w);
-                            __stcg(reinterpret_cast<float4 *>(a.dso + 2 * pl + goff), d4u);
+                        if (HEUN != 1) {
+                            __stcg(reinterpret_cast<float4 *>(a.vo + goff), ov4);
+                            __stcg(reinterpret_cast<float4 *>(a.wo + goff), ow4);
                         }
+                        __stcg(reinterpret_cast<float4 *>(a.uo + goff), ou4);
+                        if (HEUN == 1) __stcg(reinterpret_cast<float4 *>(a.dso + goff), d4u);
                     } else {
                         const float fv[4] = {ov4.x, ov4.y, ov4.z, ov4.w};
                         const float fw[4] = {ow4.x, ow4.y, ow4.z, ow4.w};
                         const float fu[4] = {ou4.x, ou4.y, ou4.z, ou4.w};
-                        const float gv[4] = {d4v.x, d4v.y, d4v.z, d4v.w};
-                        const float gw[4] = {d4w.x, d4w.y, d4w.z, d4w.w};
                         const float gu[4] = {d4u.x, d4u.y, d4u.z, d4u.w};
 #pragma unroll
                         for (int m = 0; m < 4; ++m)
                             if (stored(j + m)) {
-                                __stcg(a.vo + goff + m, fv[m]);
-                                __stcg(a.wo + goff + m, fw[m]);
-                                __stcg(a.uo + goff + m, fu[m]);
-                                if (HEUN == 1) {
-                                    __stcg(a.dso + goff + m, gv[m]);
-                                    __stcg(a.dso + pl + goff + m, gw[m]);
-                                    __stcg(a.dso + 2 * pl + goff + m, gu[m]);
+                                if (HEUN != 1) {
+                                    __stcg(a.vo + goff + m, fv[m]);
+                                    __stcg(a.wo + goff + m, fw[m]);
                                 }
+                                __stcg(a.uo + goff + m, fu[m]);
+                                if (HEUN == 1) __stcg(a.dso + goff + m, gu[m]);
                             }
                     }
                 }
