@@ -148,16 +148,45 @@ def rasterize(rows: Sequence[np.ndarray], cols: Sequence[np.ndarray], shape: Seq
     return out, int(count.item())
 
 
+SEPARABLE_MAX_TAPS = 512
+
+
+def outer_factors(weights: np.ndarray):
+    """(ky, kx) float32 with ``weights[a][b]`` = ``ky[a] kx[b]`` up to the rounding of float32
+    weights, or None: the differences must add up to no more than 2^-22 of the weights' magnitudes,
+    which bounds what they change in a sum over ``weights`` by 2^-22 of the largest input (the direct
+    float32 sum's own rounding is larger)."""
+    w = np.asarray(weights, np.float64)
+    i, j = np.unravel_index(int(np.argmax(np.abs(w))), w.shape)
+    if not np.isfinite(w[i, j]) or w[i, j] == 0.0:
+        return None
+    kx = w[i, :] / w[i, j]
+    ky = w @ kx / (kx @ kx)  # least squares: averages the rounding of a row's weights
+    kx = ky @ w / (ky @ ky)
+    ky, kx = ky.astype(_F32), kx.astype(_F32)
+    off = np.abs(np.outer(ky.astype(np.float64), kx.astype(np.float64)) - w).sum()
+    return (ky, kx) if off <= 2.0 ** -22 * np.abs(w).sum() else None
+
+
 def blur_same(plane: torch.Tensor, weights: np.ndarray, one_minus: bool = False) -> torch.Tensor:
-    """scipy.signal.convolve2d(plane, weights, "same") in float32 (``fk_conv2d_same``), or
-    1 minus it."""
+    """scipy.signal.convolve2d(plane, weights, "same") in float32, or 1 minus it:
+    ``fk_conv2d_same``, or two one-dimensional passes (``fk_conv2d_separable``) for weights that
+    are an outer product, as a Gaussian's are."""
     H, W = int(plane.shape[0]), int(plane.shape[1])
     K = int(weights.shape[0])
     if weights.shape != (K, K):
         raise ValueError("the weights must be square")
     src = plane.to(torch.float32).contiguous()
-    k = torch.as_tensor(np.ascontiguousarray(weights, _F32), device=src.device)
     out = torch.empty((H, W), dtype=torch.float32, device=src.device)
+    # below about 8 taps the direct sum reads its inputs once and is the faster one
+    factors = outer_factors(weights) if 8 <= K <= SEPARABLE_MAX_TAPS and H <= 1 << 22 else None
+    if factors is not None:
+        k = torch.as_tensor(np.stack(factors), device=src.device)
+        tmp = torch.empty_like(out)
+        N.call("fk_conv2d_separable", src.data_ptr(), H, W, W, k[0].data_ptr(), k[1].data_ptr(), K,
+               tmp.data_ptr(), W, out.data_ptr(), W, int(bool(one_minus)), stream_handle())
+        return out
+    k = torch.as_tensor(np.ascontiguousarray(weights, _F32), device=src.device)
     N.call("fk_conv2d_same", src.data_ptr(), H, W, W, k.data_ptr(), K, out.data_ptr(), W,
            int(bool(one_minus)), stream_handle())
     return out

@@ -269,6 +269,13 @@ int fk_scar_raster(const double *xs, const double *ys, const int32_t *offsets, i
 int fk_conv2d_same(const float *in, int64_t H, int64_t W, int64_t in_pitch, const float *kernel,
                    int64_t K, float *out, int64_t out_pitch, int one_minus, void *stream);
 
+/* fk_conv2d_same for weights that are an outer product, kernel[a][b] = ky[a] kx[b] (1 <= K <= 512),
+ * as a pass along the rows into `tmp` (H rows of tmp_pitch floats, apart from `in` and `out`) and one
+ * along the columns. */
+int fk_conv2d_separable(const float *in, int64_t H, int64_t W, int64_t in_pitch, const float *ky,
+                        const float *kx, int64_t K, float *tmp, int64_t tmp_pitch, float *out,
+                        int64_t out_pitch, int one_minus, void *stream);
+
 /* ---- many tissues in one launch --------------------------------------------------------------
  * No reference counterpart: the reference steps one tissue per call (its data generation loops
  * over tissues in Python, deepx/generate.py:135-210).  Here every tissue of a batch advances in
