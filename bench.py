@@ -166,7 +166,8 @@ def run_batched(steps: int, reps: int, dev):
             "speedup_vs_plain_loop": tl / tb, "frac": gcups * BYTES_PER_UPDATE / peak,
             "depth": tune["depth"], "tile_rows": tune["tile_rows"],
             "interleave": tune["interleave"], "packed": tune["packed"],
-            "graph_steps": tune["graph_steps"],
+            "graph_steps": tune["graph_steps"], "resident": tune["resident"],
+            "resident_ms_per_step": tune["resident_ms_per_step"],
             "autotune_ms_per_step": {
                 f"d{k[0]}_rows{k[1]}_{('rr' + ('' if k[2][0] == 1 else f'x{k[2][0]}')) if k[2][0] else 'runs'}"
                 f"_{'pk' if k[2][1] else 'sc'}"

@@ -5,7 +5,8 @@ temporal-block depth (one Euler step per launch, or two: the blocked kernel), an
 the batched kernel's tile geometry (work items of 32 x 64 or 16 x 64 cells), work order (the
 CTAs deal the work list round-robin, or each takes a contiguous run of it) and arithmetic
 (scalar or packed two-cell FP32), each with every ``graph_steps`` (how many steps one captured
-CUDA graph replays), over a short run with CUDA events, and keeps the fastest.  Every
+CUDA graph replays), over a short run with CUDA events, and keeps the fastest; then, where the
+tissues fit on chip, whether sets of them run all steps in one launch instead.  Every
 combination gives the same bits.
 
 ``tune_tissue``: for one tissue, times every way of taking its Euler steps -- the tiled step
@@ -61,8 +62,10 @@ def tune_batch(batch: TissueBatch, trial_steps: int = 256, candidates=GRAPH_CAND
                depths=DEPTH_CANDIDATES, verbose: bool = False) -> dict:
     """Picks the depth, tile geometry, work order, arithmetic and ``graph_steps`` for ``batch``
     (set on it) and returns ``{"depth", "tile_rows", "interleave", "packed", "graph_steps",
-    "ms_per_step": {(depth, rows, (interleave, packed), graph_steps): ms}}``; the tissues'
-    states are restored.  Depth 2 is tried only when the batch can be blocked; its tiles are
+    "ms_per_step": {(depth, rows, (interleave, packed), graph_steps): ms}, "resident",
+    "resident_ms_per_step"}``; the tissues' states are restored.  ``resident``: whether
+    :meth:`TissueBatch.set_resident` is on as well, being faster than the best of them (its time
+    None where it does not apply).  Depth 2 is tried only when the batch can be blocked; its tiles are
     32 x 64 and it takes no work-order or arithmetic options."""
     depths = tuple(d for d in depths if d == 1 or batch.can_block())
     key = (_signature(batch), trial_steps, tuple(candidates), tuple(tile_rows), tuple(options),
@@ -70,6 +73,7 @@ def tune_batch(batch: TissueBatch, trial_steps: int = 256, candidates=GRAPH_CAND
     if key in _CACHE:
         res = _CACHE[key]
         _set_batch(batch, res["choice"])
+        batch.set_resident(res["resident"])
         return res
     saved = [(t.state.clone(), None if t.activation is None else
               (t.act_first.clone(), t.act_last.clone(), t.act_count.clone()))
@@ -78,9 +82,8 @@ def tune_batch(batch: TissueBatch, trial_steps: int = 256, candidates=GRAPH_CAND
     configs = [(1, rows, tuple(opt), g) for rows in tile_rows for opt in options
                for g in candidates]
     configs += [(d, 32, (1, False), g) for d in depths if d != 1 for g in candidates]
-    for cfg in configs:
-        depth, rows, opt, g = cfg
-        _set_batch(batch, cfg)
+
+    def timed(g) -> float:
         batch.advance(0, 2, graph_steps=0)  # warm-up
         if g:
             batch.advance(0, g, graph_steps=g)  # captures the graph outside the timing
@@ -91,20 +94,33 @@ def tune_batch(batch: TissueBatch, trial_steps: int = 256, candidates=GRAPH_CAND
         batch.advance(0, trial_steps, graph_steps=g)
         e1.record()
         torch.cuda.synchronize()
-        timings[cfg] = e0.elapsed_time(e1) / trial_steps
+        return e0.elapsed_time(e1) / trial_steps
+
+    for cfg in configs:
+        depth, rows, opt, g = cfg
+        _set_batch(batch, cfg)
+        timings[cfg] = timed(g)
         if verbose:
             print(f"autotune depth={depth} tile_rows={rows} interleave={opt[0]} "
                   f"packed={opt[1]} graph_steps={g}: {timings[cfg] * 1e3:.1f} us/step")
+    best = min(timings, key=timings.get)
+    _set_batch(batch, best)
+    resident_ms = None
+    if batch.set_resident(True):
+        batch.advance(0, trial_steps)  # warm-up: the kernel's attributes
+        resident_ms = timed(0)
+        if verbose:
+            print(f"autotune resident: {resident_ms * 1e3:.1f} us/step")
+    resident = batch.set_resident(resident_ms is not None and resident_ms < timings[best])
     for t, (st, act) in zip(batch.tissues, saved):
         t.state.copy_(st)
         if act is not None:
             t.act_first.copy_(act[0])
             t.act_last.copy_(act[1])
             t.act_count.copy_(act[2])
-    best = min(timings, key=timings.get)
-    _set_batch(batch, best)
     res = {"choice": best, "depth": best[0], "tile_rows": best[1], "interleave": best[2][0],
-           "packed": best[2][1], "graph_steps": best[3], "ms_per_step": timings}
+           "packed": best[2][1], "graph_steps": best[3], "ms_per_step": timings,
+           "resident": resident, "resident_ms_per_step": resident_ms}
     _CACHE[key] = res
     return res
 

@@ -90,6 +90,17 @@ class TissueBatch:
         self.tile_rows = int(rows)
         return self
 
+    def set_resident(self, on: bool) -> bool:
+        """Whether calls of many steps keep sets of tissues on chip and run all steps of a set in
+        one launch; same results.  On from the start where every tissue can take it (16 x 16 to
+        about 1240 x 1240 cells, no activation tracking); the settings above are of the kernel
+        that takes one or two steps per launch and turn it off.  Returns whether it is on now."""
+        if on and N.lib().fk_batch_set_resident(self._plan, 1) != 0:
+            return False
+        if not on:
+            N.call("fk_batch_set_resident", self._plan, 0)
+        return bool(on)
+
     @property
     def cells(self) -> int:
         return sum(t.H * t.W for t in self.tissues)

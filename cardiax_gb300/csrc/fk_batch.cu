@@ -10,12 +10,14 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <new>
 #include <numeric>
 #include <vector>
 
 #include "../../include/cardiax_gb300.h"
 #include "fk_capi_internal.h"
+#include "fk_resident.cuh"
 #include "fk_step.cuh"
 #include "fk_tb.cuh"
 
@@ -40,7 +42,32 @@ const TileShape kShape[kShapes] = {{32, 64, 2, fk_batch_launch_rows32},
                                    {16, 64, 2, fk_batch_launch_rows16}};
 }  // namespace
 
+// One launch of the resident kernel: some of the batch's tissues, for all steps of a call.
+struct ResWave {
+    int rows = 0, threads = 0, ctas = 0;
+    size_t smem = 0;
+    double cost = 0.0;           // estimated us per step
+    int first = 0;               // its tissues' place in the device table
+    std::vector<int> tissue;
+    std::vector<ResPlan> plan;   // of each
+    ResidentArgs args{};
+};
+struct ResWaves {
+    std::vector<ResWave> w;
+    double cost = 0.0;           // us per step of all tissues
+    size_t xchg_bytes = 0;
+    bool ok() const { return !w.empty(); }
+};
+
 struct fk_batch {
+    // the resident kernel in place of one launch per step (fk_batch_set_resident; turned off by the
+    // knobs of the stepping kernel)
+    ResWaves res;
+    bool resident = false;
+    ResTissue *d_res = nullptr;
+    uint64_t *d_xchg = nullptr;
+    std::vector<ResTissue> h_res;
+    int64_t cells = 0;
     int n = 0, grid = 0, device = -1;
     int shape = 0;  // index into kShape of the tile geometry in use
     // work order (0: contiguous runs; k = 1, 2, 4, 8: round-robin in chunks of k items) and
@@ -88,10 +115,10 @@ int64_t tiles_of(const fk_grid &g, int shape) {
 }
 
 struct Layout {
-    size_t maps[kShapes], tbmaps, tissues, items[kShapes], ranges[kShapes], t, total;
+    size_t maps[kShapes], tbmaps, tissues, items[kShapes], ranges[kShapes], t, res, xchg, total;
 };
 
-Layout layout(int n, const int64_t *n_items) {
+Layout layout(int n, const int64_t *n_items, const ResWaves &res) {
     Layout L;
     size_t at = 0;
     for (int k = 0; k < kShapes; ++k) {
@@ -109,9 +136,139 @@ Layout layout(int n, const int64_t *n_items) {
         at = align_up(at + sizeof(int) * (kBatchMaxGrid + 1));
     }
     L.t = at;
-    L.total = align_up(at + 16);
+    at = align_up(at + 16);
+    L.res = at;
+    if (res.ok()) at = align_up(at + sizeof(ResTissue) * n);
+    L.xchg = at;
+    L.total = align_up(at + (res.ok() ? res.xchg_bytes : 0));
     return L;
 }
+
+// ---- the resident kernel's launches ------------------------------------------------------------------
+// The tissues of a batch are independent, so any set of them that fits on chip together can run all
+// steps of a call in one launch before the next set starts: 48 mixed tissues (5.9 M cells), 64 steps:
+// 45.6 us per step in the batched kernel (143 GCUPS: 40 % of its items are edge tiles, each loaded and
+// stored every step), 36.9 in such launches (34.8 over 256 steps; a launch also loads and stores all).
+constexpr int kResMaxTissues = 4096, kResMaxWaves = 64;
+
+ResClass res_class(const fk_tissue &t) {
+    ResClass c;
+    std::memset(&c, 0, sizeof c);
+    c.m = make_model(t.params);
+    c.dt = (float)t.dt;
+    c.rdx = 1.0f / (float)t.dx;
+    return c;
+}
+
+// The launches with `R` rows per thread, largest tissues first, each into the first launch with room.
+ResWaves plan_waves_rows(const fk_tissue *ts, int n, int ctas, int R) {
+    ResWaves out;
+    // by shape: the best plan of at most 0, 1, .. ctas tiles (the cost falls with the tiles)
+    std::map<std::pair<int64_t, int64_t>, std::vector<ResPlan>> made;
+    std::vector<const std::vector<ResPlan> *> plans(n);
+    std::vector<ResPlan> plan(n);
+    for (int k = 0; k < n; ++k) {
+        const fk_grid &g = ts[k].g;
+        std::vector<ResPlan> &p = made[{g.H, g.W}];
+        if (p.empty()) resident_plans(g.H, g.W, ctas, R, p);
+        if (!p[ctas].ok()) return out;
+        int t = 0;
+        while (!p[t].ok()) ++t;
+        plans[k] = &p;
+        plan[k] = p[t];
+    }
+    std::vector<int> order(n);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return plan[x].tiles > plan[y].tiles; });
+    std::vector<ResWave> w;
+    std::vector<std::vector<int>> cls_of;  // per launch and tissue: its class
+    for (int k : order) {
+        const ResClass c = res_class(ts[k]);
+        size_t q = 0;
+        for (;; ++q) {
+            if (q == w.size()) {
+                if ((int)q == kResMaxWaves) return out;
+                w.emplace_back();
+                cls_of.emplace_back();
+            }
+            ResWave &x = w[q];
+            if (x.ctas + plan[k].tiles > ctas) continue;
+            int id = 0;
+            for (; id < x.args.n_out; ++id)  // n_out counts the classes while planning
+                if (std::memcmp(&x.args.cls[id], &c, sizeof c) == 0) break;
+            if (id == kResMaxClasses) continue;
+            if (id == x.args.n_out) x.args.cls[x.args.n_out++] = c;
+            x.ctas += (int)plan[k].tiles;
+            x.tissue.push_back(k);
+            cls_of[q].push_back(id);
+            break;
+        }
+    }
+    int at = 0;
+    for (size_t q = 0; q < w.size(); ++q) {
+        ResWave &x = w[q];
+        // blocks left over go to the tissue that takes longest, while that helps
+        for (int left = ctas - x.ctas; left > 0;) {
+            int worst = x.tissue[0];
+            for (int k : x.tissue)
+                if (plan[k].cost > plan[worst].cost) worst = k;
+            const int tiles = (int)plan[worst].tiles;
+            int t = tiles;
+            while (t < tiles + left && !((*plans[worst])[t].cost < plan[worst].cost)) ++t;
+            const ResPlan &better = (*plans[worst])[t];
+            if (!(better.cost < plan[worst].cost)) break;
+            left -= t - tiles;
+            plan[worst] = better;
+        }
+        x.rows = R;
+        x.first = at;
+        x.args.n_out = 0;
+        x.ctas = 0;
+        for (size_t i = 0; i < x.tissue.size(); ++i) {
+            const ResPlan &p = plan[x.tissue[i]];
+            x.plan.push_back(p);
+            for (int t = 0; t < p.tiles; ++t)
+                x.args.cta[x.ctas + t] = (uint32_t)i << 8 | (uint32_t)cls_of[q][i];
+            x.ctas += (int)p.tiles;
+            x.threads = std::max(x.threads, p.threads);
+            x.args.max_q = std::max(x.args.max_q, p.max_q);
+            x.args.max_g = std::max(x.args.max_g, p.max_g);
+            x.cost = std::max(x.cost, p.cost);
+        }
+        for (int k : x.tissue) x.args.su = std::max(x.args.su, plan[k].su_w * plan[k].su_h);
+        // (threads and u buffers may come from different tissues: their sum need not fit)
+        x.smem = resident_smem(R, x.threads, x.args.su);
+        if (x.smem > kResMaxSmem) return ResWaves();
+        x.args.slot = 2 * 16 * (int64_t)x.args.max_q + 2 * 4 * (int64_t)x.args.max_g * R;
+        out.xchg_bytes = std::max(out.xchg_bytes, (size_t)(x.ctas * 2 * x.args.slot) * 8);
+        out.cost += x.cost;
+        at += (int)x.tissue.size();
+    }
+    out.w = std::move(w);
+    return out;
+}
+
+ResWaves plan_waves(const fk_tissue *ts, int n) {
+    ResWaves best;
+    const int ctas = resident_ctas();
+    if (ctas < 2 || n > kResMaxTissues) return best;
+    int64_t cells = 0;
+    for (int k = 0; k < n; ++k) {
+        if (check_grid(ts[k].g) || ts[k].act.last || ts[k].n_stimuli > kMaxStim) return best;
+        cells += ts[k].g.H * ts[k].g.W;
+    }
+    if (cells > (int64_t)kResMaxWaves * ctas * 512 * 4 * kResMaxRows) return best;
+    for (int R = kResMinRows; R <= kResMaxRows; ++R) {
+        ResWaves w = plan_waves_rows(ts, n, ctas, R);
+        if (w.ok() && (!best.ok() || w.cost < best.cost)) best = std::move(w);
+    }
+    return best;
+}
+
+// us of n steps: the resident launches (a launch's fixed cost is 15 to 30 us), and one launch per
+// step (4.4 us at least, about 140 GCUPS on mixed tissues).
+double res_time(const ResWaves &r, int64_t n) { return (double)r.w.size() * 30.0 + r.cost * (double)n; }
+double step_time(int64_t cells, int64_t n) { return std::max(4.4, (double)cells / 140e3) * (double)n; }
 
 // Relative cost of an edge tile (clamped halo, one-sided rows, bounds checks) against an
 // interior one, for balancing the CTAs' runs of the work list.
@@ -201,6 +358,81 @@ void release_graph(fk_batch *b) {
     b->graph_steps = 0;
 }
 
+// The device table of the resident launches: per tissue its arguments (state to state), its plan and
+// its place.
+void fill_resident(fk_batch *b) {
+    b->h_res.resize(b->n);
+    for (const ResWave &w : b->res.w) {
+        int block = 0;
+        for (size_t i = 0; i < w.tissue.size(); ++i) {
+            const int k = w.tissue[i];
+            const ResPlan &p = w.plan[i];
+            ResTissue &t = b->h_res[w.first + (int)i];
+            std::memset(&t, 0, sizeof t);
+            t.args = b->h_tissues[k].args[0];
+            const int64_t plane = b->grids[k].H * b->grids[k].pitch;
+            t.args.vo = const_cast<float *>(t.args.v);
+            t.args.wo = t.args.vo + plane;
+            t.args.uo = t.args.vo + 2 * plane;
+            t.nr = p.nr;
+            t.nc = p.nc;
+            t.ng = p.ng;
+            t.nq = p.nq;
+            t.su_w = p.su_w;
+            t.first = block;
+            t.id = k;
+            block += (int)p.tiles;
+        }
+    }
+}
+
+// n steps from t0 of every tissue through the resident launches: in place; or, n at most kResMaxSteps,
+// writing every state x_{t0+s}, s = 1 .. n, of tissue k to base + k * stride + s * every and leaving the
+// tissues' own as they were.
+struct ResOut {
+    float *base = nullptr;
+    int64_t stride = 0, every = 0;
+};
+int run_resident(const fk_batch *b, int64_t t0, int64_t n, const ResOut &out, cudaStream_t s) {
+    for (const ResWave &w : b->res.w) {
+        ResidentArgs ra = w.args;
+        ra.xchg = b->d_xchg;
+        ra.tissues = b->d_res + w.first;
+        ra.base = out.base;
+        ra.tissue_stride = out.stride;
+        ra.every = out.every;
+        StepArgs a{};  // the constants of the launch come from its classes
+        a.m = ra.cls[0].m;
+        a.dt = ra.cls[0].dt;
+        a.rdx = ra.cls[0].rdx;
+        for (int64_t done = 0; done < n;) {
+            const int64_t c = std::min<int64_t>(n - done, n - done == kResMaxSteps + 1 ? kResMaxSteps - 1
+                                                                                      : kResMaxSteps);
+            ra.t0 = t0 + done;
+            ra.n = (int)c;
+            ra.n_out = 1;
+            ra.out_step[0] = (int)c;
+            ra.out_off[0] = 0;
+            if (cudaMemsetAsync(b->d_xchg, 0, (size_t)(w.ctas * 2 * ra.slot) * 8, s) != cudaSuccess ||
+                launch_resident(w.rows, w.ctas, w.threads, w.smem, ra, a, s) != cudaSuccess)
+                return FK_ERR_CUDA;
+            done += c;
+        }
+    }
+    return FK_OK;
+}
+
+// Whether the tissues all lie on one grid; *ns: floats of a state.
+bool one_grid(const fk_batch *b, int64_t *ns) {
+    const StepArgs &a0 = b->h_tissues[0].args[0];
+    for (int e = 1; e < b->n; ++e) {
+        const StepArgs &a = b->h_tissues[e].args[0];
+        if (a.H != a0.H || a.W != a0.W || a.pitch != a0.pitch) return false;
+    }
+    *ns = 3 * (int64_t)a0.H * a0.pitch;
+    return true;
+}
+
 }  // namespace
 
 extern "C" {
@@ -210,7 +442,7 @@ size_t fk_batch_workspace_bytes(const fk_tissue *tissues, int n) {
     int64_t items[kShapes] = {};
     for (int k = 0; k < n; ++k)
         for (int q = 0; q < kShapes; ++q) items[q] += tiles_of(tissues[k].g, q);
-    return layout(n, items).total;
+    return layout(n, items, plan_waves(tissues, n)).total;
 }
 
 int fk_batch_create(const fk_tissue *tissues, int n, void *workspace, size_t bytes, void *stream,
@@ -236,7 +468,12 @@ int fk_batch_create(const fk_tissue *tissues, int n, void *workspace, size_t byt
     if (any_act && !all_act) return FK_ERR_ARGUMENT;  // tracking is all or nothing per batch
     for (int q = 0; q < kShapes; ++q)
         if (n_items[q] > (int64_t(1) << 30)) return FK_ERR_SHAPE;
-    const Layout L = layout(n, n_items);
+    ResWaves res = plan_waves(tissues, n);
+    Layout L = layout(n, n_items, res);
+    if (bytes < L.total && res.ok()) {  // a workspace of the stepping kernel alone will do
+        res = ResWaves();
+        L = layout(n, n_items, res);
+    }
     if (bytes < L.total) return FK_ERR_ARGUMENT;
 
     fk_batch *b = new (std::nothrow) fk_batch();
@@ -260,6 +497,11 @@ int fk_batch_create(const fk_tissue *tissues, int n, void *workspace, size_t byt
     b->tb_ok = !any_act;
     for (int k = 0; k < n; ++k) b->tb_ok &= tb_batchable(tissues[k].g.H, tissues[k].g.W);
     b->d_t = reinterpret_cast<int *>(ws + L.t);
+    b->res = std::move(res);
+    b->resident = b->res.ok();
+    b->d_res = reinterpret_cast<ResTissue *>(ws + L.res);
+    b->d_xchg = reinterpret_cast<uint64_t *>(ws + L.xchg);
+    for (int k = 0; k < n; ++k) b->cells += tissues[k].g.H * tissues[k].g.W;
     b->h_tissues.resize(n);
     for (int q = 0; q < kShapes; ++q) {
         fk_batch::PerShape &P = b->sp[q];
@@ -358,9 +600,13 @@ int fk_batch_create(const fk_tissue *tissues, int n, void *workspace, size_t byt
     b->grids.resize(n);
     for (int k = 0; k < n; ++k) b->grids[k] = tissues[k].g;
     for (int q = 0; q < kShapes; ++q) build_items(b, q);
+    if (b->res.ok()) fill_resident(b);
     cudaStream_t s = (cudaStream_t)stream;
     bool ok = cudaMemcpyAsync(b->d_tissues, b->h_tissues.data(), sizeof(BatchTissue) * n,
                               cudaMemcpyHostToDevice, s) == cudaSuccess;
+    if (ok && b->res.ok())
+        ok = cudaMemcpyAsync(b->d_res, b->h_res.data(), sizeof(ResTissue) * n, cudaMemcpyHostToDevice,
+                             s) == cudaSuccess;
     if (ok && b->tb_ok)
         ok = cudaMemcpyAsync(b->d_tbmaps, b->h_tbmaps.data(), sizeof(BatchTbMaps) * n,
                              cudaMemcpyHostToDevice, s) == cudaSuccess;
@@ -381,9 +627,17 @@ int fk_batch_create(const fk_tissue *tissues, int n, void *workspace, size_t byt
     return FK_OK;
 }
 
+int fk_batch_set_resident(fk_batch *b, int on) {
+    if (!b) return FK_ERR_NULL;
+    if (on && !b->res.ok()) return FK_ERR_ARGUMENT;
+    b->resident = on != 0;
+    return FK_OK;
+}
+
 int fk_batch_set_grid(fk_batch *b, int ctas) {
     if (!b) return FK_ERR_NULL;
     if (ctas < 1 || ctas > kBatchMaxGrid) return FK_ERR_ARGUMENT;
+    b->resident = false;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev != b->device) return FK_ERR_CUDA;
     // ordered after the plan's earlier work; the host copies stay alive in the plan
@@ -413,6 +667,7 @@ int fk_batch_set_options(fk_batch *b, int interleave, int packed) {
     if (interleave != 0 && interleave != 1 && interleave != 2 && interleave != 4 &&
         interleave != 8)
         return FK_ERR_ARGUMENT;
+    b->resident = false;
     const int il = interleave, pk = packed ? 1 : 0;
     if (il != b->interleave || pk != b->packed) release_graph(b);
     b->packed = pk;
@@ -438,6 +693,7 @@ int fk_batch_set_depth(fk_batch *b, int depth) {
     if (!b) return FK_ERR_NULL;
     if (depth != 1 && depth != kBatchTbDepth) return FK_ERR_ARGUMENT;
     if (depth != 1 && !b->tb_ok) return FK_ERR_ARGUMENT;
+    b->resident = false;
     if (depth != b->depth) release_graph(b);
     b->depth = depth;
     return FK_OK;
@@ -448,6 +704,7 @@ int fk_batch_set_tile_rows(fk_batch *b, int rows) {
     for (int q = 0; q < kShapes; ++q)
         if (kShape[q].rows == rows) {
             if (b->shape != q) release_graph(b);
+            b->resident = false;
             b->shape = q;
             return FK_OK;
         }
@@ -530,6 +787,9 @@ int fk_batch_forward_euler(fk_batch *b, int64_t t0, int64_t t1, int graph_steps,
     cudaStream_t s = (cudaStream_t)stream;
     int64_t n = t1 - t0;
     if (n == 0) return FK_OK;
+    // (two steps at least: in place, a block may write its cells only after its neighbours' first loads)
+    if (b->resident && n >= 2 && res_time(b->res, n) < step_time(b->cells, n))
+        return run_resident(b, t0, n, ResOut{}, s);
     set_int_kernel<<<1, 1, 0, s>>>(b->d_t, (int)t0);
     if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
     // the smem attribute must be set outside any capture: one plain (empty-range) call does it
@@ -580,19 +840,23 @@ int fk_batch_recompute(fk_batch *b, int64_t s, int64_t n, float *bufs, int64_t e
     if (!b || !bufs) return FK_ERR_NULL;
     if (n < 1 || s < -(int64_t(1) << 24) || s + n > (int64_t(1) << 24)) return FK_ERR_ARGUMENT;
     if (b->act) return FK_ERR_ARGUMENT;  // recomputed steps must not record activations again
-    const StepArgs &a0 = b->h_tissues[0].args[0];
-    for (int e = 1; e < b->n; ++e) {
-        const StepArgs &a = b->h_tissues[e].args[0];
-        if (a.H != a0.H || a.W != a0.W || a.pitch != a0.pitch) return FK_ERR_SHAPE;
-    }
-    const int64_t ns = 3 * (int64_t)a0.H * a0.pitch;
+    int64_t ns = 0;
+    if (!one_grid(b, &ns)) return FK_ERR_SHAPE;
     if (exp_stride < n * ns || (reinterpret_cast<uintptr_t>(bufs) & 15u) || (exp_stride & 3))
         return FK_ERR_ALIGN;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev != b->device) return FK_ERR_CUDA;
     cudaStream_t cs = (cudaStream_t)stream;
-    set_int_kernel<<<1, 1, 0, cs>>>(b->d_t, (int)s);
     const dim3 cgrid(64, b->n);
+    // (a step outside the resident kernel also copies its states out: 12 bytes per cell read and
+    // written, at about 4 TB/s from L2)
+    if (b->resident && n - 1 >= 2 && n - 1 <= kResMaxSteps &&
+        res_time(b->res, n - 1) < step_time(b->cells, n - 1) + (double)(n - 1) * (2.0 + (double)b->cells / 170e3)) {
+        batch_state_out_kernel<<<cgrid, 256, 0, cs>>>(b->d_tissues, 0, bufs, exp_stride, ns);
+        if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
+        return run_resident(b, s, n - 1, ResOut{bufs, exp_stride, ns}, cs);
+    }
+    set_int_kernel<<<1, 1, 0, cs>>>(b->d_t, (int)s);
     batch_state_out_kernel<<<cgrid, 256, 0, cs>>>(b->d_tissues, 0, bufs, exp_stride, ns);
     if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
     for (int64_t k = 1; k < n; ++k) {

@@ -438,22 +438,13 @@ int flow_run(const fk_grid &g, const float *src, float *dst, float *scratch, con
 
 // ---- resident stepping --------------------------------------------------------------------------
 // Calls of fewer steps take one launch per step.  The resident kernel's fixed cost (clearing the
-// strips, loading the state, the cooperative launch) is 13 us at 64^2 and 30 at 1200^2, against
-// 4.4 and 9.7 us per single-step launch: at 6 steps 26.7 against 33.9 us (64^2), 31.0 against 32.8
-// (512^2), 76.9 against 82.5 (1200^2).
+// strips, loading the state, the cooperative launch) is 12 us at 64^2 and 26 at 1200^2, against
+// 4.4 and 9.7 us per single-step launch: at 6 steps 24.1 against 35.4 us (64^2), 28.0 against 33.1
+// (512^2), 64.9 against 82.2 (1200^2).
 constexpr int64_t kResidentMinSteps = 6;
 
-// Steps t0 .. t0+n-1 of `n_exp` tissues from `in` through the resident kernel, states written to
-// `base` + offset after the steps listed in `outs` ((step, offset) pairs in step order, the last one
-// at step n), or with `every` after each step s to base + s * every.  `exps`: see launch_resident;
-// `tmp` (one state) holds the state between launches that end at no listed step (one tissue only).
-static int resident_run(const ResPlan &plan, const fk_grid &g, const float *in, float *base,
-                        const std::vector<std::pair<int64_t, int64_t>> &outs, int64_t every,
-                        float *tmp, const float *D, const Model &m, const Stim *st, int ns,
-                        int64_t t0, int64_t n, float dt, float rdx, const fk_activation *act,
-                        const StepArgs *exps, void *workspace, int *status, cudaStream_t s) {
-    StepArgs a;
-    ResidentArgs ra{};
+// The plan's part of a launch's arguments.
+static void resident_args(ResidentArgs &ra, const ResPlan &plan, void *workspace) {
     ra.nr = plan.nr;
     ra.nc = plan.nc;
     ra.ng = plan.ng;
@@ -461,10 +452,21 @@ static int resident_run(const ResPlan &plan, const fk_grid &g, const float *in, 
     ra.max_q = plan.max_q;
     ra.max_g = plan.max_g;
     ra.su_w = plan.su_w;
-    ra.su_h = plan.su_h;
+    ra.su = plan.su_w * plan.su_h;
     ra.slot = plan.slot;
     ra.xchg = static_cast<uint64_t *>(workspace);
-    ra.every = every;
+}
+
+// Steps t0 .. t0+n-1 from `in` through the resident kernel, states written to `base` + offset after the
+// steps listed in `outs` ((step, offset) pairs in step order, the last one at step n); `tmp` (one state)
+// holds the state between launches that end at no listed step.
+static int resident_run(const ResPlan &plan, const fk_grid &g, const float *in, float *base,
+                        const std::vector<std::pair<int64_t, int64_t>> &outs, float *tmp, const float *D,
+                        const Model &m, const Stim *st, int ns, int64_t t0, int64_t n, float dt, float rdx,
+                        const fk_activation *act, void *workspace, int *status, cudaStream_t s) {
+    StepArgs a;
+    ResidentArgs ra{};
+    resident_args(ra, plan, workspace);
     size_t k = 0;
     for (int64_t done = 0; done < n;) {
         int64_t c = n - done < kResMaxSteps ? n - done : kResMaxSteps;
@@ -472,25 +474,23 @@ static int resident_run(const ResPlan &plan, const fk_grid &g, const float *in, 
         a.vo = base;
         ra.t0 = t0 + done;
         ra.n_out = 0;
-        if (!every) {
-            for (; k < outs.size() && outs[k].first <= done + c; ++k) {
-                if (ra.n_out == kResMaxOut - 1) {  // the rest in the next launch
-                    c = ra.out_step[ra.n_out - 1];
-                    break;
-                }
-                ra.out_step[ra.n_out] = (int)(outs[k].first - done);
-                ra.out_off[ra.n_out++] = outs[k].second;
-                in = base + outs[k].second;
+        for (; k < outs.size() && outs[k].first <= done + c; ++k) {
+            if (ra.n_out == kResMaxOut - 1) {  // the rest in the next launch
+                c = ra.out_step[ra.n_out - 1];
+                break;
             }
-            if (ra.n_out == 0 || ra.out_step[ra.n_out - 1] != c) {
-                ra.out_step[ra.n_out] = (int)c;
-                ra.out_off[ra.n_out++] = tmp - base;
-                in = tmp;
-            }
+            ra.out_step[ra.n_out] = (int)(outs[k].first - done);
+            ra.out_off[ra.n_out++] = outs[k].second;
+            in = base + outs[k].second;
+        }
+        if (ra.n_out == 0 || ra.out_step[ra.n_out - 1] != c) {
+            ra.out_step[ra.n_out] = (int)c;
+            ra.out_off[ra.n_out++] = tmp - base;
+            in = tmp;
         }
         ra.n = (int)c;
         if (cudaMemsetAsync(workspace, 0, plan.workspace(), s) != cudaSuccess ||
-            launch_resident(plan, ra, a, exps, s) != cudaSuccess)
+            launch_resident(plan.rows, (int)plan.tiles, plan.threads, plan.smem, ra, a, s) != cudaSuccess)
             return FK_ERR_CUDA;
         done += c;
     }
@@ -667,7 +667,7 @@ int fk_forward_euler_tracked(fk_grid g, float *state, float *scratch, const floa
 
 size_t fk_resident_workspace_bytes(fk_grid g) {
     if (check_grid(g)) return 0;
-    const ResPlan plan = resident_plan(g.H, g.W, 1);
+    const ResPlan plan = resident_plan(g.H, g.W);
     return plan.ok() ? plan.workspace() : 0;
 }
 
@@ -677,7 +677,7 @@ static bool takes_resident(const fk_grid &g, int64_t n, int n_stimuli, const voi
     if (!workspace || n < kResidentMinSteps || n_stimuli > kMaxStim || g_step_kernel != 0 ||
         !aligned16(workspace))
         return false;
-    plan = resident_plan(g.H, g.W, 1);
+    plan = resident_plan(g.H, g.W);
     return plan.ok() && bytes >= plan.workspace();
 }
 
@@ -702,8 +702,8 @@ int fk_forward_euler_resident(fk_grid g, float *state, float *scratch, const flo
     int *status = status_ptr();
     if (!status) return FK_ERR_CUDA;
     const int64_t n = t1 - t0;
-    return resident_run(plan, g, state, state, {{n, 0}}, 0, scratch, D, make_model(*p), st,
-                        n_stimuli, t0, n, (float)dt, 1.0f / (float)dx, act, nullptr, workspace,
+    return resident_run(plan, g, state, state, {{n, 0}}, scratch, D, make_model(*p), st,
+                        n_stimuli, t0, n, (float)dt, 1.0f / (float)dx, act, workspace,
                         status, (cudaStream_t)stream);
 }
 
@@ -992,8 +992,8 @@ int fk_forward_resident(fk_grid g, const float *state0, float *scratch, const fl
     for (int i = 0; i + 1 < n_checkpoints; ++i)
         if (checkpoints[i + 1] > checkpoints[i])
             outs.push_back({checkpoints[i + 1] - t0, i * n_state});
-    if ((rc = resident_run(plan, g, state0, out, outs, 0, scratch, D, make_model(*p), st, n_stimuli,
-                           t0, n, (float)dt, 1.0f / (float)dx, nullptr, nullptr, workspace, status,
+    if ((rc = resident_run(plan, g, state0, out, outs, scratch, D, make_model(*p), st, n_stimuli,
+                           t0, n, (float)dt, 1.0f / (float)dx, nullptr, workspace, status,
                            s)))
         return rc;
     const float *cur = state0;

@@ -8,8 +8,8 @@
 // updates its cells; then the cells within 4 of a tile side go to the neighbour through global
 // memory.  Only u is exchanged, only with the 4 direct neighbours: no stencil is diagonal.
 //
-// What bounds it (us per step, GB300; one launch per step before): 256^2 2.08 (4.4), 512^2 2.48
-// (4.5), 1024^2 5.5 (8.2), 1200^2 6.4 (9.7).  One launch per step pays launch, load and store
+// What bounds it (us per step, GB300; one launch per step before): 256^2 2.00 (4.4), 512^2 2.43
+// (4.5), 1024^2 5.67 (8.2), 1200^2 6.49 (9.7).  One launch per step pays launch, load and store
 // latencies in a row whatever it computes.  Here a small grid's step is one dependent chain: about
 // 1000 cycles for a unit of 8 cells (1600 at the grid's edge), 1700 from a strip's store to its
 // neighbour's load of it through L2, and two barriers.  A large grid's step is bound by issue
@@ -29,6 +29,9 @@
 // Every wait is bounded (1 s); a tile whose wait runs out reports it and leaves, its neighbours'
 // waits then run out as well.  The launch is cooperative, so all tiles run at the same time, and
 // takes at most kResMaxSteps steps.
+//
+// Several tissues (MANY): each CTA finds its tissue in a table and takes that tissue's plan, constants
+// and buffers; the tissues of a launch share rows per thread and CTA size and nothing else.
 //
 // Per cell these are the operations of the step kernel in the same order (fk_pack.cuh): the same
 // bits.
@@ -76,15 +79,13 @@ __device__ __forceinline__ bool wait_quad(const uint64_t *p, uint32_t tag, float
     }
 }
 
-// The first slope (scaled) of a plane at (i, j) along rows (AXIS 0) or columns, edge-padded.
-template <int AXIS>
-__device__ __forceinline__ float slope_at(const Clamped &D, int i, int j, float rdx) {
-    const int x = AXIS == 0 ? i : j, N = AXIS == 0 ? D.H : D.W;
-    auto at = [&](int y) { return AXIS == 0 ? D.at(y, j) : D.at(i, y); };
+// The first slope (scaled) at cell x of a line of N cells, p its place in an edge-padded tile with
+// `stride` floats from one cell of the line to the next.
+__device__ __forceinline__ float slope(const float *p, int stride, int x, int N, float rdx) {
     float s;
-    if (x == 0) s = g_head(at(0), at(1), at(2), at(3));
-    else if (x == N - 1) s = g_tail(at(x - 3), at(x - 2), at(x - 1), at(x));
-    else s = g_central(at(x - 2), at(x - 1), at(x + 1), at(x + 2));
+    if (x == 0) s = g_head(p[0], p[stride], p[2 * stride], p[3 * stride]);
+    else if (x == N - 1) s = g_tail(p[-3 * stride], p[-2 * stride], p[-stride], p[0]);
+    else s = g_central(p[-2 * stride], p[-stride], p[stride], p[2 * stride]);
     return s * rdx;
 }
 
@@ -132,15 +133,22 @@ struct Unit {
     bool left, right, top, bottom;
 };
 
+// The tissue's constants: of the launch's one tissue, or of this block's class.
+struct Consts {
+    const Model &m;
+    float rdx, dt;
+    float2 rdx2, dt2;  // each twice
+};
+
 // One step of a unit: reads u around it at `c` (its first cell in the current buffer), writes the
 // new u to `dst` (the same place in the next one) and updates v and w in place.
 template <int R, bool ACT>
-__device__ __forceinline__ void step_unit(const StepArgs &a, const StepArgs &a0, const PackConsts &kc,
+__device__ __forceinline__ void step_unit(const StepArgs &a, const Consts &tc, const PackConsts &kc,
                                           const Unit &un, const float *c, float *dst, int SUW,
                                           const float4 *sD, int nthr, float4 (&v)[R],
                                           float4 (&w)[R], unsigned active, float t) {
-    const int H = a0.H, W = a0.W;
-    const float rdx = a0.rdx;
+    const int H = a.H, W = a.W;
+    const float rdx = tc.rdx;
     const int i0 = un.i0, j = un.j;
     // u rows -4+q and u_x rows -2+q of this quad, relative to its first row, taken as needed
     Quad U[R + 8], X[R + 4];
@@ -154,7 +162,7 @@ __device__ __forceinline__ void step_unit(const StepArgs &a, const StepArgs &a0,
             if (i0 - 2 + q <= 0) X[q] = q_head(kc, U[q + 2], U[q + 3], U[q + 4], U[q + 5]);
         if ((q == R + 1 || q == R + 2 || (R == 2 && q == R + 3)) && un.bottom)
             if (i0 - 2 + q >= H - 1) X[q] = q_tail(kc, U[q >= 1 ? q - 1 : 0], U[q], U[q + 1], U[q + 2]);
-        X[q] = q_scale(X[q], kc.rdx);
+        X[q] = q_scale(X[q], tc.rdx2);
     };
 #pragma unroll
     for (int q = 0; q < 8; ++q) take_u(q);
@@ -168,12 +176,12 @@ __device__ __forceinline__ void step_unit(const StepArgs &a, const StepArgs &a0,
         Quad uxx = q_central(kc, X[k], X[k + 1], X[k + 3], X[k + 4]);
         if (k == 0 && un.top)
             if (i == 0) {  // u_x row 3 is not taken yet
-                const Quad x3 = q_scale(q_central(kc, U[5], U[6], U[8], ld_quad(c + 5 * SUW)), kc.rdx);
+                const Quad x3 = q_scale(q_central(kc, U[5], U[6], U[8], ld_quad(c + 5 * SUW)), tc.rdx2);
                 uxx = q_head(kc, X[2], X[3], X[4], x3);
             }
         if (k == R - 1 && un.bottom)
             if (i == H - 1) uxx = q_tail(kc, X[k >= 1 ? k - 1 : 0], X[k], X[k + 1], X[k + 2]);
-        uxx = q_scale(uxx, kc.rdx);
+        uxx = q_scale(uxx, tc.rdx2);
         const Quad uc = U[k + 4];
         const float4 el = ld4(c + k * SUW - 4), er = ld4(c + k * SUW + 4);
         const float e[12] = {el.x,    el.y,    el.z, el.w, uc.lo.x, uc.lo.y,
@@ -200,7 +208,7 @@ __device__ __forceinline__ void step_unit(const StepArgs &a, const StepArgs &a0,
             }
         }
 #pragma unroll
-        for (int m = 0; m < 4; ++m) y[m] = p_mul(y[m], kc.rdx);
+        for (int m = 0; m < 4; ++m) y[m] = p_mul(y[m], tc.rdx2);
         float2 yy_lo = pg_central_row(kc, y[0].x, y[0].y, y[1].x, y[1].y, y[2].x, y[2].y);
         float2 yy_hi = pg_central_row(kc, y[1].x, y[1].y, y[2].x, y[2].y, y[3].x, y[3].y);
         if (un.left) yy_lo.x = pick(j == 0, g_head(y[1].x, y[1].y, y[2].x, y[2].y), yy_lo.x);
@@ -213,17 +221,17 @@ __device__ __forceinline__ void step_unit(const StepArgs &a, const StepArgs &a0,
             yy_hi.x = pick(n == 2, g_tail(y[0].y, y[1].x, y[1].y, y[2].x), yy_hi.x);
             yy_hi.y = pick(n == 3, g_tail(y[1].x, y[1].y, y[2].x, y[2].y), yy_hi.y);
         }
-        yy_lo = p_mul(yy_lo, kc.rdx);
-        yy_hi = p_mul(yy_hi, kc.rdx);
+        yy_lo = p_mul(yy_lo, tc.rdx2);
+        yy_hi = p_mul(yy_hi, tc.rdx2);
         const Quad d = ld_quad(reinterpret_cast<const float *>(sD + (0 * R + k) * nthr));
         const Quad dx = ld_quad(reinterpret_cast<const float *>(sD + (1 * R + k) * nthr));
         const Quad dy = ld_quad(reinterpret_cast<const float *>(sD + (2 * R + k) * nthr));
-        const Reaction r0 = reaction(uc.lo.x, v[k].x, w[k].x, a0.m);
-        const Reaction r1 = reaction(uc.lo.y, v[k].y, w[k].y, a0.m);
-        const Reaction r2 = reaction(uc.hi.x, v[k].z, w[k].z, a0.m);
-        const Reaction r3 = reaction(uc.hi.y, v[k].w, w[k].w, a0.m);
+        const Reaction r0 = reaction(uc.lo.x, v[k].x, w[k].x, tc.m);
+        const Reaction r1 = reaction(uc.lo.y, v[k].y, w[k].y, tc.m);
+        const Reaction r2 = reaction(uc.hi.x, v[k].z, w[k].z, tc.m);
+        const Reaction r3 = reaction(uc.hi.y, v[k].w, w[k].w, tc.m);
         float2 j_lo = mk2(r0.j_ion, r1.j_ion), j_hi = mk2(r2.j_ion, r3.j_ion);
-        const int64_t goff = un.off0 + (int64_t)k * a0.pitch;
+        const int64_t goff = un.off0 + (int64_t)k * a.pitch;
         if (active && k >= un.k_lo) override_current(a, active, i, j, goff, j_lo, j_hi);
         // as in the step kernel: no packed multiply feeds a packed add
         float2 du_lo = p_mul(d.lo, add_products(uxx.lo, yy_lo));
@@ -234,12 +242,12 @@ __device__ __forceinline__ void step_unit(const StepArgs &a, const StepArgs &a0,
         du_hi = p_fma(dx.hi, X[k + 2].hi, du_hi);
         du_hi = p_fma(dy.hi, y[2], du_hi);
         du_hi = p_add_product(kc, du_hi, j_hi);
-        const float dt = a0.dt;
+        const float dt = tc.dt;
         v[k] = make_float4(fmaf(r0.dv, dt, v[k].x), fmaf(r1.dv, dt, v[k].y), fmaf(r2.dv, dt, v[k].z),
                            fmaf(r3.dv, dt, v[k].w));
         w[k] = make_float4(fmaf(r0.dw, dt, w[k].x), fmaf(r1.dw, dt, w[k].y), fmaf(r2.dw, dt, w[k].z),
                            fmaf(r3.dw, dt, w[k].w));
-        const float2 u_lo = p_fma(du_lo, kc.dt, uc.lo), u_hi = p_fma(du_hi, kc.dt, uc.hi);
+        const float2 u_lo = p_fma(du_lo, tc.dt2, uc.lo), u_hi = p_fma(du_hi, tc.dt2, uc.hi);
         const bool stored = k >= un.k_lo;
         float4 u4 = make_float4(u_lo.x, u_lo.y, u_hi.x, u_hi.y);
         if (ACT) {
@@ -269,39 +277,46 @@ __device__ __forceinline__ void step_unit(const StepArgs &a, const StepArgs &a0,
 
 }  // namespace
 
-// R: rows per thread.  ACT: activation tracking.  MANY: the tissue of this CTA's tile is one of
-// several, its pointers and stimuli in exps[]; the model, sizes, dt and dx are those of `a0`.
+// R: rows per thread.  ACT: activation tracking.  MANY: the launch holds several tissues; ra.cta says
+// which tissue (of ra.tissues) and which class of constants (ra.cls) a block belongs to.  Both are read
+// from the launch's parameters by the block index, so the model's constants stay uniform operands.
 template <int R, bool ACT, bool MANY>
 __global__ void __launch_bounds__(512, 1)
     fk_resident_kernel(const __grid_constant__ ResidentArgs ra, const __grid_constant__ StepArgs a0,
-                       const __grid_constant__ PackConsts kc, const StepArgs *__restrict__ exps) {
+                       const __grid_constant__ PackConsts kc) {
     extern __shared__ __align__(16) unsigned char res_smem[];
     __shared__ unsigned s_active[64];
     __shared__ int s_abort;  // a neighbour's strip did not come in time
-    __shared__ __align__(16) unsigned char s_args[MANY ? SMEM_ARGS_BYTES : 16];
+    __shared__ __align__(16) unsigned char s_tissue[MANY ? sizeof(ResTissue) : 16];
 
     const int tid = threadIdx.x, nthr = blockDim.x;
-    const int per = ra.nr * ra.nc;
-    const int tile = MANY ? (int)(blockIdx.x % per) : (int)blockIdx.x;
+    const uint32_t cta = MANY ? ra.cta[blockIdx.x] : 0u;
     if (MANY) {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(exps + blockIdx.x / per);
-        for (int k = tid; k < (int)(sizeof(StepArgs) / 4); k += nthr)
-            reinterpret_cast<uint32_t *>(s_args)[k] = __ldg(src + k);
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(ra.tissues + (cta >> 8));
+        for (int k = tid; k < (int)(sizeof(ResTissue) / 4); k += nthr)
+            reinterpret_cast<uint32_t *>(s_tissue)[k] = __ldg(src + k);
         __syncthreads();
     }
-    const StepArgs &a = MANY ? *reinterpret_cast<const StepArgs *>(s_args) : a0;
-    const int H = a0.H, W = a0.W, pitch = a0.pitch;
-    const float rdx = a0.rdx;
-    const int tr = tile / ra.nc, tc = tile % ra.nc;
-    const int g0 = tr * ra.ng / ra.nr, g1 = (tr + 1) * ra.ng / ra.nr;
-    const int q0 = tc * ra.nq / ra.nc, q1 = (tc + 1) * ra.nq / ra.nc;
-    const int row0 = g0 * R, row1 = tr == ra.nr - 1 ? H : g1 * R;
+    const ResTissue &tis = *reinterpret_cast<const ResTissue *>(s_tissue);
+    const StepArgs &a = MANY ? tis.args : a0;
+    const ResClass &cls = ra.cls[MANY ? cta & 255u : 0];
+    const Consts tconst{MANY ? cls.m : a0.m, MANY ? cls.rdx : a0.rdx, MANY ? cls.dt : a0.dt,
+                        MANY ? mk2(cls.rdx, cls.rdx) : kc.rdx, MANY ? mk2(cls.dt, cls.dt) : kc.dt};
+    const int H = a.H, W = a.W, pitch = a.pitch;
+    const float rdx = tconst.rdx;
+    const int t_nr = MANY ? tis.nr : ra.nr, t_nc = MANY ? tis.nc : ra.nc;
+    const int t_ng = MANY ? tis.ng : ra.ng, t_nq = MANY ? tis.nq : ra.nq;
+    const int tile = (int)blockIdx.x - (MANY ? tis.first : 0);
+    const int tr = tile / t_nc, tc = tile % t_nc;
+    const int g0 = tr * t_ng / t_nr, g1 = (tr + 1) * t_ng / t_nr;
+    const int q0 = tc * t_nq / t_nc, q1 = (tc + 1) * t_nq / t_nc;
+    const int row0 = g0 * R, row1 = tr == t_nr - 1 ? H : g1 * R;
     const int th = row1 - row0, tq = q1 - q0, j0 = 4 * q0;
     // The last tile row's groups are aligned to its bottom (so that row H-1 is the last row of a
     // thread and row 0 the first): its first group may reach `shift` rows above the tile, rows
     // that belong to the tile above and are not stored here.
     const int shift = g1 * R - row1 < 0 ? 0 : g1 * R - row1;
-    const int SUW = ra.su_w, SU = ra.su_w * ra.su_h;
+    const int SUW = MANY ? tis.su_w : ra.su_w, SU = ra.su;
     const int units = (g1 - g0) * tq;
     float *su = reinterpret_cast<float *>(res_smem);  // [2][su_h][su_w]: row r, column c at
     constexpr int UROW = 4 + R - 1, UCOL = 4;          // (r + UROW) * SUW + c + UCOL
@@ -346,6 +361,25 @@ __global__ void __launch_bounds__(512, 1)
             st4(su + (r + UROW) * SUW + c + UCOL, x);
         }
     }
+    // D the same into the second u buffer (free until the first step), for its slopes
+    float *const sdt = su + SU;
+    {
+        const int nq4 = tq + 2, n = (th + 8) * nq4;
+        for (int it = tid; it < n; it += nthr) {
+            const int r = it / nq4 - 4, c = 4 * (it % nq4) - 4;
+            const float *src = a.D + (int64_t)clampi(row0 + r, 0, H - 1) * pitch;
+            float4 x;
+            if (j0 + c >= 0 && j0 + c + 3 < W) {
+                x = __ldg(reinterpret_cast<const float4 *>(src + j0 + c));
+            } else {
+                x.x = __ldg(src + clampi(j0 + c, 0, W - 1));
+                x.y = __ldg(src + clampi(j0 + c + 1, 0, W - 1));
+                x.z = __ldg(src + clampi(j0 + c + 2, 0, W - 1));
+                x.w = __ldg(src + clampi(j0 + c + 3, 0, W - 1));
+            }
+            st4(sdt + (r + UROW) * SUW + c + UCOL, x);
+        }
+    }
     float4 v[R], w[R];
     if (mine) {
 #pragma unroll
@@ -356,14 +390,17 @@ __global__ void __launch_bounds__(512, 1)
             v[k] = __ldcg(reinterpret_cast<const float4 *>(a.v + off0 + (int64_t)k * pitch));
             w[k] = __ldcg(reinterpret_cast<const float4 *>(a.w + off0 + (int64_t)k * pitch));
         }
-        const Clamped Dg{a0.D, H, W, pitch};
+    }
+    __syncthreads();
+    if (mine) {
 #pragma unroll 1
         for (int x = 4 * k_lo; x < 4 * R; ++x) {
-            const int k = x / 4, m = x % 4, jj = j + m < W ? j + m : W - 1;
+            const int k = x / 4, m = x % 4, i = i0 + k, jj = j + m < W ? j + m : W - 1;
+            const float *p = sdt + (lr + k + UROW) * SUW + lc + m - (j + m - jj) + UCOL;
             float *d = reinterpret_cast<float *>(sD + k * nthr + tid) + m;
-            d[0] = Dg.at(i0 + k, jj);
-            d[4 * R * nthr] = slope_at<0>(Dg, i0 + k, jj, rdx);
-            d[8 * R * nthr] = slope_at<1>(Dg, i0 + k, jj, rdx);
+            d[0] = p[0];
+            d[4 * R * nthr] = slope(p, SUW, i, H, rdx);
+            d[8 * R * nthr] = slope(p, 1, jj, W, rdx);
         }
     }
     // the stimuli on during steps s .. s+31, one step per lane of warp 0
@@ -382,8 +419,8 @@ __global__ void __launch_bounds__(512, 1)
     // right 4 columns (4 words per row)
     const int64_t tile_g = blockIdx.x;
     const int o_bot = 16 * ra.max_q, o_left = 2 * o_bot, o_right = o_left + 4 * ra.max_g * R;
-    const int n_top = tr > 0 ? 4 * tq : 0, n_bot = tr < ra.nr - 1 ? 4 * tq : 0;
-    const int n_left = tc > 0 ? th : 0, n_right = tc < ra.nc - 1 ? th : 0;
+    const int n_top = tr > 0 ? 4 * tq : 0, n_bot = tr < t_nr - 1 ? 4 * tq : 0;
+    const int n_left = tc > 0 ? th : 0, n_right = tc < t_nc - 1 ? th : 0;
     const int n_items = n_top + n_bot + n_left + n_right;
     // threads with a unit that meets a neighbour (whose cells it reads and sends): the block's first
     const int n_side = tq > 2 ? 2 * G + (gt + gb) * (tq - 2) : units;
@@ -401,13 +438,13 @@ __global__ void __launch_bounds__(512, 1)
             r = x / tq;
             cc = x - r * tq;
             r -= 4;
-            t -= ra.nc;
+            t -= t_nc;
             o = o_bot + 4 * x;
         } else if ((x -= n_top) < n_bot) {  // the tile below: its top rows
             r = x / tq;
             cc = x - r * tq;
             r += th;
-            t += ra.nc;
+            t += t_nc;
             o = 4 * x;
         } else if ((x -= n_bot) < n_left) {
             r = x;
@@ -467,10 +504,11 @@ __global__ void __launch_bounds__(512, 1)
         const unsigned active = s_active[s & 63];
         const uint32_t tag = (uint32_t)s + 1;
         if (mine)
-            step_unit<R, ACT>(a, a0, kc, unit, cur + ucell, nxt + ucell, SUW, sD + tid, nthr, v, w,
+            step_unit<R, ACT>(a, tconst, kc, unit, cur + ucell, nxt + ucell, SUW, sD + tid, nthr, v, w,
                               active, (float)(ra.t0 + s));
         if (s + 1 == next_step) {  // a state that is written out
             const int64_t base = ra.every ? (int64_t)(s + 1) * ra.every : ra.out_off[next_out];
+            float *const out = MANY && ra.base ? ra.base + tis.id * ra.tissue_stride : a.vo;
             const int64_t plane = (int64_t)H * pitch;
             ++next_out;
             next_step = ra.every ? s + 2 : next_out < ra.n_out ? ra.out_step[next_out] : 0;
@@ -478,7 +516,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
                 for (int k = 0; k < R; ++k) {
                     if (k < k_lo) continue;
-                    float *g = a.vo + base + off0 + (int64_t)k * pitch;
+                    float *g = out + base + off0 + (int64_t)k * pitch;
                     const float4 x = ld4(nxt + ucell + k * SUW);
                     if (j + 3 < W) {
                         __stcg(reinterpret_cast<float4 *>(g), v[k]);
@@ -527,110 +565,131 @@ __global__ void __launch_bounds__(512, 1)
         // (split: the threads that do not wait see a wait that ran out after the next barrier at
         // the latest)
         if (s_abort) {
-            if (tid == 0) atomicOr(a0.status, kStatusTimeout);
+            if (tid == 0) atomicOr(a.status, kStatusTimeout);
             return;
         }
     }
 }
 
 // ---- plan and launch -----------------------------------------------------------------------------
-ResPlan resident_plan(int64_t H, int64_t W, int64_t n_exp, int n_sm) {
-    ResPlan best;
-    if (H < 16 || W < 16 || n_exp < 1 || n_sm < 2 || H > 65536 || W > 65536) return best;
-    const int64_t most = n_sm / n_exp;  // tiles per tissue, one CTA per SM
-    if (most < 2 || H * W > most * 512 * 4 * kResMaxRows) return best;
+// us per step, fitted to sweeps of (rows, tiles) over 64^2 .. 1200^2: the chain of one unit and the
+// exchange, plus what the units sharing the SM add.
+static double step_cost(int R, int units, int items) {
+    static const double base[] = {0, 0, 2.0, 2.4, 3.3, 4.3};
+    static const double each[] = {0, 0, 2.0e-3, 3.2e-3, 3.6e-3, 4.0e-3};
+    return base[R] + each[R] * units + 5e-4 * items;
+}
+
+// Every plan of at most `most` tiles with R rows per thread.
+template <class F>
+static void each_plan(int64_t H, int64_t W, int most, int R, F take) {
+    if (H < 16 || W < 16 || most < 1 || H > 65536 || W > 65536 ||
+        H * W > (int64_t)most * 512 * 4 * R)
+        return;
     const int nq = (int)((W + 3) / 4);
-    double cost_best = 0.0;
-    for (int R = kResMinRows; R <= kResMaxRows; ++R) {
-        const int ng = (int)((H + R - 1) / R);
-        // at least two tile rows: row 0 and row H-1 then lie in tiles of their own (see `shift`)
-        for (int nr = 2; nr <= most && nr <= ng; ++nr) {
-            // the smallest tile has ng / nr groups, the last one up to R - 1 rows less; strips take
-            // 4 rows, a tile two quads (the last quad of the grid may be partial)
-            if ((ng / nr) * R - (int)(ng * (int64_t)R - H) < 4) break;
-            const int max_g = (ng + nr - 1) / nr;
-            for (int nc = 1; nc <= most / nr; ++nc) {
-                if (nc > 1 && nq / nc < 2) break;
-                const int max_q = (nq + nc - 1) / nc;
-                const int units = max_g * max_q;
-                if (units > 512) continue;
-                const int items = (nr > 1 ? 8 * max_q : 0) + (nc > 1 ? 2 * max_g * R : 0);
-                ResPlan p;
-                p.rows = R;
-                p.nr = nr;
-                p.nc = nc;
-                p.ng = ng;
-                p.nq = nq;
-                p.max_g = max_g;
-                p.max_q = max_q;
-                int want = units > items ? units : items;
-                want = (want + 31) / 32 * 32;
-                p.threads = want < 512 ? want : 512;
-                p.su_w = 4 * (max_q + 2);
-                p.su_h = max_g * R + 8 + R - 1;
-                p.smem = sizeof(float) * 2 * (size_t)p.su_w * p.su_h + (size_t)3 * R * p.threads * 16;
-                if (p.smem > 224 * 1024) continue;
-                p.slot = 2 * 16 * (int64_t)max_q + 2 * 4 * (int64_t)max_g * R;
-                p.tiles = n_exp * nr * nc;
-                // us per step, fitted to sweeps of (rows, tiles) over 64^2 .. 1200^2: the chain
-                // of one unit and the exchange, plus what the units sharing the SM add
-                static const double base[] = {0, 0, 2.0, 2.4, 3.3, 4.3};
-                static const double each[] = {0, 0, 2.0e-3, 3.2e-3, 3.6e-3, 4.0e-3};
-                const double cost = base[R] + each[R] * units + 5e-4 * items;
-                if (!best.ok() || cost < cost_best) {
-                    best = p;
-                    cost_best = cost;
-                }
-            }
+    const int ng = (int)((H + R - 1) / R);
+    // One tile row only where H is a multiple of R: with a shifted first group, row 0 and row H-1 must
+    // lie in tiles of their own (see `shift`).
+    for (int nr = ng * R == H ? 1 : 2; nr <= most && nr <= ng; ++nr) {
+        // the smallest tile has ng / nr groups, the last one up to R - 1 rows less; strips take
+        // 4 rows, a tile two quads (the last quad of the grid may be partial)
+        if ((ng / nr) * R - (int)(ng * (int64_t)R - H) < 4) break;
+        const int max_g = (ng + nr - 1) / nr;
+        if (max_g > 512) continue;
+        const int widest = 512 / max_g;  // quads of a tile: at most 512 units
+        for (int nc = (nq + widest - 1) / widest; nc <= most / nr; ++nc) {
+            if (nc > 1 && nq / nc < 2) break;
+            const int max_q = (nq + nc - 1) / nc;
+            const int units = max_g * max_q;
+            const int items = (nr > 1 ? 8 * max_q : 0) + (nc > 1 ? 2 * max_g * R : 0);
+            ResPlan p;
+            p.rows = R;
+            p.nr = nr;
+            p.nc = nc;
+            p.ng = ng;
+            p.nq = nq;
+            p.max_g = max_g;
+            p.max_q = max_q;
+            int want = units > items ? units : items;
+            want = (want + 31) / 32 * 32;
+            p.threads = want < 512 ? want : 512;
+            p.su_w = 4 * (max_q + 2);
+            p.su_h = max_g * R + 8 + R - 1;
+            p.smem = resident_smem(R, p.threads, p.su_w * p.su_h);
+            if (p.smem > kResMaxSmem) continue;
+            p.slot = 2 * 16 * (int64_t)max_q + 2 * 4 * (int64_t)max_g * R;
+            p.tiles = nr * nc;
+            p.cost = step_cost(R, units, items);
+            take(p);
         }
     }
+}
+
+void resident_plans(int64_t H, int64_t W, int most, int R, std::vector<ResPlan> &best) {
+    best.assign(most + 1, ResPlan());
+    each_plan(H, W, most, R, [&](const ResPlan &p) {
+        ResPlan &b = best[p.tiles];
+        if (!b.ok() || p.cost < b.cost) b = p;
+    });
+    for (int t = 1; t <= most; ++t)
+        if (!best[t].ok() || (best[t - 1].ok() && best[t - 1].cost <= best[t].cost)) best[t] = best[t - 1];
+}
+
+ResPlan resident_plan(int64_t H, int64_t W, int n_sm) {
+    ResPlan best;
+    for (int R = kResMinRows; R <= kResMaxRows; ++R)
+        each_plan(H, W, n_sm, R, [&](const ResPlan &p) {
+            if (!best.ok() || p.cost < best.cost) best = p;
+        });
     return best;
 }
 
-ResPlan resident_plan(int64_t H, int64_t W, int64_t n_exp) {
+int resident_ctas() {
     static thread_local int dev_cached = -1, n_sm = 0;
     int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess) return ResPlan();
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (dev != dev_cached) {
         int coop = 0;
         if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
             n_sm = 0;
+        if (n_sm > kResMaxCtas) n_sm = kResMaxCtas;
         dev_cached = dev;
     }
-    return resident_plan(H, W, n_exp, n_sm);
+    return n_sm;
 }
+
+ResPlan resident_plan(int64_t H, int64_t W) { return resident_plan(H, W, resident_ctas()); }
 
 template <int R, bool ACT, bool MANY>
 static cudaError_t launch_one(const cudaLaunchConfig_t &cfg, const ResidentArgs &ra, const StepArgs &a,
-                              const PackConsts &k, const StepArgs *exps) {
+                              const PackConsts &k) {
     // the attribute is per function and per context: set again whenever the context changes
     static thread_local uint64_t configured_ctx = 0;
     if (context_changed(configured_ctx)) {
         const cudaError_t e = cudaFuncSetAttribute(fk_resident_kernel<R, ACT, MANY>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   224 * 1024);
+                                                   (int)kResMaxSmem);
         if (e != cudaSuccess) {
             configured_ctx = 0;
             return e;
         }
     }
-    return cudaLaunchKernelEx(&cfg, fk_resident_kernel<R, ACT, MANY>, ra, a, k, exps);
+    return cudaLaunchKernelEx(&cfg, fk_resident_kernel<R, ACT, MANY>, ra, a, k);
 }
 template <int R>
 static cudaError_t launch_rows(const cudaLaunchConfig_t &cfg, const ResidentArgs &ra, const StepArgs &a,
-                               const PackConsts &k, const StepArgs *exps) {
-    if (exps) return launch_one<R, false, true>(cfg, ra, a, k, exps);
-    return a.act_last ? launch_one<R, true, false>(cfg, ra, a, k, exps)
-                      : launch_one<R, false, false>(cfg, ra, a, k, exps);
+                               const PackConsts &k) {
+    if (ra.tissues) return launch_one<R, false, true>(cfg, ra, a, k);
+    return a.act_last ? launch_one<R, true, false>(cfg, ra, a, k) : launch_one<R, false, false>(cfg, ra, a, k);
 }
 
-cudaError_t launch_resident(const ResPlan &p, const ResidentArgs &ra, const StepArgs &a,
-                            const StepArgs *exps, cudaStream_t stream) {
+cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, const ResidentArgs &ra,
+                            const StepArgs &a, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)p.tiles);
-    cfg.blockDim = dim3((unsigned)p.threads);
-    cfg.dynamicSmemBytes = p.smem;
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -638,11 +697,11 @@ cudaError_t launch_resident(const ResPlan &p, const ResidentArgs &ra, const Step
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const PackConsts k = make_pack_consts(a.m, a.rdx, a.dt);
-    switch (p.rows) {
-        case 2: return launch_rows<2>(cfg, ra, a, k, exps);
-        case 3: return launch_rows<3>(cfg, ra, a, k, exps);
-        case 4: return launch_rows<4>(cfg, ra, a, k, exps);
-        case 5: return launch_rows<5>(cfg, ra, a, k, exps);
+    switch (rows) {
+        case 2: return launch_rows<2>(cfg, ra, a, k);
+        case 3: return launch_rows<3>(cfg, ra, a, k);
+        case 4: return launch_rows<4>(cfg, ra, a, k);
+        case 5: return launch_rows<5>(cfg, ra, a, k);
         default: return cudaErrorInvalidValue;
     }
 }

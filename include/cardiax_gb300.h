@@ -332,6 +332,13 @@ int fk_batch_set_options(fk_batch *plan, int interleave, int packed);
  * otherwise.  Same bits either way.  No counterpart in the reference. */
 int fk_batch_set_depth(fk_batch *plan, int depth);
 
+/* The resident kernel (fk_forward_euler_resident) in place of one launch per step, for sets of the
+ * plan's tissues that fit on chip together, one set after the other: on by default where every tissue
+ * can take it (16 x 16 to about 1240 x 1240, no activation tracking) and a call has steps enough to
+ * gain; the results do not change.  The other knobs tune the stepping kernel and turn it off.  Turning
+ * it on where it does not apply is FK_ERR_ARGUMENT. */
+int fk_batch_set_resident(fk_batch *plan, int on);
+
 int fk_batch_destroy(fk_batch *plan);
 
 /* ---- reverse mode ---------------------------------------------------------------------------
