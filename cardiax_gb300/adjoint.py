@@ -41,6 +41,19 @@ def _lib():
                                    ctypes.c_void_p, ctypes.POINTER(N.Params),
                                    ctypes.POINTER(N.Stimulus), ctypes.c_int, ctypes.c_double,
                                    ctypes.c_double, ctypes.c_void_p, ctypes.c_void_p]
+        L.fk_recompute_resident.restype = ctypes.c_int
+        L.fk_recompute_resident.argtypes = (L.fk_recompute.argtypes[:-1]
+                                            + [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p])
+        L.fk_forward_states.restype = ctypes.c_int
+        L.fk_forward_states.argtypes = [
+            N.Grid, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(N.Params),
+            ctypes.POINTER(N.Stimulus), ctypes.c_int, ctypes.c_int64, ctypes.POINTER(ctypes.c_int64),
+            ctypes.POINTER(ctypes.c_void_p), ctypes.c_int, ctypes.c_double, ctypes.c_double,
+            ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
+        L.fk_batch_forward_states.restype = ctypes.c_int
+        L.fk_batch_forward_states.argtypes = [
+            ctypes.c_void_p, ctypes.c_int64, ctypes.POINTER(ctypes.c_int64),
+            ctypes.POINTER(ctypes.c_void_p), ctypes.c_int, ctypes.c_int64, ctypes.c_void_p]
         L.fk_adjoint_range.restype = ctypes.c_int
         L.fk_adjoint_range.argtypes = [N.Grid, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                        ctypes.c_void_p, ctypes.POINTER(N.Params),
@@ -123,11 +136,12 @@ class Adjoint:
             for k in obs_index[t1]:
                 lam += obs_grads[k]
         buf = torch.empty((seg,) + tuple(state0.shape), dtype=state0.dtype, device=state0.device)
+        ws, ws_bytes = T._resident_workspace()
         for s, st in reversed(ckpts):
             e = min(s + seg, t1)
-            rc = L.fk_recompute(T.grid, st.data_ptr(), s, e - s, T.D.data_ptr(),
-                                ctypes.byref(T.params), T.stim, T.n_stim, T.dt, T.dx,
-                                buf.data_ptr(), stream_handle())
+            rc = L.fk_recompute_resident(T.grid, st.data_ptr(), s, e - s, T.D.data_ptr(),
+                                         ctypes.byref(T.params), T.stim, T.n_stim, T.dt, T.dx,
+                                         buf.data_ptr(), ws, ws_bytes, stream_handle())
             if rc:
                 raise N.FkError(rc, "fk_recompute")
             inj = [(tt, k) for tt in range(s, e) for k in obs_index.get(tt, [])]
@@ -152,21 +166,64 @@ def forward_checkpoints(T: Tissue, state0: torch.Tensor, t0: int, t1: int, seg: 
     also returns clones of the (v, w, u) planes at each step in ``stops``."""
     ckpts, snaps = [], {}
     T.state.copy_(state0)
-    marks = sorted(set(range(t0, t1, seg)) | {int(x) for x in stops if t0 <= int(x) <= t1})
-    cur = t0
-    for m in marks:
-        if m > cur:
-            T.advance(cur, m)
-            cur = m
+    stops = {int(x) for x in stops}
+    marks = sorted(set(range(t0, t1, seg)) | {x for x in stops if t0 <= x <= t1})
+
+    def keep(m, st, owned):
         if (m - t0) % seg == 0 and m < t1:
-            ckpts.append((m, T.state.clone()))
+            ckpts.append((m, st if owned else st.clone()))
         if m in stops:
-            snaps[m] = T.state[:, :, :T.W].clone()
+            snaps[m] = st[:, :, :T.W].clone()
+
+    def states(t, steps, outs):
+        rc = _lib().fk_forward_states(
+            T.grid, T.state.data_ptr(), T.scratch.data_ptr(), T.D.data_ptr(),
+            ctypes.byref(T.params), T.stim, T.n_stim, t, *_step_list(steps, outs), T.dt, T.dx,
+            ws, ws_bytes, stream_handle())
+        if rc:
+            raise N.FkError(rc, "fk_forward_states")
+
+    ws, ws_bytes = T._resident_workspace()
+    many = bool(ws) and T.activation is None
+    cur = _states_at(T.advance, states if many else None, t0, marks,
+                     lambda m: (m - t0) % seg == 0 and m < t1, T.state, keep)
     if t1 > cur:
         T.advance(cur, t1)
-        if t1 in stops:
-            snaps[t1] = T.state[:, :, :T.W].clone()
     return (ckpts, snaps) if stops else ckpts
+
+
+# states one call writes: what is not kept goes through as many buffers, used again by the next call
+STATES_PER_CALL = 16
+
+
+def _step_list(steps, outs):
+    return ((ctypes.c_int64 * len(steps))(*steps),
+            (ctypes.c_void_p * len(steps))(*[o.data_ptr() for o in outs]), len(steps))
+
+
+def _states_at(advance, run, t0: int, marks, own, state: torch.Tensor, take) -> int:
+    """Steps ``state`` from t0 through ``marks`` (ascending): ``take(mark, x, owned)`` gets each
+    mark's state.  ``run(t, steps, outs)`` writes several states by one call (one launch where they
+    fit on chip): a state is then its taker's (owned) where ``own(mark)``, else in a buffer that the
+    next call writes again.  Without ``run``, each is ``state`` itself after ``advance(t, mark)``.
+    Returns the last mark, t0 without any."""
+    spare, cur = [], t0
+    for i in range(0, len(marks), STATES_PER_CALL if run else 1):
+        part = marks[i:i + (STATES_PER_CALL if run else 1)]
+        if not run:
+            if part[0] > cur:
+                advance(cur, part[0])
+            take(part[0], state, False)
+        else:
+            while len(spare) < sum(not own(m) for m in part):
+                spare.append(torch.empty_like(state))
+            left = list(spare)
+            outs = [torch.empty_like(state) if own(m) else left.pop() for m in part]
+            run(cur, part, outs)
+            for m, x in zip(part, outs):
+                take(m, x, own(m))
+        cur = part[-1]
+    return cur
 
 
 class _Rollout(torch.autograd.Function):
@@ -220,7 +277,8 @@ def rollout(v0, w0, u0, D, theta, stimuli, t0: int, t1: int, obs_times: Sequence
 
 class _BatchPlan:
     """B experiments on one grid sharing D and the parameters, as one fk_batch plan (their
-    forward steps and recomputed segments are one launch per step for all of them)."""
+    forward steps and recomputed segments are one launch per step for all of them, or one launch
+    for many steps of as many as fit on chip)."""
 
     def __init__(self, states0, Dp, params, stimuli, dt, dx):
         B, _, H, W = states0.shape
@@ -250,9 +308,17 @@ class _BatchPlan:
         plan = ctypes.c_void_p()
         N.call("fk_batch_create", descs, B, base, nbytes, stream_handle(), ctypes.byref(plan))
         self.plan = plan
+        self.resident = L.fk_batch_set_resident(plan, 1) == 0
 
     def advance(self, t0: int, t1: int):
         N.call("fk_batch_forward_euler", self.plan, int(t0), int(t1), 0, stream_handle())
+
+    def states(self, t: int, steps: Sequence[int], outs: Sequence[torch.Tensor]):
+        """Steps from t, writing all experiments' states at ``steps`` to ``outs``."""
+        rc = _lib().fk_batch_forward_states(self.plan, t, *_step_list(steps, outs),
+                                            self.S[0].numel(), stream_handle())
+        if rc:
+            raise N.FkError(rc, "fk_batch_forward_states")
 
     def close(self):
         if getattr(self, "plan", None):
@@ -268,9 +334,10 @@ class _BatchPlan:
 
 class _RolloutBatch(torch.autograd.Function):
     """States at ``obs_times`` of B tissues sharing D and theta (one stimulus list per tissue).
-    Forward, segment recomputation and the adjoint are each one launch per step for all B
-    tissues (fk_batch_forward_euler, fk_batch_recompute, fk_adjoint_batch_range), with
-    checkpoints every ``seg`` steps as in :func:`rollout`."""
+    The adjoint is one launch per step for all B tissues (fk_adjoint_batch_range); so are forward
+    and segment recomputation (fk_batch_forward_states, fk_batch_recompute) where the tissues do
+    not fit on chip, else one launch for many steps.  Checkpoints lie every ``seg`` steps as in
+    :func:`rollout`."""
 
     @staticmethod
     def forward(ctx, states0, D, theta, Cm, stimuli, t0, t1, obs_times, dt, dx, seg):
@@ -285,20 +352,23 @@ class _RolloutBatch(torch.autograd.Function):
         obs_at = {}
         for k, t in enumerate(obs_times):
             obs_at.setdefault(int(t), []).append(k)
-        marks = sorted(set(range(t0, t_end, seg)) | set(obs_at))
-        ckpts, cur = [], t0
-        for m in marks:
-            if m > cur:
-                bp.advance(cur, m)
-                cur = m
-            if (m - t0) % seg == 0 and m < t_end:
-                ckpts.append((m, bp.S.clone()))
+        # (the last step is an observation, or t0)
+        marks = sorted(set(range(t0, t_end, seg)) | {m for m in obs_at if m >= t0})
+        ckpts = []
+
+        def own(m):
+            return (m - t0) % seg == 0 and m < t_end
+
+        def keep(m, st, owned):
+            if m >= t0 and own(m):
+                ckpts.append((m, st if owned else st.clone()))
             for k in obs_at.get(m, []):
-                out[:, k] = bp.S[..., :W]
-        if t_end > cur:
-            bp.advance(cur, t_end)
-            for k in obs_at.get(t_end, []):
-                out[:, k] = bp.S[..., :W]
+                out[:, k] = st[..., :W]
+
+        for m in obs_at:
+            if m < t0:
+                keep(m, bp.S, False)
+        _states_at(bp.advance, bp.states if bp.resident else None, t0, marks, own, bp.S, keep)
         ctx.bp, ctx.ckpts = bp, ckpts
         ctx.t0, ctx.t1, ctx.obs_times, ctx.seg = t0, t_end, list(obs_times), seg
         return out

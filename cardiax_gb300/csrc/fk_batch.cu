@@ -387,11 +387,15 @@ void fill_resident(fk_batch *b) {
 }
 
 // n steps from t0 of every tissue through the resident launches: in place; or, n at most kResMaxSteps,
-// writing every state x_{t0+s}, s = 1 .. n, of tissue k to base + k * stride + s * every and leaving the
-// tissues' own as they were.
+// leaving the tissues' own states as they were and writing those of tissue k to base + k * stride + an
+// offset: every x_{t0+s}, s = 1 .. n, at offset s * every, or those of the steps steps[i] (n_outs of
+// them, the last one t0 + n) at offset outs[i] - base.
 struct ResOut {
     float *base = nullptr;
     int64_t stride = 0, every = 0;
+    const int64_t *steps = nullptr;
+    float *const *outs = nullptr;
+    int n_outs = 0;
 };
 int run_resident(const fk_batch *b, int64_t t0, int64_t n, const ResOut &out, cudaStream_t s) {
     for (const ResWave &w : b->res.w) {
@@ -413,6 +417,13 @@ int run_resident(const fk_batch *b, int64_t t0, int64_t n, const ResOut &out, cu
             ra.n_out = 1;
             ra.out_step[0] = (int)c;
             ra.out_off[0] = 0;
+            if (out.outs) {
+                ra.n_out = out.n_outs;
+                for (int k = 0; k < out.n_outs; ++k) {
+                    ra.out_step[k] = (int)(out.steps[k] - t0);
+                    ra.out_off[k] = out.outs[k] - out.base;
+                }
+            }
             if (cudaMemsetAsync(b->d_xchg, 0, (size_t)(w.ctas * 2 * ra.slot) * 8, s) != cudaSuccess ||
                 launch_resident(w.rows, w.ctas, w.threads, w.smem, ra, a, s) != cudaSuccess)
                 return FK_ERR_CUDA;
@@ -835,6 +846,60 @@ __global__ static void batch_state_out_kernel(const BatchTissue *tissues, int pa
         out[k] = __ldcg(src + k);
 }
 
+// The other way: tissue e's state from src + e * exp_stride.
+__global__ static void batch_state_in_kernel(const BatchTissue *tissues, const float *src, int64_t exp_stride,
+                                             int64_t ns) {
+    float4 *dst = reinterpret_cast<float4 *>(const_cast<float *>(tissues[blockIdx.y].args[0].v));
+    const float4 *in = reinterpret_cast<const float4 *>(src + (int64_t)blockIdx.y * exp_stride);
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < ns / 4;
+         k += (int64_t)gridDim.x * blockDim.x)
+        __stcg(dst + k, __ldcg(in + k));
+}
+
+int fk_batch_forward_states(fk_batch *b, int64_t t0, const int64_t *steps, float *const *outs, int n_steps,
+                            int64_t exp_stride, void *stream) {
+    if (!b || (n_steps > 0 && (!steps || !outs))) return FK_ERR_NULL;
+    if (n_steps < 0 || t0 < -(int64_t(1) << 24)) return FK_ERR_ARGUMENT;
+    int64_t ns = 0;
+    if (!one_grid(b, &ns)) return FK_ERR_SHAPE;
+    if ((exp_stride & 3) || exp_stride < ns) return FK_ERR_ALIGN;
+    for (int k = 0; k < n_steps; ++k) {
+        if (steps[k] < (k ? steps[k - 1] : t0) || steps[k] > (int64_t(1) << 24)) return FK_ERR_ARGUMENT;
+        if (!outs[k]) return FK_ERR_NULL;
+        if (reinterpret_cast<uintptr_t>(outs[k]) & 15u) return FK_ERR_ALIGN;
+    }
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev != b->device) return FK_ERR_CUDA;
+    cudaStream_t s = (cudaStream_t)stream;
+    const dim3 cgrid(64, b->n);
+    int64_t t = t0;
+    for (int k = 0; k < n_steps;) {
+        // as many states, of distinct steps, as one resident launch writes
+        int m = 0;
+        if (b->resident)
+            while (k + m < n_steps && m < kResMaxOut && steps[k + m] > (m ? steps[k + m - 1] : t) &&
+                   steps[k + m] - t <= kResMaxSteps)
+                ++m;
+        const int64_t n = m ? steps[k + m - 1] - t : 0;
+        // (a stepped state is also copied out, and one more resident launch copies the last one back)
+        const double copy = 2.0 + (double)b->cells / 170e3;
+        if (m && res_time(b->res, n) + copy < step_time(b->cells, n) + m * copy) {
+            int rc = run_resident(b, t, n, ResOut{outs[k], exp_stride, 0, steps + k, outs + k, m}, s);
+            if (rc) return rc;
+            k += m;
+            batch_state_in_kernel<<<cgrid, 256, 0, s>>>(b->d_tissues, outs[k - 1], exp_stride, ns);
+        } else {
+            int rc = fk_batch_forward_euler(b, t, steps[k], 0, stream);
+            if (rc) return rc;
+            batch_state_out_kernel<<<cgrid, 256, 0, s>>>(b->d_tissues, 0, outs[k], exp_stride, ns);
+            ++k;
+        }
+        if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
+        t = steps[k - 1];
+    }
+    return FK_OK;
+}
+
 int fk_batch_recompute(fk_batch *b, int64_t s, int64_t n, float *bufs, int64_t exp_stride,
                        void *stream) {
     if (!b || !bufs) return FK_ERR_NULL;
@@ -854,7 +919,7 @@ int fk_batch_recompute(fk_batch *b, int64_t s, int64_t n, float *bufs, int64_t e
         res_time(b->res, n - 1) < step_time(b->cells, n - 1) + (double)(n - 1) * (2.0 + (double)b->cells / 170e3)) {
         batch_state_out_kernel<<<cgrid, 256, 0, cs>>>(b->d_tissues, 0, bufs, exp_stride, ns);
         if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
-        return run_resident(b, s, n - 1, ResOut{bufs, exp_stride, ns}, cs);
+        return run_resident(b, s, n - 1, ResOut{bufs, exp_stride, ns, nullptr, nullptr, 0}, cs);
     }
     set_int_kernel<<<1, 1, 0, cs>>>(b->d_t, (int)s);
     batch_state_out_kernel<<<cgrid, 256, 0, cs>>>(b->d_tissues, 0, bufs, exp_stride, ns);

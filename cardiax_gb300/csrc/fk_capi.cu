@@ -1008,6 +1008,54 @@ int fk_forward_resident(fk_grid g, const float *state0, float *scratch, const fl
     return FK_OK;
 }
 
+int fk_forward_states(fk_grid g, float *state, float *scratch, const float *D, const fk_params *p,
+                      const fk_stimulus *stimuli, int n_stimuli, int64_t t0, const int64_t *steps,
+                      float *const *outs, int n_steps, double dt, double dx, void *workspace,
+                      size_t workspace_bytes, void *stream) {
+    int rc = common_checks(g, state, scratch, D, p, dx);
+    if (rc) return rc;
+    if (n_steps > 0 && (!steps || !outs)) return FK_ERR_NULL;
+    if (n_steps < 0 || !std::isfinite(dt)) return FK_ERR_ARGUMENT;
+    for (int k = 0; k < n_steps; ++k) {
+        if (steps[k] < (k ? steps[k - 1] : t0)) return FK_ERR_ARGUMENT;
+        if (!outs[k]) return FK_ERR_NULL;
+        if (!aligned16(outs[k])) return FK_ERR_ALIGN;
+    }
+    if (n_steps == 0) return FK_OK;
+    const size_t bytes = sizeof(float) * 3 * g.H * g.pitch;
+    const int64_t n = steps[n_steps - 1] - t0;
+    cudaStream_t s = (cudaStream_t)stream;
+    ResPlan plan;
+    if (!takes_resident(g, n, n_stimuli, workspace, workspace_bytes, plan)) {
+        for (int k = 0; k < n_steps; ++k) {
+            if ((rc = fk_forward_euler_tracked(g, state, scratch, D, p, stimuli, n_stimuli,
+                                               k ? steps[k - 1] : t0, steps[k], dt, dx, nullptr, stream)))
+                return rc;
+            if (cudaMemcpyAsync(outs[k], state, bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+                return FK_ERR_CUDA;
+        }
+        return FK_OK;
+    }
+    Stim st[kMaxStim];
+    if ((rc = make_stims(stimuli, n_stimuli, g, st))) return rc;
+    int *status = status_ptr();
+    if (!status) return FK_ERR_CUDA;
+    std::vector<std::pair<int64_t, int64_t>> at;
+    for (int k = 0; k < n_steps; ++k)
+        if (steps[k] > (k ? steps[k - 1] : t0)) at.push_back({steps[k] - t0, outs[k] - state});
+    if ((rc = resident_run(plan, g, state, state, at, scratch, D, make_model(*p), st, n_stimuli, t0, n,
+                           (float)dt, 1.0f / (float)dx, nullptr, workspace, status, s)))
+        return rc;
+    for (int k = 0; k <= n_steps; ++k) {  // steps listed twice; then the state itself
+        const float *src = k ? outs[k - 1] : state;
+        if ((k == n_steps || steps[k] == (k ? steps[k - 1] : t0)) &&
+            cudaMemcpyAsync(k == n_steps ? state : outs[k], src, bytes, cudaMemcpyDeviceToDevice, s) !=
+                cudaSuccess)
+            return FK_ERR_CUDA;
+    }
+    return FK_OK;
+}
+
 int64_t fk_adjoint_slots(fk_grid g) {
     if (check_grid(g)) return 0;
     return adjoint_slots((int)g.H, (int)g.W);
@@ -1151,6 +1199,38 @@ int fk_recompute(fk_grid g, const float *state, int64_t s, int64_t n, const floa
                        rdx, false, tm_d, maps, status, cs);
         if (rc) return rc;
     }
+    return FK_OK;
+}
+
+int fk_recompute_resident(fk_grid g, const float *state, int64_t s, int64_t n, const float *D,
+                          const fk_params *p, const fk_stimulus *stimuli, int n_stimuli, double dt,
+                          double dx, float *buf, void *workspace, size_t workspace_bytes, void *stream) {
+    ResPlan plan;
+    if (check_grid(g) || n - 1 > kResMaxSteps ||  // (one launch writes every state)
+        !takes_resident(g, n - 1, n_stimuli, workspace, workspace_bytes, plan))
+        return fk_recompute(g, state, s, n, D, p, stimuli, n_stimuli, dt, dx, buf, stream);
+    int rc = common_checks(g, state, buf, D, p, dx);
+    if (rc) return rc;
+    if (!std::isfinite(dt)) return FK_ERR_ARGUMENT;
+    Stim st[kMaxStim];
+    if ((rc = make_stims(stimuli, n_stimuli, g, st))) return rc;
+    int *status = status_ptr();
+    if (!status) return FK_ERR_CUDA;
+    const int64_t ns = 3 * g.H * g.pitch;
+    cudaStream_t cs = (cudaStream_t)stream;
+    if (cudaMemcpyAsync(buf, state, sizeof(float) * ns, cudaMemcpyDeviceToDevice, cs) != cudaSuccess)
+        return FK_ERR_CUDA;
+    StepArgs a;
+    fill_args(a, g, state, D, make_model(*p), st, n_stimuli, (float)dt, 1.0f / (float)dx, status, nullptr);
+    a.vo = buf;
+    ResidentArgs ra{};
+    resident_args(ra, plan, workspace);
+    ra.t0 = s;
+    ra.n = (int)(n - 1);
+    ra.every = ns;
+    if (cudaMemsetAsync(workspace, 0, plan.workspace(), cs) != cudaSuccess ||
+        launch_resident(plan.rows, (int)plan.tiles, plan.threads, plan.smem, ra, a, cs) != cudaSuccess)
+        return FK_ERR_CUDA;
     return FK_OK;
 }
 

@@ -187,6 +187,19 @@ int fk_forward_resident(fk_grid g, const float *state0, float *scratch, const fl
                         const int64_t *checkpoints, int n_checkpoints, double dt, double dx,
                         float *out, void *workspace, size_t workspace_bytes, void *stream);
 
+/* fk_recompute (below) the same way: every state of a segment, kept on chip between steps. */
+int fk_recompute_resident(fk_grid g, const float *state, int64_t s, int64_t n, const float *D,
+                          const fk_params *p, const fk_stimulus *stimuli, int n_stimuli, double dt,
+                          double dx, float *buf, void *workspace, size_t workspace_bytes, void *stream);
+
+/* Euler steps from t0 in place, the states at steps[0] <= steps[1] <= ... (each at least t0) written to
+ * outs[k] as well (host array of device pointers, 16-byte aligned, apart from state, scratch and one
+ * another); `state` ends at the last step. */
+int fk_forward_states(fk_grid g, float *state, float *scratch, const float *D, const fk_params *p,
+                      const fk_stimulus *stimuli, int n_stimuli, int64_t t0, const int64_t *steps,
+                      float *const *outs, int n_steps, double dt, double dx, void *workspace,
+                      size_t workspace_bytes, void *stream);
+
 /* Temporal blocking (no reference counterpart; same results bit for bit): fk_forward_euler with
  * `depth` steps (1, 2, 4 or 8) per launch.  Each tile is loaded once with a 4*depth-cell halo,
  * advanced `depth` times in shared memory (recomputing the halo ring) and stored once; the last
@@ -373,6 +386,13 @@ int fk_adjoint_range(fk_grid g, const float *buf, int64_t s, int64_t n, const fl
                      double dx, float *lam, float *lam_tmp, const int64_t *inj_steps,
                      const float *const *inj_grads, int n_inj, float *grad_D,
                      double *grad_theta_slots, void *stream);
+
+/* Advances a plan whose tissues lie on one grid from step t0 through steps[0] <= steps[1] <= ... (each at
+ * least t0), writing tissue e's state at steps[k] to outs[k] + e * exp_stride (floats; host array of device
+ * pointers, 16-byte aligned, apart from the tissues' buffers and one another); the tissues end at the last
+ * step.  One launch for several of the states where the resident kernel takes the plan. */
+int fk_batch_forward_states(fk_batch *plan, int64_t t0, const int64_t *steps, float *const *outs, int n_steps,
+                            int64_t exp_stride, void *stream);
 
 /* Batched reverse pass: E experiments on one grid that share D and the parameters (each with
  * its own stimuli and state), as in an inverse problem fitted to several recordings.  No
