@@ -7,8 +7,10 @@ gates and the stimulus replacement contributing zero derivative.  Gradients are 
 respect to the initial state, the per-cell diffusivity D and the first 13 fields of ``Params``
 (``Cm`` is held fixed).
 
-Memory: a rollout of T steps keeps ceil(T / K) checkpoints plus one segment of K recomputed
-states, K = ceil(sqrt(T)) by default (e.g. 1e4 steps at 512^2: 200 states of 3 MiB).
+Memory: a rollout of T steps keeps all its states while they are small next to the device's memory
+(_room_for_states), else ceil(T / K) checkpoints plus one segment of K recomputed states,
+K = ceil(sqrt(T)) by default (e.g. 1e4 steps at 512^2: 200 states of 3 MiB); with ``seg`` given,
+segments of ``seg`` steps in any case.
 """
 from __future__ import annotations
 
@@ -113,20 +115,35 @@ class Adjoint:
         return self.gD[:, :self.t.W]
 
     # -- rollouts -----------------------------------------------------------------------------
+    def recompute(self, state: torch.Tensor, s: int, n: int, buf: torch.Tensor):
+        """The n states from step s, that of step s being ``state``, into ``buf``."""
+        T = self.t
+        ws, ws_bytes = T._resident_workspace()
+        rc = _lib().fk_recompute_resident(T.grid, state.data_ptr(), s, n, T.D.data_ptr(),
+                                          ctypes.byref(T.params), T.stim, T.n_stim, T.dt, T.dx,
+                                          buf.data_ptr(), ws, ws_bytes, stream_handle())
+        if rc:
+            raise N.FkError(rc, "fk_recompute")
+
     def rollout_gradient(self, state0: torch.Tensor, t0: int, t1: int, obs_times: Sequence[int],
-                         obs_grads: torch.Tensor, seg: int = None, ckpts=None) -> torch.Tensor:
+                         obs_grads: torch.Tensor, seg: int = None, ckpts=None,
+                         states: torch.Tensor = None) -> torch.Tensor:
         """Backward pass of a rollout from ``state0`` ((3, H, pitch)) over steps t0 .. t1-1,
         where the loss depends on the states at ``obs_times`` (each in [t0, t1]) with
         dL/dx_{obs_times[k]} = obs_grads[k] ((n_obs, 3, H, pitch)).  Returns dL/dx_{t0};
         dL/dD and dL/dtheta accumulate in this object.  Uses checkpoints every ``seg`` steps
         (default ceil(sqrt(T))) and recomputes one segment at a time; ``ckpts`` = the
-        [(step, state)] checkpoints at t0, t0+seg, ... when the caller kept them."""
+        [(step, state)] checkpoints at t0, t0+seg, ... when the caller kept them; ``states`` =
+        every state from t0 on, (at least t1 - t0, 3, H, pitch), when it kept those: nothing is
+        recomputed then."""
         T = self.t
         n = t1 - t0
         seg = seg or default_segment(n)
         obs_index = {}
         for k, tt in enumerate(obs_times):
             obs_index.setdefault(int(tt), []).append(k)
+        if states is not None:
+            seg, ckpts = max(n, 1), [(t0, None)] if n else []
         if ckpts is None:  # forward: checkpoints at t0, t0+seg, ...
             ckpts = forward_checkpoints(T, state0, t0, t1, seg)
         L = _lib()
@@ -135,15 +152,13 @@ class Adjoint:
         if t1 in obs_index:
             for k in obs_index[t1]:
                 lam += obs_grads[k]
-        buf = torch.empty((seg,) + tuple(state0.shape), dtype=state0.dtype, device=state0.device)
-        ws, ws_bytes = T._resident_workspace()
+        buf = states
+        if buf is None:
+            buf = torch.empty((seg,) + tuple(state0.shape), dtype=state0.dtype, device=state0.device)
         for s, st in reversed(ckpts):
             e = min(s + seg, t1)
-            rc = L.fk_recompute_resident(T.grid, st.data_ptr(), s, e - s, T.D.data_ptr(),
-                                         ctypes.byref(T.params), T.stim, T.n_stim, T.dt, T.dx,
-                                         buf.data_ptr(), ws, ws_bytes, stream_handle())
-            if rc:
-                raise N.FkError(rc, "fk_recompute")
+            if st is not None:
+                self.recompute(st, s, e - s, buf)
             inj = [(tt, k) for tt in range(s, e) for k in obs_index.get(tt, [])]
             steps = (ctypes.c_int64 * max(1, len(inj)))(*[tt for tt, _ in inj])
             grads = (ctypes.c_void_p * max(1, len(inj)))(*[obs_grads[k].data_ptr() for _, k in inj])
@@ -154,6 +169,28 @@ class Adjoint:
             if rc:
                 raise N.FkError(rc, "fk_adjoint_range")
         return lam
+
+
+def _room_for_states(n: int, like: torch.Tensor, lead: int = 0):
+    """A buffer for the states of n steps and the first one (dimension ``lead`` of the result), or
+    None where recomputing segments is the better use of memory: more than 1/64 of the device's (4.5
+    of 288 GB), or less than half of it free.  With every state kept a gradient pass runs the
+    forward steps once, not twice: 4865 -> 4027 us (16 x 256^2 cells, 80 steps: 1 GB), 2171 -> 1783
+    (151 x 203, 100 steps)."""
+    total = torch.cuda.get_device_properties(like.device).total_memory
+    if not 1 <= n <= MOST_KEPT or (n + 1) * like.numel() * 4 > total // 64:
+        return None
+    if torch.cuda.mem_get_info(like.device)[0] < total // 2:
+        return None
+    shape = list(like.shape)
+    shape.insert(lead, n + 1)
+    try:
+        return torch.empty(shape, dtype=torch.float32, device=like.device)
+    except torch.cuda.OutOfMemoryError:  # a limit on this process
+        return None
+
+
+MOST_KEPT = 8192  # steps of one resident launch
 
 
 def default_segment(n_steps: int) -> int:
@@ -237,14 +274,22 @@ class _Rollout(torch.autograd.Function):
         tis.set_state((v0.detach(), w0.detach(), u0.detach()))
         state0 = tis.state.clone()
         t_end = max([t0] + [int(t) for t in obs_times])
+        states, ckpts = None, None
+        if not seg and any(ctx.needs_input_grad) and all(int(t) >= t0 for t in obs_times):
+            states = _room_for_states(t_end - t0, state0)
         seg = seg or default_segment(t_end - t0)
-        ckpts, snaps = forward_checkpoints(tis, state0, t0, t_end, seg, stops=list(obs_times))
         out = torch.empty((len(obs_times), 3, H, W), dtype=torch.float32, device=u0.device)
-        for k, t in enumerate(obs_times):
-            out[k] = snaps[int(t)]
+        if states is not None:
+            Adjoint(tis).recompute(state0, t0, t_end - t0 + 1, states)
+            for k, t in enumerate(obs_times):
+                out[k] = states[int(t) - t0, :, :, :W]
+        else:
+            ckpts, snaps = forward_checkpoints(tis, state0, t0, t_end, seg, stops=list(obs_times))
+            for k, t in enumerate(obs_times):
+                out[k] = snaps[int(t)]
         ctx.save_for_backward(state0)
         ctx.tis, ctx.t0, ctx.t1, ctx.obs_times, ctx.seg, ctx.W = tis, t0, t_end, list(obs_times), seg, W
-        ctx.ckpts = ckpts
+        ctx.ckpts, ctx.states = ckpts, states
         return out
 
     @staticmethod
@@ -256,8 +301,8 @@ class _Rollout(torch.autograd.Function):
                         device=state0.device)
         g[..., :W] = grad_out.to(torch.float32)
         lam0 = adj.rollout_gradient(state0, ctx.t0, ctx.t1, ctx.obs_times, g, seg=ctx.seg,
-                                    ckpts=ctx.ckpts)
-        ctx.ckpts = None
+                                    ckpts=ctx.ckpts, states=ctx.states)
+        ctx.ckpts = ctx.states = None
         gth = adj.grad_theta().to(torch.float32)
         return (lam0[0, :, :W], lam0[1, :, :W], lam0[2, :, :W], adj.grad_D().clone(), gth,
                 None, None, None, None, None, None, None, None)
@@ -268,7 +313,7 @@ def rollout(v0, w0, u0, D, theta, stimuli, t0: int, t1: int, obs_times: Sequence
     """Differentiable rollout: the states (n_obs, 3, H, W) at ``obs_times`` (steps in
     [t0, t1]) starting from (v0, w0, u0) at step t0.  Gradients flow to v0, w0, u0, D and
     ``theta`` (the 13 first Params fields) through the hand-written adjoint kernel with
-    sqrt(T) checkpointing."""
+    sqrt(T) checkpointing, or every state kept where they are few."""
     dev = u0.device if isinstance(u0, torch.Tensor) and u0.is_cuda else torch.device("cuda")
     to = lambda x: x if isinstance(x, torch.Tensor) and x.is_cuda else as_cuda_f32(x, dev)  # noqa: E731
     return _Rollout.apply(to(v0), to(w0), to(u0), to(D), to(theta), Cm, list(stimuli), int(t0),
@@ -320,6 +365,14 @@ class _BatchPlan:
         if rc:
             raise N.FkError(rc, "fk_batch_forward_states")
 
+    def recompute(self, s: int, n: int, buf: torch.Tensor):
+        """Steps from s (the experiments' states now), the n states from there on to ``buf``
+        ((B, at least n, 3, H, pitch))."""
+        rc = _lib().fk_batch_recompute(self.plan, s, n, buf.data_ptr(), buf[0].numel(),
+                                       stream_handle())
+        if rc:
+            raise N.FkError(rc, "fk_batch_recompute")
+
     def close(self):
         if getattr(self, "plan", None):
             N.lib().fk_batch_destroy(self.plan)
@@ -345,6 +398,7 @@ class _RolloutBatch(torch.autograd.Function):
         B, _, H, W = states0.shape
         dev = states0.device
         t_end = max([t0] + [int(t) for t in obs_times])
+        whole = not seg and any(ctx.needs_input_grad) and all(int(t) >= t0 for t in obs_times)
         seg = seg or default_segment(t_end - t0)
         Dp = to_pitched(D.detach(), H, W, pitch_of(W), dev)
         bp = _BatchPlan(states0.detach(), Dp, params, stimuli, dt, dx)
@@ -368,8 +422,15 @@ class _RolloutBatch(torch.autograd.Function):
         for m in obs_at:
             if m < t0:
                 keep(m, bp.S, False)
-        _states_at(bp.advance, bp.states if bp.resident else None, t0, marks, own, bp.S, keep)
-        ctx.bp, ctx.ckpts = bp, ckpts
+        states = _room_for_states(t_end - t0, bp.S, 1) if whole else None
+        if states is not None:
+            bp.recompute(t0, t_end - t0 + 1, states)
+            for k, t in enumerate(obs_times):
+                out[:, k] = states[:, int(t) - t0, :, :, :W]
+            seg, ckpts = t_end - t0, [(t0, None)]
+        else:
+            _states_at(bp.advance, bp.states if bp.resident else None, t0, marks, own, bp.S, keep)
+        ctx.bp, ctx.ckpts, ctx.states = bp, ckpts, states
         ctx.t0, ctx.t1, ctx.obs_times, ctx.seg = t0, t_end, list(obs_times), seg
         return out
 
@@ -391,7 +452,10 @@ class _RolloutBatch(torch.autograd.Function):
         for k in obs_index.get(t1, []):
             lam += g[k]
         ns = 3 * H * pitch
-        buf = torch.empty((B, seg, 3, H, pitch), dtype=torch.float32, device=dev)
+        buf = ctx.states
+        if buf is None:
+            buf = torch.empty((B, seg, 3, H, pitch), dtype=torch.float32, device=dev)
+        room = buf.shape[1]  # states an experiment has in buf
         slots = int(L.fk_adjoint_slots(bp.grid))
         gD = torch.zeros((B, H, pitch), dtype=torch.float32, device=dev)
         gth = torch.zeros((B, slots, 16), dtype=torch.float64, device=dev)
@@ -402,15 +466,13 @@ class _RolloutBatch(torch.autograd.Function):
         n_stims = (ctypes.c_int * B)(*[n for _, n in bp.stims])
         for s, st in reversed(ctx.ckpts):
             e = min(s + seg, t1)
-            bp.S.copy_(st)
-            rc = L.fk_batch_recompute(bp.plan, s, e - s, buf.data_ptr(), seg * ns,
-                                      stream_handle())
-            if rc:
-                raise N.FkError(rc, "fk_batch_recompute")
+            if st is not None:
+                bp.S.copy_(st)
+                bp.recompute(s, e - s, buf)
             inj = [(tt, k) for tt in range(s, e) for k in obs_index.get(tt, [])]
             steps = (ctypes.c_int64 * max(1, len(inj)))(*[tt for tt, _ in inj])
             grads = (ctypes.c_void_p * max(1, len(inj)))(*[g[k].data_ptr() for _, k in inj])
-            rc = L.fk_adjoint_batch_range(B, bp.grid, buf.data_ptr(), seg * ns, s, e - s,
+            rc = L.fk_adjoint_batch_range(B, bp.grid, buf.data_ptr(), room * ns, s, e - s,
                                           bp.D.data_ptr(), ctypes.byref(bp.params), stim_ptrs,
                                           n_stims, bp.dt, bp.dx, lam.data_ptr(),
                                           lam_tmp.data_ptr(), steps, grads, len(inj),
@@ -418,7 +480,7 @@ class _RolloutBatch(torch.autograd.Function):
                                           stream_handle())
             if rc:
                 raise N.FkError(rc, "fk_adjoint_batch_range")
-        ctx.ckpts = None
+        ctx.ckpts = ctx.states = None
         gD_sum = gD[0, :, :W].clone()
         gth_sum = gth[0, :, :N_THETA].sum(0)
         for b in range(1, B):  # fixed order: deterministic sums

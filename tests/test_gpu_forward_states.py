@@ -130,3 +130,38 @@ def test_rollouts_of_many_observations(H, W, monkeypatch):
         got.append([out.detach(), xl.grad, Dl.grad, th.grad, outb.detach(), xb.grad, Db.grad])
     for p, q in zip(*got):
         assert torch.isfinite(p).all() and torch.equal(p, q)
+
+
+@pytest.mark.parametrize("H,W,B", [(40, 52, 2), (70, 131, 3), (8, 30, 2)])
+def test_gradients_with_every_state_kept(H, W, B, monkeypatch):
+    """All states kept, against segments of ceil(sqrt(steps)) recomputed: the same bits; and what falls
+    back to segments."""
+    D, x, st = _inputs(H, W)
+    obs = [0, 7, 7, 31, 12]
+    taken = []
+    room = A._room_for_states
+
+    def spied(*a):
+        r = room(*a)
+        taken.append(r is not None)
+        return r
+
+    monkeypatch.setattr(A, "_room_for_states", spied)
+    got = []
+    for seg in (None, 6):
+        Dl, xl = D.clone().requires_grad_(True), x.clone().requires_grad_(True)
+        th = torch.tensor(Pm.PARAMSET_3[:13], device="cuda", requires_grad=True)
+        out = A.rollout(xl[0], xl[1], xl[2], Dl, th, st, 0, 40, obs, seg=seg)
+        (out ** 2).sum().backward()
+        xb = torch.stack([(1 - 0.1 * k) * x for k in range(B)]).requires_grad_(True)
+        outb = A.rollout_batch(xb, Dl, th, [st] * B, 0, 40, obs, seg=seg)
+        (outb ** 2).sum().backward()
+        got.append([out.detach(), xl.grad, Dl.grad, th.grad, outb.detach(), xb.grad])
+    assert taken == [True, True]
+    for p, q in zip(*got):
+        assert torch.isfinite(p).all() and torch.equal(p, q)
+    A.rollout(x[0], x[1], x[2], D, th.detach(), st, 0, 40, obs)  # nothing to differentiate
+    assert taken == [True, True]
+    assert room(0, x) is None and room(A.MOST_KEPT + 1, x) is None
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (0, 1))
+    assert room(10, x) is None
