@@ -23,6 +23,7 @@
 #include <cstdint>
 
 #include "fk_adjoint.cuh"
+#include "fk_capi_internal.h"
 #include "fk_math.cuh"
 #include "fk_ptx.cuh"
 
@@ -530,15 +531,14 @@ __global__ void __launch_bounds__(ANT, 4) fk_adjoint_kernel(const __grid_constan
     adjoint_tile(a, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
-// ---- lines of at least kLineMin cells: two threads per unit of two rows of a quad, one stage -------
+// ---- lines of at least kLineMin cells: two or four threads per unit of two rows of a quad ----------
 // What bounds it: the tile kernel above stages six derivative planes, reads ten-cell products for
 // each cell of the 6-cell edge band, tests every stimulus's protocol in every cell and reduces 13
 // parameter sums over a warp for every two cells (us per step: 39.5 for 16 experiments of 256^2,
 // 10.9 for one 151 x 203 grid, 10.5 for 16 of 64^2).  Here everything comes from one staged tile of
-// u, D and lambda_u and stays in registers: 28.6, 7.1 and 7.9 us.  At 16 x 256^2 a step executes 400
-// instructions per cell at 42 % of the issue slots; one small grid waits for its loads (0.5 us),
-// then for the longest chain of a unit, 2500 cycles for each half of it.  The operations are fewer
-// because they are regrouped:
+// u, D and lambda_u and stays in registers: 24.2, 5.0 and 6.0 us.  At 16 x 256^2 a step executes some
+// 390 instructions per cell, 210 of them the stencils and currents; one small grid waits for its
+// launch (4 us without any work) and then for the longest chain of a unit.  The operations are fewer because they are regrouped:
 //   * both transposed products of an axis share their second operator,
 //       A^T (D mu) + B^T ((B D) mu) = (E^T G^T / dx) (G^T C^T (D mu) / dx + C^T (B D) mu),
 //   * G^T on central rows is -G; the one-sided rows 0 and N-1 (and the pad rows -1 and N in the
@@ -549,14 +549,17 @@ __global__ void __launch_bounds__(ANT, 4) fk_adjoint_kernel(const __grid_constan
 constexpr int kLineMin = 20;  // shorter lines (fewer than three quads or nine rows in a last tile)
                               // take the tile kernel above
 constexpr int LR = 2;         // rows per thread
-constexpr int LG = 8, LQ = 16;                   // most row groups and quads of a tile
-constexpr int LU = LG * LQ;                      // units of a tile; two threads share one
-constexpr int LNT = 2 * LU;
-constexpr int LSW = 4 * LQ + 12;                 // staged row: 4 cells on either side, and 4 more so
-                                                 // that 8 lanes (2 quads of 4 groups) read from 8
-                                                 // different 16-byte banks
-constexpr int LSH = LG * LR + 8 + 1;             // 4 rows above and below; the first group of the
-                                                 // last tile row may reach one row further up
+constexpr int LG = 8;         // most row groups of a tile
+constexpr int LNT = 256;      // threads of a block: two or four share a unit (see fk_adjoint_line_kernel)
+template <int SHARE>
+struct LineTile {
+    static constexpr int LU = LNT / SHARE, LQ = LU / LG;  // units, most quads of a tile
+    static constexpr int LSW = 4 * LQ + 12;  // staged row: 4 cells on either side, and 4 more so that 8 lanes
+                                             // (2 quads of 4 groups) read from 8 different 16-byte banks
+    static constexpr int LSH = LG * LR + 8 + 1;  // 4 rows above and below; the first group of the last
+                                                 // tile row may reach one row further up
+    static constexpr int SMEM = (3 * LSH * LSW + 6 * LR * LU * 4) * 4;
+};
 
 __constant__ float kHeadC[4] = {C_HEAD0, C_THREE, -C_3_2, C_1_3};
 __constant__ float kTailC[4] = {C_TAIL0, C_3_2, -C_THREE, C_TAIL3};
@@ -755,130 +758,170 @@ __device__ __forceinline__ void cp_async16(float *dst, const float *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 
-// Tile (bx, by) of an nbx x nby cut of the grid (rows in groups of LR, columns in quads, dealt out
-// evenly; the last tile row's groups are aligned to the bottom, so that rows 0 and H-1 are the first
-// and the last row of a thread).  Its dL/dtheta sums go to slot by * nbx + bx of a.gtheta.
-__device__ __forceinline__ void adjoint_line_tile(const AdjointArgs &a, int bx, int by, int nbx,
-                                                  int nby) {
-    __shared__ __align__(16) float su[LSH * LSW];
-    __shared__ __align__(16) float sd[LSH * LSW];
-    __shared__ __align__(16) float sl[LSH * LSW];
-    __shared__ float4 sp[4][LR][LU];  // a unit's own v, w, lambda_v, lambda_w; the first then its
-                                      // lambda_u through the currents
-    __shared__ float4 sr[2][LR][LU];  // the x direction's part of lambda_u and of dL/dD
-    __shared__ float red[LU / 32][16];
+// The tiles of a launch: block (x, y, e) takes tile (x, y) of a cut of the grid (rows in groups of LR,
+// columns in quads, dealt out evenly, the larger shares last) of experiment e.  No division is left to the
+// device: a thread has a few cells, and one division costs as much as one of them.
+struct LineRun {
+    int64_t state, lam, plane, theta;  // elements from one experiment to the next: state, cotangent, gD, gtheta
+    const AdjointArgs *exps;           // the experiments' stimuli; null: one experiment, those of the arguments
+    int early;                         // the launch before is the reverse step before, or waits for it
+    int g_each, g_small, q_each, q_small;  // groups (quads) of a tile, and tiles that have one less
+    int inv[2], inv_q[2];                  // 2^16 / groups of a tile (/ its quads + 2), rounded up: for the
+                                           // tiles that have one less, and for the others
+};
+
+// The arguments stay in the constant bank, for many experiments those of the first one and the distance to
+// the others.  With programmatic dependent launch the state and D, which no reverse step writes, are fetched
+// before the step before has ended.  (us per step with the arguments copied from memory and all loads after
+// the step before: 28.4 for 16 experiments of 256^2, 7.1 for 151 x 203, against 24.2 and 5.0.  Blocks that
+// walk over tiles, the next one's loads in flight: 28.1; their shares are fixed, some take four tiles where
+// 3.4 are the mean.)
+//
+// SHARE: threads that share a unit.  What a thread does once per tile (places, addresses, loads, sums) costs
+// it as much as two cells, so many tiles take two threads per unit (tiles of 16 x 64 cells); where all tiles
+// run at once the chain of a thread counts, and four take it (16 x 32).  us per step with 2 | 4: 151 x 203
+// 6.0 | 5.0, 16 of 64^2 6.8 | 6.0, 512^2 (512 tiles of 16 x 32 on 304 places) 7.4 | 9.4, 16 of 256^2
+// 24.2 | 30.3.  (Three blocks per SM, at 80 registers, spill: 512^2 9.5, 16 of 256^2 24.0.)
+template <int SHARE>
+__global__ void __launch_bounds__(LNT, 2)
+    fk_adjoint_line_kernel(const __grid_constant__ AdjointArgs a, const __grid_constant__ LineRun b) {
+    using T_ = LineTile<SHARE>;
+    constexpr int LU = T_::LU, LSW = T_::LSW, LSH = T_::LSH;
+    // u, D, lambda_u with 4 cells around; a unit's own v, w, lambda_v, lambda_w, the first then its lambda_u
+    // through the currents; the x direction's part of lambda_u and of dL/dD
+    extern __shared__ __align__(16) float line_smem[];
+    float *const su = line_smem, *const sd = su + LSH * LSW, *const sl = sd + LSH * LSW;
+    float4(*const sp)[LR][LU] = reinterpret_cast<float4(*)[LR][LU]>(sl + LSH * LSW);
+    float4(*const sr)[LR][LU] = sp + 4;
+    constexpr int PT_WARPS = SHARE == 4 ? 2 * LU / 32 : LU / 32;
+    __shared__ float red[PT_WARPS][16];
     const int tid = threadIdx.x, lane = tid & 31;
     const int role = tid / LU, unit = tid % LU;
     const int H = a.H, W = a.W, pitch = a.pitch;
     const float dt = a.dt, rdx = a.rdx;
-    const int ng = (H + LR - 1) / LR, nq = (W + 3) / 4;
-    const int g0 = by * ng / nby, g1 = (by + 1) * ng / nby;
-    const int c0 = bx * nq / nbx, c1 = (bx + 1) * nq / nbx;
-    const int shift = by == nby - 1 ? ng * LR - H : 0;
-    const int row0 = g0 * LR - shift, j0 = 4 * c0;   // the tile's first group's first row
-    const int rows = (g1 - g0) * LR, tq = c1 - c0;
+
+    const int bx = blockIdx.x, by = blockIdx.y;
+    const int64_t e = blockIdx.z;
+    const int G = b.g_each - (by < b.g_small), tq = b.q_each - (bx < b.q_small);  // groups and quads
+    // the last tile row's groups are aligned to the bottom, so that rows 0 and H-1 are the first and the last
+    // row of a thread; rows above the tile's own belong to the tile above
+    const int shift = by == (int)gridDim.y - 1 ? H & (LR - 1) : 0;
+    const int row0 = (by * b.g_each - min(by, b.g_small)) * LR - shift;  // the first group's first row
+    const int j0 = 4 * (bx * b.q_each - min(bx, b.q_small));
     // units by pairs of quad columns: those near the left and right sides then lie in few warps
-    const int G = g1 - g0, pair = (unit >> 1) / G;
+    const int pair = (unit >> 1) * b.inv[by >= b.g_small] >> 16;
     const bool mine = 2 * pair + (unit & 1) < tq;
     const int lq = mine ? 2 * pair + (unit & 1) : 0, lg = mine ? (unit >> 1) - pair * G : 0;
     const int i0 = row0 + lg * LR, j = j0 + 4 * lq;
-    const int k_lo = by == nby - 1 && lg == 0 ? shift : 0;  // rows before it belong to the tile above
+    const int k_lo = lg == 0 ? shift : 0;  // rows before it belong to the tile above
     const int64_t off0 = (int64_t)i0 * pitch + j;
+    const int64_t e_state = e * b.state, e_lam = e * b.lam, e_plane = e * b.plane;
 
-    // All reads go through L2: with programmatic dependent launch this block may have started before
-    // the step that wrote lambda and dL/dD ended, and L1 is not coherent with the other SMs.
-    // ---- stage u, D, lambda_u with 4 cells around: clamped copies outside the grid, lambda 0 ------
-    constexpr int N4 = LSW / 4, RPP = LNT / N4;  // quads of a staged row, rows per pass
-    if (tid < RPP * N4 && tid % N4 < tq + 2) {
-        const int c = 4 * (tid % N4), jc = j0 - 4 + c;
-        const bool quad_in = jc >= 0 && jc + 3 < W;
-        for (int r = tid / N4; r < rows + 8; r += RPP) {
-            const int i = row0 - 4 + r;
-            const int64_t g = (int64_t)clampi(i, 0, H - 1) * pitch;
-            const int o = r * LSW + c;
-            const bool row_in = i >= 0 && i < H;
-            if (quad_in) {
-                cp_async16(su + o, a.u + g + jc);
-                cp_async16(sd + o, a.D + g + jc);
-                if (row_in) cp_async16(sl + o, a.lu + g + jc);
-                else *reinterpret_cast<float4 *>(sl + o) = make_float4(0.f, 0.f, 0.f, 0.f);
-            } else {
-                // a quad across or beyond the grid's side: the nearest cell in place of those outside
-                const int jn = clampi(jc, 0, 4 * (nq - 1));  // the quad of the row that has it
-                float4 x = __ldcg(reinterpret_cast<const float4 *>(a.u + g + jn));
-                float4 y = __ldcg(reinterpret_cast<const float4 *>(a.D + g + jn));
-                float4 z = __ldcg(reinterpret_cast<const float4 *>(a.lu + g + jn));
-                if (jc < 0) {
-                    x.y = x.z = x.w = x.x;
-                    y.y = y.z = y.w = y.x;
-                }
-                const int n = W - 1 - jn;  // the last cell's place in the quad
-                if (n < 1) x.y = x.x, y.y = y.x;
-                if (n < 2) x.z = x.y, y.z = y.y;
-                if (n < 3) x.w = x.z, y.w = y.z;
-                if (jc > jn) {
-                    x.x = x.y = x.z = x.w;
-                    y.x = y.y = y.z = y.w;
-                }
-                const bool l_in = row_in && jc == jn;
-                z.x = l_in ? z.x : 0.0f;
-                z.y = l_in && n >= 1 ? z.y : 0.0f;
-                z.z = l_in && n >= 2 ? z.z : 0.0f;
-                z.w = l_in && n >= 3 ? z.w : 0.0f;
-                *reinterpret_cast<float4 *>(su + o) = x;
-                *reinterpret_cast<float4 *>(sd + o) = y;
-                *reinterpret_cast<float4 *>(sl + o) = z;
+    // the staged quads that this thread brings in: f(row, quad)
+    auto each_quad = [&](auto f) {
+        const int per = tq + 2, n = (G * LR + 8) * per, inv = b.inv_q[bx >= b.q_small];
+#pragma unroll
+        for (int pass = 0; pass < ((LG * LR + 8) * (T_::LQ + 2) + LNT - 1) / LNT; ++pass) {
+            const int x = tid + pass * LNT, r = x * inv >> 16;
+            if (x < n) f(r, x - r * per);
+        }
+    };
+    // Starts the loads of the state and D, or of the cotangent (all through L2: with programmatic dependent
+    // launch L1 may hold lines of the step before the last).
+    auto load = [&](bool state, bool lam) {
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        each_quad([&](int r, int q) {
+            const int i = row0 - 4 + r, jc = j0 - 4 + 4 * q, o = r * LSW + 4 * q;
+            const bool col_in = jc >= 0 && jc < W;  // (the quads outside: below)
+            const int64_t g = (int64_t)clampi(i, 0, H - 1) * pitch + jc;
+            if (state && col_in) {
+                cp_async16(su + o, a.u + e_state + g);
+                cp_async16(sd + o, a.D + g);
+            }
+            if (lam) {
+                if (col_in && i >= 0 && i < H) cp_async16(sl + o, a.lu + e_lam + g);
+                else *reinterpret_cast<float4 *>(sl + o) = zero;
+            }
+        });
+        // a unit's v, w, lambda_v, lambda_w, dealt out over its threads
+#pragma unroll
+        for (int x = 0; x < 4 / SHARE; ++x) {
+            const int f = role + SHARE * x;
+            if (!(f < 2 ? state : lam)) continue;
+            const float *const src = (f == 0 ? a.v : f == 1 ? a.w : f == 2 ? a.lv : a.lw) + (f < 2 ? e_state : e_lam) + off0;
+#pragma unroll
+            for (int k = 0; k < LR; ++k) {
+                if (mine && k >= k_lo) cp_async16(reinterpret_cast<float *>(&sp[f][k][unit]), src + (int64_t)k * pitch);
+                else sp[f][k][unit] = zero;
             }
         }
+    };
+    if (b.early) load(true, false);
+    grid_dependency_wait();
+    grid_launch_dependents();
+    load(!b.early, true);
+
+    double *const slot = a.gtheta + e * b.theta + (int64_t)(by * (int)gridDim.x + bx) * kAdjParamStride + (tid < 12 ? tid : 0);
+    const double slot_was = a.gtheta && tid < 12 ? __ldcg(slot) : 0.0;  // early: its trip overlaps the work
+    const Stim *const stims = b.exps ? b.exps[e].stim : a.stim;
+    unsigned active = 0;
+    if (role < SHARE / 2) {
+        const int n_stim = b.exps ? b.exps[e].n_stim : a.n_stim;
+        active = __ballot_sync(0xffffffffu, lane < n_stim && stim_active(stims[lane < kMaxStim ? lane : 0], a.t));
     }
-    if (role == 0)
-#pragma unroll
-        for (int k = 0; k < LR; ++k)
-            if (mine && k >= k_lo) {
-                const int64_t o = off0 + (int64_t)k * pitch;  // j < W: the quad lies in the pitched row
-                cp_async16(reinterpret_cast<float *>(&sp[0][k][unit]), a.v + o);
-                cp_async16(reinterpret_cast<float *>(&sp[1][k][unit]), a.w + o);
-                cp_async16(reinterpret_cast<float *>(&sp[2][k][unit]), a.lv + o);
-                cp_async16(reinterpret_cast<float *>(&sp[3][k][unit]), a.lw + o);
-            } else {
-#pragma unroll
-                for (int f = 0; f < 4; ++f) sp[f][k][unit] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-    const unsigned active = __ballot_sync(0xffffffffu, lane < a.n_stim && stim_active(a.stim[lane < kMaxStim ? lane : 0], a.t));
     asm volatile("cp.async.wait_all;" ::: "memory");
+    // A thread's own loads have arrived: at the grid's left and right sides the nearest cell takes the place
+    // of those of u and D outside, zero that of lambda.
+    if (bx == 0 || bx == (int)gridDim.x - 1) {
+        const int n = W - 1 - (j0 + 4 * (tq - 1));  // the last cell's place in the last quad
+        each_quad([&](int r, int c) {
+            const bool left = bx == 0 && c == 1, right = bx == (int)gridDim.x - 1 && c == tq;
+            if (!left && !right) return;
+#pragma unroll
+            for (int f = 0; f < 3; ++f) {
+                float4 *const q = reinterpret_cast<float4 *>(line_smem + f * LSH * LSW + r * LSW) + c;
+                float4 y = *q;
+                if (f < 2 && left) q[-1] = make_float4(y.x, y.x, y.x, y.x);
+                if (right) {
+                    if (n < 1) y.y = f < 2 ? y.x : 0.0f;
+                    if (n < 2) y.z = f < 2 ? y.y : 0.0f;
+                    if (n < 3) y.w = f < 2 ? y.z : 0.0f;
+                    q[0] = y;
+                    if (f < 2) q[1] = make_float4(y.w, y.w, y.w, y.w);
+                }
+            }
+        });
+    }
     __syncthreads();
 
-    double *const slot = a.gtheta + (int64_t)(by * nbx + bx) * kAdjParamStride + (tid < 12 ? tid : 0);
-    const double slot_was = a.gtheta && tid < 12 ? __ldcg(slot) : 0.0;  // early: its trip overlaps the work
-
-    // Role 0 takes the pointwise part, role 1 the x direction (along rows), of the unit's two rows;
-    // then the y direction of row 0 and of row 1: the chain of one thread is half as long.
+    // Four threads of a unit: 0 and 1 take the pointwise part of its two rows, 2 and 3 the two sums of the
+    // x direction (along rows); then each one of the two sums of the y direction of one of the rows.  Two
+    // threads: 0 the pointwise part, 1 the x direction; then each the y direction of one row.
     const int base = (lg * LR + 4) * LSW + 4 * lq + 4;  // the unit's first cell
-    if (role == 0) {
+    if (role < SHARE / 2) {
         const Model &md = a.m;
         float gth[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) gth[k] = 0.0f;
+        for (int q = 0; q < 16; ++q) gth[q] = 0.0f;
 #pragma unroll 1
-        for (int k = 0; k < LR; ++k) {
-            const float4 v4 = sp[0][k][unit], w4 = sp[1][k][unit];
+        for (int k = SHARE == 4 ? role : 0; k < (SHARE == 4 ? role + 1 : LR); ++k) {
+            const bool stored = mine && k >= k_lo;
+            const int64_t o = off0 + (int64_t)k * pitch;
+            float4 v4 = sp[0][k][unit], w4 = sp[1][k][unit];
             float4 lv4 = sp[2][k][unit], lw4 = sp[3][k][unit];
             const float4 u4 = *reinterpret_cast<const float4 *>(su + base + k * LSW);
             const float4 l4 = *reinterpret_cast<const float4 *>(sl + base + k * LSW);
             float4 lj4 = l4;  // lambda_u where the current is the model's
             const int i = i0 + k;
-            const int64_t o = off0 + (int64_t)k * pitch;
-            const bool row_ok = mine && k >= k_lo;
-            if (!row_ok) lj4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j + 3 >= W) {  // columns beyond W (lambda_u is zero there)
-                if (j + 1 >= W) lv4.y = lw4.y = 0.f;
-                if (j + 2 >= W) lv4.z = lw4.z = 0.f;
-                lv4.w = j + 3 >= W ? 0.f : lv4.w;
-                lw4.w = j + 3 >= W ? 0.f : lw4.w;
+            if (!stored) lj4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j + 3 >= W) {  // columns beyond W: whatever lies in the padding (lambda_u is zero there)
+                if (j + 1 >= W) v4.y = w4.y = lv4.y = lw4.y = 0.f;
+                if (j + 2 >= W) v4.z = w4.z = lv4.z = lw4.z = 0.f;
+                if (j + 3 >= W) v4.w = w4.w = lv4.w = lw4.w = 0.f;
             }
-            if (active && row_ok)  // cells whose current a stimulus replaces
+            if (active && stored)  // cells whose current a stimulus replaces
                 for (unsigned x = active; x; x &= x - 1) {
-                    const Stim &st = a.stim[__ffs(x) - 1];
+                    const Stim &st = stims[__ffs(x) - 1];
                     float4 f;
                     if (st.field) {
                         f = __ldg(reinterpret_cast<const float4 *>(st.field + o));
@@ -936,23 +979,23 @@ __device__ __forceinline__ void adjoint_line_tile(const AdjointArgs &a, int bx, 
                 gth[11] += jv;
             }
             sp[0][k][unit] = make_float4(pu[0], pu[1], pu[2], pu[3]);
-            if (row_ok) {
+            if (stored) {
                 if (j + 3 < W) {
-                    *reinterpret_cast<float4 *>(a.olv + o) = make_float4(ov[0], ov[1], ov[2], ov[3]);
-                    *reinterpret_cast<float4 *>(a.olw + o) = make_float4(ow[0], ow[1], ow[2], ow[3]);
+                    *reinterpret_cast<float4 *>(a.olv + e_lam + o) = make_float4(ov[0], ov[1], ov[2], ov[3]);
+                    *reinterpret_cast<float4 *>(a.olw + e_lam + o) = make_float4(ow[0], ow[1], ow[2], ow[3]);
                 } else {
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
                         if (j + c < W) {
-                            a.olv[o + c] = ov[c];
-                            a.olw[o + c] = ow[c];
+                            a.olv[e_lam + o + c] = ov[c];
+                            a.olw[e_lam + o + c] = ow[c];
                         }
                 }
             }
         }
         if (a.gtheta) {
             const float x = warp_sum16(gth);
-            if (lane < 16) red[unit / 32][lane] = x;
+            if (lane < 16) red[tid / 32][lane] = x;
         }
     } else {
         V4 x[LR];
@@ -961,75 +1004,77 @@ __device__ __forceinline__ void adjoint_line_tile(const AdjointArgs &a, int bx, 
         };
         auto of = [&](int f, int t) { return cell(f, t - 4); };
         const bool edge = __any_sync(0xffffffffu, mine && (i0 <= 5 || i0 + LR + 1 >= H - 4)) != 0;
-        if (edge) axis_gd<LR, true, V4>(i0, H, of, cell, x);
-        else axis_gd<LR, false, V4>(i0, H, of, cell, x);
+        auto keep = [&](int f) {
 #pragma unroll
-        for (int k = 0; k < LR; ++k) sr[1][k][unit] = make_float4(x[k].x, x[k].y, x[k].z, x[k].w);
-        if (edge) axis_at<LR, true, V4>(i0, H, of, cell, x);
-        else axis_at<LR, false, V4>(i0, H, of, cell, x);
-#pragma unroll
-        for (int k = 0; k < LR; ++k) sr[0][k][unit] = make_float4(x[k].x, x[k].y, x[k].z, x[k].w);
+            for (int k = 0; k < LR; ++k) sr[f][k][unit] = make_float4(x[k].x, x[k].y, x[k].z, x[k].w);
+        };
+        if (SHARE == 2 || role == 2) {
+            if (edge) axis_gd<LR, true, V4>(i0, H, of, cell, x);
+            else axis_gd<LR, false, V4>(i0, H, of, cell, x);
+            keep(1);
+        }
+        if (SHARE == 2 || role == 3) {
+            if (edge) axis_at<LR, true, V4>(i0, H, of, cell, x);
+            else axis_at<LR, false, V4>(i0, H, of, cell, x);
+            keep(0);
+        }
     }
-    const int k = role;  // LR == 2
+    const int k = role & 1;
     const bool stored = mine && k >= k_lo;
-    const int64_t g = off0 + (int64_t)k * pitch;
+    const bool takes_gd = SHARE == 2 || role < 2, takes_at = SHARE == 2 || role >= 2;
+    const int64_t o = off0 + (int64_t)k * pitch;
     float4 gd4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (a.gD && stored) gd4 = __ldcg(reinterpret_cast<const float4 *>(a.gD + g));
+    if (takes_gd && a.gD && stored) gd4 = __ldcg(reinterpret_cast<const float4 *>(a.gD + e_plane + o));
     float ay[4], gy[4];
     {
-        const int o = base + k * LSW;
-        auto cell = [&](int f, int d) { return (f == 0 ? su : f == 1 ? sd : sl)[o + d]; };
+        const int c0 = base + k * LSW;
+        auto cell = [&](int f, int d) { return (f == 0 ? su : f == 1 ? sd : sl)[c0 + d]; };
         float L[12], F[12];
         auto row = [&](const float *p, float (&x)[12]) {
 #pragma unroll
             for (int t = 0; t < 3; ++t) {
-                const float4 y = *reinterpret_cast<const float4 *>(p + o + 4 * t - 4);
-                x[4 * t] = y.x, x[4 * t + 1] = y.y, x[4 * t + 2] = y.z, x[4 * t + 3] = y.w;
+                const float4 q = *reinterpret_cast<const float4 *>(p + c0 + 4 * t - 4);
+                x[4 * t] = q.x, x[4 * t + 1] = q.y, x[4 * t + 2] = q.z, x[4 * t + 3] = q.w;
             }
         };
-        row(sl, L);
-        row(su, F);
-        auto of = [&](int f, int t) { return f == 2 ? L[t] : F[t]; };
         const bool edge = __any_sync(0xffffffffu, mine && (j <= 5 || j + 5 >= W - 4)) != 0;
-        if (edge) axis_gd<4, true, float>(j, W, of, cell, gy);
-        else axis_gd<4, false, float>(j, W, of, cell, gy);
-        row(sd, F);
-        if (edge) axis_at<4, true, float>(j, W, of, cell, ay);
-        else axis_at<4, false, float>(j, W, of, cell, ay);
-    }
-    __syncthreads();
-    if (stored) {
-        const float c2 = rdx * rdx * dt;
-        const float4 pu = sp[0][k][unit], ax = sr[0][k][unit], gx = sr[1][k][unit];
-        const float4 r = make_float4(fmaf(c2, ax.x + ay[0], pu.x), fmaf(c2, ax.y + ay[1], pu.y),
-                                     fmaf(c2, ax.z + ay[2], pu.z), fmaf(c2, ax.w + ay[3], pu.w));
-        gd4 = make_float4(fmaf(c2, gx.x + gy[0], gd4.x), fmaf(c2, gx.y + gy[1], gd4.y),
-                          fmaf(c2, gx.z + gy[2], gd4.z), fmaf(c2, gx.w + gy[3], gd4.w));
-        if (j + 3 < W) {
-            *reinterpret_cast<float4 *>(a.olu + g) = r;
-            if (a.gD) __stcg(reinterpret_cast<float4 *>(a.gD + g), gd4);
-        } else {
-            const float rr[4] = {r.x, r.y, r.z, r.w}, ee[4] = {gd4.x, gd4.y, gd4.z, gd4.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (j + c < W) {
-                    a.olu[g + c] = rr[c];
-                    if (a.gD) __stcg(a.gD + g + c, ee[c]);
-                }
+        row(sl, L);
+        row(takes_gd ? su : sd, F);
+        auto of = [&](int f, int t) { return f == 2 ? L[t] : F[t]; };
+        if (takes_gd) {
+            if (edge) axis_gd<4, true, float>(j, W, of, cell, gy);
+            else axis_gd<4, false, float>(j, W, of, cell, gy);
+        }
+        if (takes_at) {
+            if (takes_gd) row(sd, F);
+            if (edge) axis_at<4, true, float>(j, W, of, cell, ay);
+            else axis_at<4, false, float>(j, W, of, cell, ay);
         }
     }
+    __syncthreads();
+    // (rdx^2 and dt apart: their product rounds, the same way in every step)
+    const float r2 = rdx * rdx;
+    // r2 dt (x + y) onto z, stored to `out`
+    auto put = [&](float4 x, const float (&y)[4], float4 z, float *out) {
+        z = make_float4(fmaf(r2, dt * (x.x + y[0]), z.x), fmaf(r2, dt * (x.y + y[1]), z.y),
+                        fmaf(r2, dt * (x.z + y[2]), z.z), fmaf(r2, dt * (x.w + y[3]), z.w));
+        if (j + 3 < W) {
+            __stcg(reinterpret_cast<float4 *>(out), z);
+        } else {
+            const float zz[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (j + c < W) __stcg(out + c, zz[c]);
+        }
+    };
+    if (stored && takes_at) put(sr[0][k][unit], ay, sp[0][k][unit], a.olu + e_lam + o);
+    if (stored && takes_gd && a.gD) put(sr[1][k][unit], gy, gd4, a.gD + e_plane + o);
     if (a.gtheta && tid < 12) {
         double x = 0.0;
 #pragma unroll
-        for (int w = 0; w < LU / 32; ++w) x += (double)red[w][tid];
+        for (int w = 0; w < PT_WARPS; ++w) x += (double)red[w][tid];
         __stcg(slot, fma(a.theta_factor[tid], x, slot_was));
     }
-}
-
-__global__ void __launch_bounds__(LNT, 2) fk_adjoint_line_kernel(const __grid_constant__ AdjointArgs a) {
-    grid_dependency_wait();
-    grid_launch_dependents();
-    adjoint_line_tile(a, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
 }
 
 // The device copy of an experiment's arguments, moved to step k of its segment (see
@@ -1070,35 +1115,63 @@ __global__ void __launch_bounds__(ANT, 4) fk_adjoint_batch_kernel(const AdjointA
     adjoint_tile(sa, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
-__global__ void __launch_bounds__(LNT, 2)
-    fk_adjoint_line_batch_kernel(const AdjointArgs *__restrict__ exps, int64_t k_stride, int k,
-                                 int parity, float t) {
-    __shared__ __align__(16) AdjointArgs sa;
-    grid_dependency_wait();
-    grid_launch_dependents();
-    stage_experiment(sa, exps, k_stride, k, parity, t);
-    adjoint_line_tile(sa, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y);
-}
-
 // Which kernel takes a grid, and its blocks.
 bool long_lines(int H, int W) { return H >= kLineMin && W >= kLineMin; }
 dim3 adjoint_grid(int H, int W, int n_exp) {
-    if (!long_lines(H, W)) return dim3((W + ATX - 1) / ATX, (H + ATY - 1) / ATY, n_exp);
-    return dim3(((W + 3) / 4 + LQ - 1) / LQ, ((H + LR - 1) / LR + LG - 1) / LG, n_exp);
+    return dim3((W + ATX - 1) / ATX, (H + ATY - 1) / ATY, n_exp);
+}
+template <int SHARE>
+dim3 line_grid(int H, int W) {
+    constexpr int LQ = LineTile<SHARE>::LQ;
+    return dim3(((W + 3) / 4 + LQ - 1) / LQ, ((H + LR - 1) / LR + LG - 1) / LG);
 }
 
-template <class K, class... A>
-cudaError_t launch_line(K kernel, dim3 grid, cudaStream_t stream, A... args) {
+template <int SHARE>
+cudaError_t launch_line_as(const AdjointArgs &a, LineRun b, int n_exp, cudaStream_t stream) {
+    const dim3 cut = line_grid<SHARE>(a.H, a.W);
+    const int ng = (a.H + LR - 1) / LR, nq = (a.W + 3) / 4, nbx = (int)cut.x, nby = (int)cut.y;
+    b.g_each = (ng + nby - 1) / nby;
+    b.g_small = b.g_each * nby - ng;
+    b.q_each = (nq + nbx - 1) / nbx;
+    b.q_small = b.q_each * nbx - nq;
+    for (int q = 0; q < 2; ++q) {  // (shares of five groups, or three quads, at least)
+        b.inv[q] = (65536 + b.g_each - 2 + q) / (b.g_each - 1 + q);
+        b.inv_q[q] = (65536 + b.q_each + q) / (b.q_each + 1 + q);
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
+    cfg.gridDim = dim3(nbx, nby, n_exp);
     cfg.blockDim = dim3(LNT);
+    cfg.dynamicSmemBytes = LineTile<SHARE>::SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
+    return cudaLaunchKernelEx(&cfg, fk_adjoint_line_kernel<SHARE>, a, b);
+}
+
+cudaError_t launch_line(const AdjointArgs &a, LineRun b, int n_exp, bool chained, cudaStream_t stream) {
+    // the attribute is per function and per context: set again whenever the context changes
+    static thread_local uint64_t configured_ctx = 0;
+    static thread_local int n_sm = 0;
+    if (context_changed(configured_ctx)) {
+        cudaError_t e;
+        int dev = -1;
+        if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+            (e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+            (e = cudaFuncSetAttribute(fk_adjoint_line_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      LineTile<2>::SMEM)) != cudaSuccess ||
+            (e = cudaFuncSetAttribute(fk_adjoint_line_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      LineTile<4>::SMEM)) != cudaSuccess) {
+            configured_ctx = 0;
+            return e;
+        }
+    }
+    b.early = chained;
+    const dim3 cut = line_grid<4>(a.H, a.W);
+    const bool at_once = (int64_t)cut.x * cut.y * n_exp <= 2 * n_sm;
+    return at_once ? launch_line_as<4>(a, b, n_exp, stream) : launch_line_as<2>(a, b, n_exp, stream);
 }
 
 }  // namespace
@@ -1124,25 +1197,47 @@ void set_theta_factors(AdjointArgs &a) {
 }
 
 int64_t adjoint_slots(int H, int W) {
-    const dim3 g = adjoint_grid(H, W, 1);
+    const dim3 g = long_lines(H, W) ? line_grid<4>(H, W) : adjoint_grid(H, W, 1);
     return (int64_t)g.x * g.y;
 }
 
-cudaError_t launch_adjoint(const AdjointArgs &a, cudaStream_t stream) {
-    const dim3 grid = adjoint_grid(a.H, a.W, 1);
-    if (long_lines(a.H, a.W)) return launch_line(fk_adjoint_line_kernel, grid, stream, a);
-    fk_adjoint_kernel<<<grid, ANT, 0, stream>>>(a);
+cudaError_t launch_adjoint(const AdjointArgs &a, bool chained, cudaStream_t stream) {
+    if (long_lines(a.H, a.W)) {
+        return launch_line(a, LineRun{}, 1, chained, stream);
+    }
+    fk_adjoint_kernel<<<adjoint_grid(a.H, a.W, 1), ANT, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_batch(const AdjointArgs *exps, int n_exp, int H, int W, int64_t k_stride,
-                                 int k, int parity, float t, cudaStream_t stream) {
+cudaError_t launch_adjoint_batch(const AdjointArgs &first, const AdjointArgs *exps, int n_exp, int64_t exp_stride,
+                                 int k, int parity, float t, bool chained, cudaStream_t stream) {
     if (n_exp < 1) return cudaSuccess;
-    const dim3 grid = adjoint_grid(H, W, n_exp);
-    if (long_lines(H, W))
-        return launch_line(fk_adjoint_line_batch_kernel, grid, stream, exps, k_stride, k, parity, t);
-    fk_adjoint_batch_kernel<<<grid, ANT, 0, stream>>>(exps, k_stride, k, parity, t);
-    return cudaGetLastError();
+    const int64_t plane = (int64_t)first.H * first.pitch, ns = 3 * plane;
+    if (!long_lines(first.H, first.W)) {
+        fk_adjoint_batch_kernel<<<adjoint_grid(first.H, first.W, n_exp), ANT, 0, stream>>>(exps, ns, k, parity, t);
+        return cudaGetLastError();
+    }
+    AdjointArgs a = first;
+    a.u += k * ns;
+    a.v += k * ns;
+    a.w += k * ns;
+    a.t = t;
+    if (parity) {
+        const float *const lu = a.lu, *const lv = a.lv, *const lw = a.lw;
+        a.lu = a.olu;
+        a.lv = a.olv;
+        a.lw = a.olw;
+        a.olu = const_cast<float *>(lu);
+        a.olv = const_cast<float *>(lv);
+        a.olw = const_cast<float *>(lw);
+    }
+    LineRun b{};
+    b.exps = exps;
+    b.state = exp_stride;
+    b.lam = ns;
+    b.plane = plane;
+    b.theta = adjoint_slots(a.H, a.W) * kAdjParamStride;
+    return launch_line(a, b, n_exp, chained, stream);
 }
 
 }  // namespace fk

@@ -32,10 +32,14 @@ void set_theta_factors(AdjointArgs &a);
 
 // Number of dL/dtheta slots (kAdjParamStride doubles each) written by launch_adjoint.
 int64_t adjoint_slots(int H, int W);
-cudaError_t launch_adjoint(const AdjointArgs &a, cudaStream_t stream);
-// Reverse step k of a segment for n_exp experiments of the same H x W grid (device descriptors
-// `exps`, see fk_adjoint_batch_kernel); parity selects the cotangent buffer read.
-cudaError_t launch_adjoint_batch(const AdjointArgs *exps, int n_exp, int H, int W, int64_t k_stride,
-                                 int k, int parity, float t, cudaStream_t stream);
+// One reverse step.  chained: the launch before it on the stream is the reverse step before it, or waits
+// for that one in full, so that the state and D may be read before it has ended.
+cudaError_t launch_adjoint(const AdjointArgs &a, bool chained, cudaStream_t stream);
+// Reverse step k of a segment for n_exp experiments of one grid that share D and the parameters:
+// `first` (and, in device memory, exps[0]) describes step 0 of the first one's segment, the others' states
+// lie exp_stride floats apart and their cotangents, dL/dD and slots one after the other; exps[e] has the
+// stimuli of experiment e.  parity selects the cotangent buffer read.
+cudaError_t launch_adjoint_batch(const AdjointArgs &first, const AdjointArgs *exps, int n_exp, int64_t exp_stride,
+                                 int k, int parity, float t, bool chained, cudaStream_t stream);
 
 }  // namespace fk

@@ -1061,10 +1061,11 @@ int64_t fk_adjoint_slots(fk_grid g) {
     return adjoint_slots((int)g.H, (int)g.W);
 }
 
-int fk_adjoint_step(fk_grid g, const float *state, const float *D, const fk_params *p,
+// chained: see launch_adjoint.
+static int adjoint_step(fk_grid g, const float *state, const float *D, const fk_params *p,
                     const fk_stimulus *stimuli, int n_stimuli, int64_t t, double dt, double dx,
                     const float *lam_next, float *lam, float *grad_D, double *grad_theta_slots,
-                    void *stream) {
+                    bool chained, void *stream) {
     int rc = common_checks(g, state, lam, D, p, dx);
     if (rc) return rc;
     if (!lam_next) return FK_ERR_NULL;
@@ -1094,7 +1095,15 @@ int fk_adjoint_step(fk_grid g, const float *state, const float *D, const fk_para
     a.n_stim = n_stimuli;
     a.m = make_model(*p);
     set_theta_factors(a);
-    return launch_adjoint(a, (cudaStream_t)stream) == cudaSuccess ? FK_OK : FK_ERR_CUDA;
+    return launch_adjoint(a, chained, (cudaStream_t)stream) == cudaSuccess ? FK_OK : FK_ERR_CUDA;
+}
+
+int fk_adjoint_step(fk_grid g, const float *state, const float *D, const fk_params *p,
+                    const fk_stimulus *stimuli, int n_stimuli, int64_t t, double dt, double dx,
+                    const float *lam_next, float *lam, float *grad_D, double *grad_theta_slots,
+                    void *stream) {
+    return adjoint_step(g, state, D, p, stimuli, n_stimuli, t, dt, dx, lam_next, lam, grad_D, grad_theta_slots,
+                        false, stream);
 }
 
 size_t fk_adjoint_batch_workspace_bytes(int n_exp) {
@@ -1158,8 +1167,8 @@ int fk_adjoint_batch_range(int n_exp, fk_grid g, const float *bufs, int64_t exp_
         return FK_ERR_CUDA;
     // reverse step r (k = n-1-r) reads buffer r&1 (0: lam, 1: lam_tmp) and writes the other
     for (int64_t k = n - 1, r = 0; k >= 0; --k, ++r) {
-        if (launch_adjoint_batch(dexp, n_exp, (int)g.H, (int)g.W, ns, (int)k, (int)(r & 1),
-                                 (float)(s + k), cs) != cudaSuccess)
+        if (launch_adjoint_batch(h[0], dexp, n_exp, exp_stride, (int)k, (int)(r & 1), (float)(s + k), r > 0, cs) !=
+            cudaSuccess)
             return FK_ERR_CUDA;
         float *cur = (r & 1) ? lam : lam_tmp;
         for (int j = 0; j < n_inj; ++j)
@@ -1247,8 +1256,8 @@ int fk_adjoint_range(fk_grid g, const float *buf, int64_t s, int64_t n, const fl
     cudaStream_t cs = (cudaStream_t)stream;
     float *cur = lam, *other = lam_tmp;
     for (int64_t k = n - 1; k >= 0; --k) {
-        rc = fk_adjoint_step(g, buf + k * ns, D, p, stimuli, n_stimuli, s + k, dt, dx, cur, other,
-                             grad_D, grad_theta_slots, stream);
+        rc = adjoint_step(g, buf + k * ns, D, p, stimuli, n_stimuli, s + k, dt, dx, cur, other, grad_D,
+                          grad_theta_slots, k < n - 1, stream);
         if (rc) return rc;
         float *tmp = cur;
         cur = other;

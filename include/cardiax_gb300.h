@@ -397,7 +397,8 @@ int fk_batch_forward_states(fk_batch *plan, int64_t t0, const int64_t *steps, fl
 /* Batched reverse pass: E experiments on one grid that share D and the parameters (each with
  * its own stimuli and state), as in an inverse problem fitted to several recordings.  No
  * reference counterpart.  Per experiment the results equal fk_recompute / fk_adjoint_range bit
- * for bit; every step is one launch for all experiments.
+ * for bit, but for the grouping of dL/dtheta's partial sums (the tiles depend on how many there are);
+ * every step is one launch for all experiments.
  *
  * fk_batch_recompute: `plan` holds the E experiments as its tissues (one grid, no activation
  * tracking); each tissue's state buffer holds x_s on entry.  Writes x_s .. x_{s+n-1} of tissue
