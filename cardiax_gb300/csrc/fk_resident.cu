@@ -8,8 +8,8 @@
 // updates its cells; then the cells within 4 of a tile side go to the neighbour through global
 // memory.  Only u is exchanged, only with the 4 direct neighbours: no stencil is diagonal.
 //
-// What bounds it (us per step, GB300; one launch per step before): 256^2 2.00 (4.4), 512^2 2.43
-// (4.5), 1024^2 5.67 (8.2), 1200^2 6.49 (9.7).  One launch per step pays launch, load and store
+// What bounds it (us per step, GB300; one launch per step before): 256^2 2.04 (4.4), 512^2 2.38
+// (4.5), 1024^2 5.31 (8.2), 1200^2 6.02 (9.7).  One launch per step pays launch, load and store
 // latencies in a row whatever it computes.  Here a small grid's step is one dependent chain: about
 // 1000 cycles for a unit of 8 cells (1600 at the grid's edge), 1700 from a strip's store to its
 // neighbour's load of it through L2, and two barriers.  A large grid's step is bound by issue
@@ -497,6 +497,39 @@ __global__ void __launch_bounds__(512, 1)
                     any(i0 <= (R == 2 ? 2 : 0)), any(i0 + R + (R == 2 ? 2 : 0) >= H)};
     int next_out = 0, next_step = ra.every ? 1 : ra.out_step[0];
 
+    // a state that is written out
+    auto write_out = [&](int s, const float *nxt) {
+        if (s + 1 != next_step) return;
+        const int64_t base = ra.every ? (int64_t)(s + 1) * ra.every : ra.out_off[next_out];
+        float *const out = MANY && ra.base ? ra.base + tis.id * ra.tissue_stride : a.vo;
+        const int64_t plane = (int64_t)H * pitch;
+        ++next_out;
+        next_step = ra.every ? s + 2 : next_out < ra.n_out ? ra.out_step[next_out] : 0;
+        if (mine)
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                if (k < k_lo) continue;
+                float *g = out + base + off0 + (int64_t)k * pitch;
+                const float4 x = ld4(nxt + ucell + k * SUW);
+                if (j + 3 < W) {
+                    __stcg(reinterpret_cast<float4 *>(g), v[k]);
+                    __stcg(reinterpret_cast<float4 *>(g + plane), w[k]);
+                    __stcg(reinterpret_cast<float4 *>(g + 2 * plane), x);
+                } else {
+                    const float fv[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+                    const float fw[4] = {w[k].x, w[k].y, w[k].z, w[k].w};
+                    const float fu[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (int m = 0; m < 4; ++m)
+                        if (j + m < W) {
+                            __stcg(g + m, fv[m]);
+                            __stcg(g + plane + m, fw[m]);
+                            __stcg(g + 2 * plane + m, fu[m]);
+                        }
+                }
+            }
+    };
+
     for (int s = 0; s < ra.n; ++s) {
         const float *cur = su + (s & 1) * SU;
         float *nxt = su + ((s + 1) & 1) * SU;
@@ -506,46 +539,25 @@ __global__ void __launch_bounds__(512, 1)
         if (mine)
             step_unit<R, ACT>(a, tconst, kc, unit, cur + ucell, nxt + ucell, SUW, sD + tid, nthr, v, w,
                               active, (float)(ra.t0 + s));
-        if (s + 1 == next_step) {  // a state that is written out
-            const int64_t base = ra.every ? (int64_t)(s + 1) * ra.every : ra.out_off[next_out];
-            float *const out = MANY && ra.base ? ra.base + tis.id * ra.tissue_stride : a.vo;
-            const int64_t plane = (int64_t)H * pitch;
-            ++next_out;
-            next_step = ra.every ? s + 2 : next_out < ra.n_out ? ra.out_step[next_out] : 0;
-            if (mine)
-#pragma unroll
-                for (int k = 0; k < R; ++k) {
-                    if (k < k_lo) continue;
-                    float *g = out + base + off0 + (int64_t)k * pitch;
-                    const float4 x = ld4(nxt + ucell + k * SUW);
-                    if (j + 3 < W) {
-                        __stcg(reinterpret_cast<float4 *>(g), v[k]);
-                        __stcg(reinterpret_cast<float4 *>(g + plane), w[k]);
-                        __stcg(reinterpret_cast<float4 *>(g + 2 * plane), x);
-                    } else {
-                        const float fv[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
-                        const float fw[4] = {w[k].x, w[k].y, w[k].z, w[k].w};
-                        const float fu[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                        for (int m = 0; m < 4; ++m)
-                            if (j + m < W) {
-                                __stcg(g + m, fv[m]);
-                                __stcg(g + plane + m, fw[m]);
-                                __stcg(g + 2 * plane + m, fu[m]);
-                            }
-                    }
+        const int64_t par = (s & 1) * ra.slot;
+        // Where the stores of a written state stand: of many tissues ahead of the barrier, where those of the warps
+        // that are done overlap with the others' work (every state of 16 x 256^2: 9.7 us per step, behind the
+        // strips 9.9); of one tissue behind the strips, out of the way of the code of a step that writes none
+        // (1200^2 6.02 against 6.46 us, 1024^2 5.31 against 5.60, 128^2 1.83 against 1.89).
+        if (MANY) write_out(s, nxt);
+        if (!last) {
+            if (tid < 32 && (s & 31) == 31) fill_active(s + 1);
+            __syncthreads();
+            // ---- this tile's strips out, and the neighbours' into the next buffer's halo ----------
+            if (tid < n_ring)
+                for (int it = tid; it < n_items; it += n_ring) {
+                    if (it != tid) locate_out(it, out_src, out_dst);
+                    send_quad(out_strips + par + out_dst, ld4(nxt + out_src), tag);
                 }
         }
+        if (!MANY) write_out(s, nxt);
         if (last) return;
-        if (tid < 32 && (s & 31) == 31) fill_active(s + 1);
-        __syncthreads();
-        // ---- this tile's strips out, and the neighbours' into the next buffer's halo --------------
         if (tid < n_ring) {
-            const int64_t par = (s & 1) * ra.slot;
-            for (int it = tid; it < n_items; it += n_ring) {
-                if (it != tid) locate_out(it, out_src, out_dst);
-                send_quad(out_strips + par + out_dst, ld4(nxt + out_src), tag);
-            }
             for (int it = tid; it < n_items; it += n_ring) {
                 if (it != tid) locate(it, in_src, in_dst);
                 float4 q;
