@@ -69,6 +69,9 @@ def _lib():
         L.fk_batch_recompute.restype = ctypes.c_int
         L.fk_batch_recompute.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                          ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]
+        L.fk_adjoint_sum.restype = ctypes.c_int
+        L.fk_adjoint_sum.argtypes = [ctypes.c_int, N.Grid, ctypes.c_void_p, ctypes.c_void_p,
+                                     ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
         L.fk_adjoint_batch_range.restype = ctypes.c_int
         L.fk_adjoint_batch_range.argtypes = [
             ctypes.c_int, N.Grid, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64,
@@ -263,6 +266,18 @@ def _states_at(advance, run, t0: int, marks, own, state: torch.Tensor, take) -> 
     return cur
 
 
+def _summed(grid, gD: torch.Tensor, gtheta: torch.Tensor):
+    """dL/dD (H, W) and dL/dtheta (13 values) summed over the experiments (first dimension), in their
+    order, and the slots."""
+    out_D = torch.empty((grid.H, grid.W), dtype=torch.float32, device=gD.device)
+    out_theta = torch.empty(N_THETA, dtype=torch.float32, device=gD.device)
+    rc = _lib().fk_adjoint_sum(gD.shape[0], grid, gD.data_ptr(), gtheta.data_ptr(), out_D.data_ptr(),
+                               out_theta.data_ptr(), stream_handle())
+    if rc:
+        raise N.FkError(rc, "fk_adjoint_sum")
+    return out_D, out_theta
+
+
 class _Rollout(torch.autograd.Function):
     """States at ``obs_times`` of a rollout, differentiable w.r.t. (v0, w0, u0, D, theta)."""
 
@@ -303,8 +318,8 @@ class _Rollout(torch.autograd.Function):
         lam0 = adj.rollout_gradient(state0, ctx.t0, ctx.t1, ctx.obs_times, g, seg=ctx.seg,
                                     ckpts=ctx.ckpts, states=ctx.states)
         ctx.ckpts = ctx.states = None
-        gth = adj.grad_theta().to(torch.float32)
-        return (lam0[0, :, :W], lam0[1, :, :W], lam0[2, :, :W], adj.grad_D().clone(), gth,
+        gD, gth = _summed(tis.grid, adj.gD[None], adj.gtheta[None])
+        return (lam0[0, :, :W], lam0[1, :, :W], lam0[2, :, :W], gD, gth,
                 None, None, None, None, None, None, None, None)
 
 
@@ -481,14 +496,10 @@ class _RolloutBatch(torch.autograd.Function):
             if rc:
                 raise N.FkError(rc, "fk_adjoint_batch_range")
         ctx.ckpts = ctx.states = None
-        gD_sum = gD[0, :, :W].clone()
-        gth_sum = gth[0, :, :N_THETA].sum(0)
-        for b in range(1, B):  # fixed order: deterministic sums
-            gD_sum += gD[b, :, :W]
-            gth_sum = gth_sum + gth[b, :, :N_THETA].sum(0)
+        gD_sum, gth_sum = _summed(bp.grid, gD, gth)
         ctx.bp = None
         bp.close()
-        return (lam[..., :W], gD_sum, gth_sum.to(torch.float32), None, None, None, None, None,
+        return (lam[..., :W], gD_sum, gth_sum, None, None, None, None, None,
                 None, None, None)
 
 

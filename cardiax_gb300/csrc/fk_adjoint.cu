@@ -1115,6 +1115,43 @@ __global__ void __launch_bounds__(ANT, 4) fk_adjoint_batch_kernel(const AdjointA
     adjoint_tile(sa, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
+// Sums over the experiments in their order: dL/dD to the dense H x W plane oD, and (the last block) dL/dtheta,
+// over the slots as well, to oth.
+__global__ void __launch_bounds__(32 * kAdjParams)
+    fk_adjoint_sum_kernel(const float *gD, const double *gtheta, int n_exp, int H, int W, int pitch, int slots,
+                          float *oD, float *oth) {
+    if (blockIdx.x == gridDim.x - 1) {
+        const int p = threadIdx.x / 32, lane = threadIdx.x % 32;
+        double sum = 0.0;
+        for (int e = 0; e < n_exp; ++e) {
+            double x = 0.0;
+            for (int k = lane; k < slots; k += 32) x += __ldg(gtheta + ((int64_t)e * slots + k) * kAdjParamStride + p);
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            sum += x;
+        }
+        if (lane == 0) oth[p] = (float)sum;
+        return;
+    }
+    const int64_t plane = (int64_t)H * pitch, quads = (int64_t)H * (pitch / 4);
+    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < quads;
+         x += (int64_t)(gridDim.x - 1) * blockDim.x) {
+        const int i = (int)(x / (pitch / 4)), j = 4 * (int)(x - (int64_t)i * (pitch / 4));
+        if (j >= W) continue;
+        const float *src = gD + (int64_t)i * pitch + j;
+        float4 s = __ldg(reinterpret_cast<const float4 *>(src));
+#pragma unroll 8
+        for (int e = 1; e < n_exp; ++e) {
+            const float4 y = __ldg(reinterpret_cast<const float4 *>(src + e * plane));
+            s = make_float4(s.x + y.x, s.y + y.y, s.z + y.z, s.w + y.w);
+        }
+        float *out = oD + (int64_t)i * W + j;
+        const float f[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            if (j + m < W) out[m] = f[m];
+    }
+}
+
 // Which kernel takes a grid, and its blocks.
 bool long_lines(int H, int W) { return H >= kLineMin && W >= kLineMin; }
 dim3 adjoint_grid(int H, int W, int n_exp) {
@@ -1238,6 +1275,15 @@ cudaError_t launch_adjoint_batch(const AdjointArgs &first, const AdjointArgs *ex
     b.plane = plane;
     b.theta = adjoint_slots(a.H, a.W) * kAdjParamStride;
     return launch_line(a, b, n_exp, chained, stream);
+}
+
+cudaError_t launch_adjoint_sum(const float *gD, const double *gtheta, int n_exp, int H, int W, int pitch, float *oD,
+                               float *oth, cudaStream_t stream) {
+    const int64_t quads = (int64_t)H * (pitch / 4), n = 32 * kAdjParams;
+    const int64_t blocks = (quads + n - 1) / n;
+    fk_adjoint_sum_kernel<<<(int)(blocks < 1024 ? blocks : 1024) + 1, (int)n, 0, stream>>>(
+        gD, gtheta, n_exp, H, W, pitch, (int)adjoint_slots(H, W), oD, oth);
+    return cudaGetLastError();
 }
 
 }  // namespace fk

@@ -1184,6 +1184,18 @@ int fk_adjoint_batch_range(int n_exp, fk_grid g, const float *bufs, int64_t exp_
     return FK_OK;
 }
 
+int fk_adjoint_sum(int n_exp, fk_grid g, const float *grad_D, const double *grad_theta_slots, float *out_D,
+                   float *out_theta, void *stream) {
+    if (int rc = check_grid(g)) return rc;
+    if (!grad_D || !grad_theta_slots || !out_D || !out_theta) return FK_ERR_NULL;
+    if (n_exp < 1) return FK_ERR_ARGUMENT;
+    if (!aligned16(grad_D)) return FK_ERR_ALIGN;
+    return launch_adjoint_sum(grad_D, grad_theta_slots, n_exp, (int)g.H, (int)g.W, (int)g.pitch, out_D, out_theta,
+                              (cudaStream_t)stream) == cudaSuccess
+               ? FK_OK
+               : FK_ERR_CUDA;
+}
+
 int fk_recompute(fk_grid g, const float *state, int64_t s, int64_t n, const float *D,
                  const fk_params *p, const fk_stimulus *stimuli, int n_stimuli, double dt,
                  double dx, float *buf, void *stream) {

@@ -421,6 +421,11 @@ int fk_adjoint_batch_range(int n_exp, fk_grid g, const float *bufs, int64_t exp_
                            const float *const *inj_grads, int n_inj, float *grad_D,
                            double *grad_theta_slots, void *workspace, size_t workspace_bytes,
                            void *stream);
+/* Sums over E experiments, in their order: grad_D (E planes) to out_D (H * W floats without row padding),
+ * grad_theta_slots over the slots as well to out_theta (13 floats). */
+int fk_adjoint_sum(int n_exp, fk_grid g, const float *grad_D, const double *grad_theta_slots, float *out_D,
+                   float *out_theta, void *stream);
+
 
 #ifdef __cplusplus
 }

@@ -74,3 +74,25 @@ def test_many_experiments_equal_one_at_a_time(H, W, E, n):
         assert torch.equal(one[0][0], many[0][e]) and torch.equal(one[1][0], many[1][e])
         d = (one[2][0] - many[2][e]).norm() / one[2][0].norm()
         assert float(d) < 2.2e-4
+
+
+@pytest.mark.parametrize("H,W,E", [(16, 16, 1), (21, 35, 3), (64, 65, 17), (300, 131, 2)])
+def test_sums_over_the_experiments(H, W, E):
+    """dL/dD: the same float32 additions in the same order.  dL/dtheta: float64 sums of some thousand terms of
+    one sign, 1e3 * 2^-53 apart at most, then rounded once to float32."""
+    L = A._lib()
+    pitch = A.pitch_of(W)
+    grid = N.Grid(H, W, pitch)
+    g = torch.Generator().manual_seed(7)
+    gD = torch.full((E, H, pitch), float("nan"))
+    gD[..., :W] = torch.randn((E, H, W), generator=g)
+    gD = gD.cuda()
+    gth = torch.rand((E, int(L.fk_adjoint_slots(grid)), 16), generator=g, dtype=torch.float64).cuda()
+    oD, oth = torch.full((H * W + 8,), 7.0, device="cuda"), torch.full((16,), 7.0, device="cuda")
+    assert L.fk_adjoint_sum(E, grid, gD.data_ptr(), gth.data_ptr(), oD.data_ptr(), oth.data_ptr(), stream_handle()) == 0
+    want = gD[0, :, :W].clone()
+    for e in range(1, E):
+        want += gD[e, :, :W]
+    assert torch.equal(oD[:H * W].view(H, W), want) and (oD[H * W:] == 7.0).all() and (oth[13:] == 7.0).all()
+    ref = gth[..., :13].sum((0, 1))
+    assert ((oth[:13].double() - ref).abs() <= 2.0 ** -24 * ref * (1 + 1e-6)).all()
