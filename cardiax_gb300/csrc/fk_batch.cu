@@ -425,7 +425,7 @@ int run_resident(const fk_batch *b, int64_t t0, int64_t n, const ResOut &out, cu
                 }
             }
             if (cudaMemsetAsync(b->d_xchg, 0, (size_t)(w.ctas * 2 * ra.slot) * 8, s) != cudaSuccess ||
-                launch_resident(w.rows, w.ctas, w.threads, w.smem, ra, a, s) != cudaSuccess)
+                launch_resident(w.rows, w.ctas, w.threads, w.smem, false, ra, a, s) != cudaSuccess)
                 return FK_ERR_CUDA;
             done += c;
         }

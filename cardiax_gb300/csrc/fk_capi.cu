@@ -457,6 +457,14 @@ static void resident_args(ResidentArgs &ra, const ResPlan &plan, void *workspace
     ra.xchg = static_cast<uint64_t *>(workspace);
 }
 
+// The strips in memory start out without a tag; a cluster's tiles exchange none there.
+static cudaError_t launch_plan(const ResPlan &plan, void *workspace, const ResidentArgs &ra, const StepArgs &a,
+                               cudaStream_t s) {
+    const cudaError_t e = plan.cluster ? cudaSuccess : cudaMemsetAsync(workspace, 0, plan.workspace(), s);
+    return e != cudaSuccess ? e
+                            : launch_resident(plan.rows, (int)plan.tiles, plan.threads, plan.smem, plan.cluster, ra, a, s);
+}
+
 // Steps t0 .. t0+n-1 from `in` through the resident kernel, states written to `base` + offset after the
 // steps listed in `outs` ((step, offset) pairs in step order, the last one at step n); `tmp` (one state)
 // holds the state between launches that end at no listed step.
@@ -489,8 +497,7 @@ static int resident_run(const ResPlan &plan, const fk_grid &g, const float *in, 
             in = tmp;
         }
         ra.n = (int)c;
-        if (cudaMemsetAsync(workspace, 0, plan.workspace(), s) != cudaSuccess ||
-            launch_resident(plan.rows, (int)plan.tiles, plan.threads, plan.smem, ra, a, s) != cudaSuccess)
+        if (launch_plan(plan, workspace, ra, a, s) != cudaSuccess)
             return FK_ERR_CUDA;
         done += c;
     }
@@ -1249,8 +1256,7 @@ int fk_recompute_resident(fk_grid g, const float *state, int64_t s, int64_t n, c
     ra.t0 = s;
     ra.n = (int)(n - 1);
     ra.every = ns;
-    if (cudaMemsetAsync(workspace, 0, plan.workspace(), cs) != cudaSuccess ||
-        launch_resident(plan.rows, (int)plan.tiles, plan.threads, plan.smem, ra, a, cs) != cudaSuccess)
+    if (launch_plan(plan, workspace, ra, a, cs) != cudaSuccess)
         return FK_ERR_CUDA;
     return FK_OK;
 }

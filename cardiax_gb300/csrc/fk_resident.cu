@@ -26,7 +26,11 @@
 // overwrites the strip of step s at step s + 2, after it has read its neighbours' strips of step
 // s + 1, which they sent after they had read its strip of step s.
 //
-// Every wait is bounded (1 s); a tile whose wait runs out reports it and leaves, its neighbours'
+// A tissue of few cells per SM on 16 SMs runs as one cluster instead: the strips are stored straight into the
+// neighbours' u tiles (distributed shared memory) and the cluster's barrier takes the place of the tags; no
+// words in memory, no spinning, no cooperative launch.  64^2 1.88 -> 1.61 us per step, 128^2 1.87 -> 1.75.
+//
+// Every wait on memory is bounded (1 s); a tile whose wait runs out reports it and leaves, its neighbours'
 // waits then run out as well.  The launch is cooperative, so all tiles run at the same time, and
 // takes at most kResMaxSteps steps.
 //
@@ -52,6 +56,19 @@ __device__ __forceinline__ void st_tagged(uint64_t *p, float a, float b, uint32_
 __device__ __forceinline__ void ld_tagged(const uint64_t *p, uint64_t &x, uint64_t &y) {
     asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p) : "memory");
 }
+// The other CTAs of the cluster: an address of theirs for one of this CTA's, a store there, and the barrier
+// (arrive releases this CTA's stores, wait acquires the others').
+__device__ __forceinline__ uint32_t cluster_addr(const float *p, int rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, float4 q) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(q.x), "f"(q.y), "f"(q.z), "f"(q.w)
+                 : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // A quad of a strip: two 16-byte accesses.
 __device__ __forceinline__ void send_quad(uint64_t *p, float4 q, uint32_t tag) {
     st_tagged(p, q.x, q.y, tag);
@@ -280,7 +297,8 @@ __device__ __forceinline__ void step_unit(const StepArgs &a, const Consts &tc, c
 // R: rows per thread.  ACT: activation tracking.  MANY: the launch holds several tissues; ra.cta says
 // which tissue (of ra.tissues) and which class of constants (ra.cls) a block belongs to.  Both are read
 // from the launch's parameters by the block index, so the model's constants stay uniform operands.
-template <int R, bool ACT, bool MANY>
+// CL: the tiles are one thread-block cluster, their rank in it their number.
+template <int R, bool ACT, bool MANY, bool CL>
 __global__ void __launch_bounds__(512, 1)
     fk_resident_kernel(const __grid_constant__ ResidentArgs ra, const __grid_constant__ StepArgs a0,
                        const __grid_constant__ PackConsts kc) {
@@ -413,6 +431,10 @@ __global__ void __launch_bounds__(512, 1)
     };
     if (tid < 32) fill_active(0);
     if (tid == 0) s_abort = 0;
+    if (CL) {  // (the neighbours write into the second u buffer, which held D)
+        cluster_arrive();
+        cluster_wait();
+    }
     __syncthreads();
 
     // strips: [0, 16 max_q) the tile's top 4 rows, then its bottom 4 rows, then its left and its
@@ -490,6 +512,36 @@ __global__ void __launch_bounds__(512, 1)
     };
     int out_src = 0, out_dst = 0;
     if (tid < n_ring && tid < n_items) locate_out(tid, out_src, out_dst);
+    // CL: item x's place in this tile's u buffer, and in its neighbour's (a shared::cluster address, buffer 0)
+    auto locate_far = [&](int x, int &src, uint32_t &dst) {
+        int r, cc, t, far_r, far_c;
+        if (x < n_top) {  // the tile above: below its last row
+            r = x / tq;
+            cc = far_c = x - r * tq;
+            t = tile - t_nc;
+            far_r = row0 - (tr - 1) * t_ng / t_nr * R + r;
+        } else if ((x -= n_top) < n_bot) {
+            r = x / tq;
+            cc = far_c = x - r * tq;
+            t = tile + t_nc;
+            far_r = r - 4;
+            r += th - 4;
+        } else if ((x -= n_bot) < n_left) {  // right of its last quad
+            r = far_r = x;
+            cc = 0;
+            t = tile - 1;
+            far_c = q0 - (tc - 1) * t_nq / t_nc;
+        } else {
+            r = far_r = x - n_left;
+            cc = tq - 1;
+            t = tile + 1;
+            far_c = -1;
+        }
+        src = (r + UROW) * SUW + 4 * cc + UCOL;
+        dst = cluster_addr(su + (far_r + UROW) * SUW + 4 * far_c + UCOL, t);
+    };
+    uint32_t far_dst = 0;
+    if (CL && tid < n_items) locate_far(tid, out_src, far_dst);
     uint64_t *const out_strips = ra.xchg + 2 * tile_g * ra.slot;
     const int ucell = (lr + UROW) * SUW + lc + UCOL;
     auto any = [&](bool x) { return __any_sync(0xffffffffu, mine && x) != 0; };
@@ -549,14 +601,27 @@ __global__ void __launch_bounds__(512, 1)
             if (tid < 32 && (s & 31) == 31) fill_active(s + 1);
             __syncthreads();
             // ---- this tile's strips out, and the neighbours' into the next buffer's halo ----------
-            if (tid < n_ring)
+            if (CL) {
+                const uint32_t far_buf = ((s + 1) & 1) * SU * 4;
+                for (int it = tid; it < n_items; it += nthr) {
+                    if (it != tid) locate_far(it, out_src, far_dst);
+                    st_cluster(far_dst + far_buf, ld4(nxt + out_src));
+                }
+                if (n_items > nthr && tid < n_items) locate_far(tid, out_src, far_dst);
+                cluster_arrive();
+            } else if (tid < n_ring) {
                 for (int it = tid; it < n_items; it += n_ring) {
                     if (it != tid) locate_out(it, out_src, out_dst);
                     send_quad(out_strips + par + out_dst, ld4(nxt + out_src), tag);
                 }
+            }
         }
         if (!MANY) write_out(s, nxt);
         if (last) return;
+        if (CL) {
+            cluster_wait();
+            continue;
+        }
         if (tid < n_ring) {
             for (int it = tid; it < n_items; it += n_ring) {
                 if (it != tid) locate(it, in_src, in_dst);
@@ -591,6 +656,11 @@ static double step_cost(int R, int units, int items) {
     static const double each[] = {0, 0, 2.0e-3, 3.2e-3, 3.6e-3, 4.0e-3};
     return base[R] + each[R] * units + 5e-4 * items;
 }
+
+// The same with the tiles in one cluster: the faster one up to some 140^2 cells (us per step in a cluster | in
+// blocks all over the device: 64^2 1.61 | 1.88, 128^2 1.75 | 1.87, 160^2 2.09 | 1.88, 200^2 2.30 | 1.97: 16 SMs
+// have more units each).
+static double cluster_cost(int units, int items) { return 1.66 + 2.0e-3 * units + 7e-4 * items; }
 
 // Every plan of at most `most` tiles with R rows per thread.
 template <class F>
@@ -647,12 +717,18 @@ void resident_plans(int64_t H, int64_t W, int most, int R, std::vector<ResPlan> 
         if (!best[t].ok() || (best[t - 1].ok() && best[t - 1].cost <= best[t].cost)) best[t] = best[t - 1];
 }
 
-ResPlan resident_plan(int64_t H, int64_t W, int n_sm) {
+ResPlan resident_plan(int64_t H, int64_t W, int n_sm, int max_cluster) {
     ResPlan best;
     for (int R = kResMinRows; R <= kResMaxRows; ++R)
         each_plan(H, W, n_sm, R, [&](const ResPlan &p) {
             if (!best.ok() || p.cost < best.cost) best = p;
         });
+    each_plan(H, W, max_cluster, kResClusterRows, [&](ResPlan p) {
+        if (p.tiles & (p.tiles - 1)) return;
+        p.cluster = true;
+        p.cost = cluster_cost(p.max_g * p.max_q, (p.nr > 1 ? 8 * p.max_q : 0) + (p.nc > 1 ? 2 * p.max_g * p.rows : 0));
+        if (p.cost < best.cost) best = p;
+    });
     return best;
 }
 
@@ -671,23 +747,71 @@ int resident_ctas() {
     return n_sm;
 }
 
-ResPlan resident_plan(int64_t H, int64_t W) { return resident_plan(H, W, resident_ctas()); }
+template <int R, bool ACT, bool MANY, bool CL>
+static cudaError_t configure() {
+    // the attributes are per function and per context: set again whenever the context changes
+    static thread_local uint64_t configured_ctx = 0;
+    if (!context_changed(configured_ctx)) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(fk_resident_kernel<R, ACT, MANY, CL>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResMaxSmem);
+    if (CL && e == cudaSuccess)
+        e = cudaFuncSetAttribute(fk_resident_kernel<R, ACT, MANY, CL>, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                 1);
+    if (e != cudaSuccess) configured_ctx = 0;
+    return e;
+}
 
-template <int R, bool ACT, bool MANY>
+// Launch of `ctas` blocks that run at the same time: cooperative, or one cluster.
+struct ResLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    ResLaunch(int ctas, int threads, size_t smem, bool cluster, cudaStream_t stream) {
+        cfg.gridDim = dim3((unsigned)ctas);
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        if (cluster) {
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)ctas;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        } else {
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+        }
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+};
+
+// The largest cluster (16, 8 or none: 0) of full-size blocks that the current device takes.
+static int resident_cluster() {
+    static thread_local int dev_cached = -1, most = 0;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev != dev_cached) {
+        most = 0;
+        if (resident_ctas() > 0 && configure<kResClusterRows, false, false, true>() == cudaSuccess)
+            for (int c = 16; c >= 8 && most == 0; c /= 2) {
+                ResLaunch l(c, 512, kResMaxSmem, true, nullptr);
+                int n = 0;
+                if (cudaOccupancyMaxActiveClusters(&n, fk_resident_kernel<kResClusterRows, false, false, true>,
+                                                   &l.cfg) == cudaSuccess && n >= 1)
+                    most = c;
+                else
+                    cudaGetLastError();
+            }
+        dev_cached = dev;
+    }
+    return most;
+}
+
+ResPlan resident_plan(int64_t H, int64_t W) { return resident_plan(H, W, resident_ctas(), resident_cluster()); }
+
+template <int R, bool ACT, bool MANY, bool CL = false>
 static cudaError_t launch_one(const cudaLaunchConfig_t &cfg, const ResidentArgs &ra, const StepArgs &a,
                               const PackConsts &k) {
-    // the attribute is per function and per context: set again whenever the context changes
-    static thread_local uint64_t configured_ctx = 0;
-    if (context_changed(configured_ctx)) {
-        const cudaError_t e = cudaFuncSetAttribute(fk_resident_kernel<R, ACT, MANY>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)kResMaxSmem);
-        if (e != cudaSuccess) {
-            configured_ctx = 0;
-            return e;
-        }
-    }
-    return cudaLaunchKernelEx(&cfg, fk_resident_kernel<R, ACT, MANY>, ra, a, k);
+    const cudaError_t e = configure<R, ACT, MANY, CL>();
+    return e != cudaSuccess ? e : cudaLaunchKernelEx(&cfg, fk_resident_kernel<R, ACT, MANY, CL>, ra, a, k);
 }
 template <int R>
 static cudaError_t launch_rows(const cudaLaunchConfig_t &cfg, const ResidentArgs &ra, const StepArgs &a,
@@ -696,24 +820,20 @@ static cudaError_t launch_rows(const cudaLaunchConfig_t &cfg, const ResidentArgs
     return a.act_last ? launch_one<R, true, false>(cfg, ra, a, k) : launch_one<R, false, false>(cfg, ra, a, k);
 }
 
-cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, const ResidentArgs &ra,
+cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, bool cluster, const ResidentArgs &ra,
                             const StepArgs &a, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    const ResLaunch l(ctas, threads, smem, cluster, stream);
     const PackConsts k = make_pack_consts(a.m, a.rdx, a.dt);
+    if (cluster) {
+        if (rows != kResClusterRows || ra.tissues) return cudaErrorInvalidValue;
+        return a.act_last ? launch_one<kResClusterRows, true, false, true>(l.cfg, ra, a, k)
+                          : launch_one<kResClusterRows, false, false, true>(l.cfg, ra, a, k);
+    }
     switch (rows) {
-        case 2: return launch_rows<2>(cfg, ra, a, k);
-        case 3: return launch_rows<3>(cfg, ra, a, k);
-        case 4: return launch_rows<4>(cfg, ra, a, k);
-        case 5: return launch_rows<5>(cfg, ra, a, k);
+        case 2: return launch_rows<2>(l.cfg, ra, a, k);
+        case 3: return launch_rows<3>(l.cfg, ra, a, k);
+        case 4: return launch_rows<4>(l.cfg, ra, a, k);
+        case 5: return launch_rows<5>(l.cfg, ra, a, k);
         default: return cudaErrorInvalidValue;
     }
 }

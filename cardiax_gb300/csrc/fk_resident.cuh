@@ -16,6 +16,7 @@ constexpr int kResMaxOut = 32;       // states one launch can write out by list
 constexpr int kResMaxSteps = 8192;   // steps of one launch: a launch ends within some 50 ms
 constexpr int kResMinRows = 2, kResMaxRows = 5;  // rows per thread the kernel is built for
 
+constexpr int kResClusterRows = 2;   // rows per thread where the tiles are one cluster
 constexpr int kResMaxCtas = 160;     // blocks of one launch (at most one per SM)
 constexpr int kResMaxClasses = 16;   // sets of constants one launch of several tissues holds
 constexpr size_t kResMaxSmem = 224 * 1024;
@@ -32,6 +33,7 @@ struct ResPlan {
     int64_t slot = 0;          // 64-bit words of one tile's outgoing strips (one parity)
     int64_t tiles = 0;
     double cost = 0.0;         // estimated us per step
+    bool cluster = false;      // the tiles are one thread-block cluster
     bool ok() const { return rows != 0; }
     size_t workspace() const { return (size_t)(tiles * 2 * slot) * 8; }
 };
@@ -42,8 +44,8 @@ inline size_t resident_smem(int rows, int threads, int su_floats) {
 // best[t], t = 0 .. most: the fastest plan of `rows` rows per thread and at most t tiles (of equal ones
 // that of the fewest tiles); not ok() where there is none.
 void resident_plans(int64_t H, int64_t W, int most, int rows, std::vector<ResPlan> &best);
-// The fastest plan on a device of n_sm SMs, and on the current device (not ok() without one).
-ResPlan resident_plan(int64_t H, int64_t W, int n_sm);
+// The fastest plan on a device of n_sm SMs that takes clusters of up to max_cluster blocks, and on the current device (not ok() without one).
+ResPlan resident_plan(int64_t H, int64_t W, int n_sm, int max_cluster);
 ResPlan resident_plan(int64_t H, int64_t W);
 // The most blocks a launch may use on the current device (0: no cooperative launches, no device).
 int resident_ctas();
@@ -85,7 +87,7 @@ struct ResidentArgs {
 // Launches ra.n steps with `rows` rows per thread; `a` describes the one tissue (several: only its
 // dt and dx constants are read, by the launch-wide stencil coefficients).  The words of the strips
 // must be zero.
-cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, const ResidentArgs &ra,
+cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, bool cluster, const ResidentArgs &ra,
                             const StepArgs &a, cudaStream_t stream);
 
 }  // namespace fk
