@@ -148,7 +148,7 @@ Layout layout(int n, const int64_t *n_items, const ResWaves &res) {
 // The tissues of a batch are independent, so any set of them that fits on chip together can run all
 // steps of a call in one launch before the next set starts: 48 mixed tissues (5.9 M cells), 64 steps:
 // 45.6 us per step in the batched kernel (143 GCUPS: 40 % of its items are edge tiles, each loaded and
-// stored every step), 36.9 in such launches (34.8 over 256 steps; a launch also loads and stores all).
+// stored every step), 35.7 in such launches (33.6 over 256 steps; a launch also loads and stores all).
 constexpr int kResMaxTissues = 4096, kResMaxWaves = 64;
 
 ResClass res_class(const fk_tissue &t) {
@@ -160,109 +160,146 @@ ResClass res_class(const fk_tissue &t) {
     return c;
 }
 
-// The launches with `R` rows per thread, largest tissues first, each into the first launch with room.
-ResWaves plan_waves_rows(const fk_tissue *ts, int n, int ctas, int R) {
+// By shape and rows per thread: the best plan of at most 0, 1, .. ctas tiles (the cost falls with the tiles).
+struct ResPlans {
+    struct Shape {
+        std::vector<ResPlan> best;
+        int least = 0;  // the fewest tiles that hold the tissue (ctas where all blocks do not)
+    };
+    int ctas;
+    std::map<std::pair<int64_t, int64_t>, Shape> made[kResMaxRows + 1];
+    const Shape &of(const fk_grid &g, int R) {
+        Shape &p = made[R][{g.H, g.W}];
+        if (p.best.empty()) {
+            resident_plans(g.H, g.W, ctas, R, p.best);
+            while (p.least < ctas && !p.best[p.least].ok()) ++p.least;
+        }
+        return p;
+    }
+    const ResPlan &least(const fk_grid &g, int R) {
+        const Shape &p = of(g, R);
+        return p.best[p.least];
+    }
+};
+
+// The launch of wave x's tissues with R rows per thread (x.rows stays 0 where they do not fit).
+void plan_wave(const fk_tissue *ts, ResPlans &plans, int R, const std::vector<int> &cls, ResWave &x) {
+    const int n = (int)x.tissue.size();
+    x.plan.resize(n);
+    int left = plans.ctas;
+    for (int i = 0; i < n; ++i) {
+        x.plan[i] = plans.least(ts[x.tissue[i]].g, R);
+        if (!x.plan[i].ok()) return;
+        left -= (int)x.plan[i].tiles;
+    }
+    if (left < 0) return;
+    // blocks left over go to the tissue that takes longest, while that helps
+    while (left > 0) {
+        int worst = 0;
+        for (int i = 1; i < n; ++i)
+            if (x.plan[i].cost > x.plan[worst].cost) worst = i;
+        const std::vector<ResPlan> &p = plans.of(ts[x.tissue[worst]].g, R).best;
+        const int tiles = (int)x.plan[worst].tiles;
+        int t = tiles;
+        while (t < tiles + left && !(p[t].cost < x.plan[worst].cost)) ++t;
+        if (!(p[t].cost < x.plan[worst].cost)) break;
+        left -= t - tiles;
+        x.plan[worst] = p[t];
+    }
+    for (int i = 0; i < n; ++i) {
+        const ResPlan &p = x.plan[i];
+        for (int t = 0; t < p.tiles; ++t) x.args.cta[x.ctas + t] = (uint32_t)i << 8 | (uint32_t)cls[i];
+        x.ctas += (int)p.tiles;
+        x.threads = std::max(x.threads, p.threads);
+        x.args.max_q = std::max(x.args.max_q, p.max_q);
+        x.args.max_g = std::max(x.args.max_g, p.max_g);
+        x.args.su = std::max(x.args.su, p.su_w * p.su_h);
+        x.cost = std::max(x.cost, p.cost);
+    }
+    // (threads and u buffers may come from different tissues: their sum need not fit)
+    x.smem = resident_smem(R, x.threads, x.args.su);
+    if (x.smem > kResMaxSmem) return;
+    x.args.slot = 2 * 16 * (int64_t)x.args.max_q + 2 * 4 * (int64_t)x.args.max_g * R;
+    x.rows = R;
+}
+
+// Sets made with `R` rows per thread, largest tissues first, each into the first set with room; with `each` a
+// set then takes the rows that are fastest for it (the last sets hold few tissues: 48 mixed ones, six sets of 4 rows,
+// the last of two 512^2 tissues then of 2 rows: 37.2 -> 35.7 us per step).
+ResWaves plan_waves_rows(const fk_tissue *ts, int n, ResPlans &plans, int R, bool each) {
     ResWaves out;
-    // by shape: the best plan of at most 0, 1, .. ctas tiles (the cost falls with the tiles)
-    std::map<std::pair<int64_t, int64_t>, std::vector<ResPlan>> made;
-    std::vector<const std::vector<ResPlan> *> plans(n);
     std::vector<ResPlan> plan(n);
     for (int k = 0; k < n; ++k) {
-        const fk_grid &g = ts[k].g;
-        std::vector<ResPlan> &p = made[{g.H, g.W}];
-        if (p.empty()) resident_plans(g.H, g.W, ctas, R, p);
-        if (!p[ctas].ok()) return out;
-        int t = 0;
-        while (!p[t].ok()) ++t;
-        plans[k] = &p;
-        plan[k] = p[t];
+        plan[k] = plans.least(ts[k].g, R);
+        if (!plan[k].ok()) return out;
     }
     std::vector<int> order(n);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return plan[x].tiles > plan[y].tiles; });
-    std::vector<ResWave> w;
-    std::vector<std::vector<int>> cls_of;  // per launch and tissue: its class
+    struct Set {
+        int ctas = 0, n_cls = 0;
+        std::vector<int> tissue, cls;
+        ResClass c[kResMaxClasses];
+    };
+    std::vector<Set> sets;
     for (int k : order) {
         const ResClass c = res_class(ts[k]);
-        size_t q = 0;
-        for (;; ++q) {
-            if (q == w.size()) {
+        for (size_t q = 0;; ++q) {
+            if (q == sets.size()) {
                 if ((int)q == kResMaxWaves) return out;
-                w.emplace_back();
-                cls_of.emplace_back();
+                sets.emplace_back();
             }
-            ResWave &x = w[q];
-            if (x.ctas + plan[k].tiles > ctas) continue;
+            Set &x = sets[q];
+            if (x.ctas + plan[k].tiles > plans.ctas) continue;
             int id = 0;
-            for (; id < x.args.n_out; ++id)  // n_out counts the classes while planning
-                if (std::memcmp(&x.args.cls[id], &c, sizeof c) == 0) break;
+            while (id < x.n_cls && std::memcmp(&x.c[id], &c, sizeof c) != 0) ++id;
             if (id == kResMaxClasses) continue;
-            if (id == x.args.n_out) x.args.cls[x.args.n_out++] = c;
+            if (id == x.n_cls) x.c[x.n_cls++] = c;
             x.ctas += (int)plan[k].tiles;
             x.tissue.push_back(k);
-            cls_of[q].push_back(id);
+            x.cls.push_back(id);
             break;
         }
     }
     int at = 0;
-    for (size_t q = 0; q < w.size(); ++q) {
-        ResWave &x = w[q];
-        // blocks left over go to the tissue that takes longest, while that helps
-        for (int left = ctas - x.ctas; left > 0;) {
-            int worst = x.tissue[0];
-            for (int k : x.tissue)
-                if (plan[k].cost > plan[worst].cost) worst = k;
-            const int tiles = (int)plan[worst].tiles;
-            int t = tiles;
-            while (t < tiles + left && !((*plans[worst])[t].cost < plan[worst].cost)) ++t;
-            const ResPlan &better = (*plans[worst])[t];
-            if (!(better.cost < plan[worst].cost)) break;
-            left -= t - tiles;
-            plan[worst] = better;
+    for (const Set &x : sets) {
+        ResWave best;
+        for (int r = each ? kResMinRows : R; r <= (each ? kResMaxRows : R); ++r) {
+            ResWave w;
+            w.tissue = x.tissue;
+            plan_wave(ts, plans, r, x.cls, w);
+            if (w.rows && (!best.rows || w.cost < best.cost)) best = std::move(w);
         }
-        x.rows = R;
-        x.first = at;
-        x.args.n_out = 0;
-        x.ctas = 0;
-        for (size_t i = 0; i < x.tissue.size(); ++i) {
-            const ResPlan &p = plan[x.tissue[i]];
-            x.plan.push_back(p);
-            for (int t = 0; t < p.tiles; ++t)
-                x.args.cta[x.ctas + t] = (uint32_t)i << 8 | (uint32_t)cls_of[q][i];
-            x.ctas += (int)p.tiles;
-            x.threads = std::max(x.threads, p.threads);
-            x.args.max_q = std::max(x.args.max_q, p.max_q);
-            x.args.max_g = std::max(x.args.max_g, p.max_g);
-            x.cost = std::max(x.cost, p.cost);
-        }
-        for (int k : x.tissue) x.args.su = std::max(x.args.su, plan[k].su_w * plan[k].su_h);
-        // (threads and u buffers may come from different tissues: their sum need not fit)
-        x.smem = resident_smem(R, x.threads, x.args.su);
-        if (x.smem > kResMaxSmem) return ResWaves();
-        x.args.slot = 2 * 16 * (int64_t)x.args.max_q + 2 * 4 * (int64_t)x.args.max_g * R;
-        out.xchg_bytes = std::max(out.xchg_bytes, (size_t)(x.ctas * 2 * x.args.slot) * 8);
-        out.cost += x.cost;
+        if (!best.rows) return ResWaves();
+        std::copy(x.c, x.c + x.n_cls, best.args.cls);
+        best.first = at;
         at += (int)x.tissue.size();
+        out.xchg_bytes = std::max(out.xchg_bytes, (size_t)(best.ctas * 2 * best.args.slot) * 8);
+        out.cost += best.cost;
+        out.w.push_back(std::move(best));
     }
-    out.w = std::move(w);
     return out;
 }
 
 ResWaves plan_waves(const fk_tissue *ts, int n) {
     ResWaves best;
-    const int ctas = resident_ctas();
-    if (ctas < 2 || n > kResMaxTissues) return best;
+    ResPlans plans{resident_ctas(), {}};
+    if (plans.ctas < 2 || n > kResMaxTissues) return best;
     int64_t cells = 0;
     for (int k = 0; k < n; ++k) {
         if (check_grid(ts[k].g) || ts[k].act.last || ts[k].n_stimuli > kMaxStim) return best;
         cells += ts[k].g.H * ts[k].g.W;
     }
-    if (cells > (int64_t)kResMaxWaves * ctas * 512 * 4 * kResMaxRows) return best;
+    if (cells > (int64_t)kResMaxWaves * plans.ctas * 512 * 4 * kResMaxRows) return best;
+    int rows = 0;
     for (int R = kResMinRows; R <= kResMaxRows; ++R) {
-        ResWaves w = plan_waves_rows(ts, n, ctas, R);
-        if (w.ok() && (!best.ok() || w.cost < best.cost)) best = std::move(w);
+        ResWaves w = plan_waves_rows(ts, n, plans, R, false);
+        if (w.ok() && (!best.ok() || w.cost < best.cost)) {
+            best = std::move(w);
+            rows = R;
+        }
     }
-    return best;
+    return best.w.size() > 1 ? plan_waves_rows(ts, n, plans, rows, true) : best;
 }
 
 // us of n steps: the resident launches (a launch's fixed cost is 15 to 30 us), and one launch per
