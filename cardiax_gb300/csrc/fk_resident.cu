@@ -8,8 +8,8 @@
 // updates its cells; then the cells within 4 of a tile side go to the neighbour through global
 // memory.  Only u is exchanged, only with the 4 direct neighbours: no stencil is diagonal.
 //
-// What bounds it (us per step, GB300; one launch per step before): 256^2 2.04 (4.4), 512^2 2.38
-// (4.5), 1024^2 5.31 (8.2), 1200^2 6.02 (9.7).  One launch per step pays launch, load and store
+// What bounds it (us per step, GB300; one launch per step before): 256^2 1.88 (4.4), 512^2 2.36
+// (4.5), 1024^2 5.08 (8.2), 1200^2 5.98 (9.7).  One launch per step pays launch, load and store
 // latencies in a row whatever it computes.  Here a small grid's step is one dependent chain: about
 // 1000 cycles for a unit of 8 cells (1600 at the grid's edge), 1700 from a strip's store to its
 // neighbour's load of it through L2, and two barriers.  A large grid's step is bound by issue
@@ -28,7 +28,7 @@
 //
 // A tissue of few cells per SM on 16 SMs runs as one cluster instead: the strips are stored straight into the
 // neighbours' u tiles (distributed shared memory) and the cluster's barrier takes the place of the tags; no
-// words in memory, no spinning, no cooperative launch.  64^2 1.88 -> 1.61 us per step, 128^2 1.87 -> 1.75.
+// words in memory, no spinning, no cooperative launch.  64^2 1.88 -> 1.54 us per step, 128^2 1.87 -> 1.63.
 //
 // Every wait on memory is bounded (1 s); a tile whose wait runs out reports it and leaves, its neighbours'
 // waits then run out as well.  The launch is cooperative, so all tiles run at the same time, and
@@ -662,6 +662,16 @@ static double step_cost(int R, int units, int items) {
 // have more units each).
 static double cluster_cost(int units, int items) { return 1.66 + 2.0e-3 * units + 7e-4 * items; }
 
+// Quads of a row of the u tile.  Of 8 lanes that load 16 bytes each, those beyond the end of a group of R rows
+// go on in the next one: with this many quads in a row in the 16-byte banks after the others' (where R and the
+// count allow it).  us per step without | with: 64^2 1.61 | 1.54, 128^2 1.75 | 1.63, 256^2 1.92 | 1.88, 1024^2
+// 5.30 | 5.08, 1200^2 6.03 | 5.98 (27 % of the wavefronts there were conflicts).
+static int tile_quads(int R, int max_q) {
+    for (int x = max_q + 2; x < max_q + 10; ++x)
+        if ((R * x - (max_q - 2)) % 8 == 0) return x;
+    return max_q + 2;
+}
+
 // Every plan of at most `most` tiles with R rows per thread.
 template <class F>
 static void each_plan(int64_t H, int64_t W, int most, int R, F take) {
@@ -695,8 +705,9 @@ static void each_plan(int64_t H, int64_t W, int most, int R, F take) {
             int want = units > items ? units : items;
             want = (want + 31) / 32 * 32;
             p.threads = want < 512 ? want : 512;
-            p.su_w = 4 * (max_q + 2);
             p.su_h = max_g * R + 8 + R - 1;
+            p.su_w = 4 * tile_quads(R, max_q);
+            if (resident_smem(R, p.threads, p.su_w * p.su_h) > kResMaxSmem) p.su_w = 4 * (max_q + 2);
             p.smem = resident_smem(R, p.threads, p.su_w * p.su_h);
             if (p.smem > kResMaxSmem) continue;
             p.slot = 2 * 16 * (int64_t)max_q + 2 * 4 * (int64_t)max_g * R;
