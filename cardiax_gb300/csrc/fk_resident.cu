@@ -13,7 +13,7 @@
 // latencies in a row whatever it computes.  Here a small grid's step is one dependent chain: about
 // 1000 cycles for a unit of 8 cells (1600 at the grid's edge), 1700 from a strip's store to its
 // neighbour's load of it through L2, and two barriers.  A large grid's step is bound by issue
-// slots and instruction fetch (107 instructions per cell); the loop's code is kept small for that
+// slots and instruction fetch (some 89 instructions per cell); the loop's code is kept small for that
 // reason (see Unit).
 //
 // Rows per thread: more rows share u rows and u_x, and hold more cells (512 threads of 4 R cells
@@ -658,7 +658,7 @@ static double step_cost(int R, int units, int items) {
 }
 
 // The same with the tiles in one cluster: the faster one up to some 140^2 cells (us per step in a cluster | in
-// blocks all over the device: 64^2 1.61 | 1.88, 128^2 1.75 | 1.87, 160^2 2.09 | 1.88, 200^2 2.30 | 1.97: 16 SMs
+// blocks all over the device: 64^2 1.54 | 1.93, 128^2 1.61 | 2.02, 160^2 2.09 | 1.93, 200^2 2.30 | 2.03: 16 SMs
 // have more units each).
 static double cluster_cost(int units, int items) { return 1.66 + 2.0e-3 * units + 7e-4 * items; }
 
