@@ -25,6 +25,7 @@
 #include "fk_adjoint.cuh"
 #include "fk_capi_internal.h"
 #include "fk_math.cuh"
+#include "fk_pack.cuh"
 #include "fk_ptx.cuh"
 
 namespace fk {
@@ -532,209 +533,192 @@ __global__ void __launch_bounds__(ANT, 4) fk_adjoint_kernel(const __grid_constan
 }
 
 // ---- lines of at least kLineMin cells: two or four threads per unit of two rows of a quad ----------
-// What bounds it: the tile kernel above stages six derivative planes, reads ten-cell products for
-// each cell of the 6-cell edge band, tests every stimulus's protocol in every cell and reduces 13
-// parameter sums over a warp for every two cells (us per step: 39.5 for 16 experiments of 256^2,
-// 10.9 for one 151 x 203 grid, 10.5 for 16 of 64^2).  Here everything comes from one staged tile of
-// u, D and lambda_u and stays in registers: 24.2, 5.0 and 6.0 us.  At 16 x 256^2 a step executes some
-// 390 instructions per cell, 210 of them the stencils and currents; one small grid waits for its
-// launch (4 us without any work) and then for the longest chain of a unit.  The operations are fewer because they are regrouped:
-//   * both transposed products of an axis share their second operator,
-//       A^T (D mu) + B^T ((B D) mu) = (E^T G^T / dx) (G^T C^T (D mu) / dx + C^T (B D) mu),
-//   * G^T on central rows is -G; the one-sided rows 0 and N-1 (and the pad rows -1 and N in the
-//     second operator) are taken out of the central sum and added as rank-one terms to the four
-//     cells they reach, only by the warps that hold such cells,
-//   * 1/dx^2, dt and the constant factors of the parameter sums are applied once, to the sums, and a
-//     parameter sum is reduced over a warp once per 8 cells.
-constexpr int kLineMin = 20;  // shorter lines (fewer than three quads or nine rows in a last tile)
-                              // take the tile kernel above
+// What bounds it: the tile kernel above stages six derivative planes, tests every stimulus's protocol in every
+// cell and reduces 13 parameter sums over a warp for every two cells (us per step: 39.5 for 16 experiments of
+// 256^2, 10.9 for one 151 x 203 grid, 10.5 for 16 of 64^2).  Here everything comes from one staged tile of u, D
+// and lambda_u and stays in registers: 24.7, 5.0 and 5.2 us.  Many experiments are bound by the instructions of the
+// stencils and currents; one small grid waits for its launch (4 us without any work) and then for the longest
+// chain of a unit.
+//   * lambda and dL/dD are the tile kernel's operations in the same order: the same bits.  (Regrouped, the two
+//     products of an axis sharing their second operator and the one-sided rows as rank-one terms, the step took
+//     24.1, 5.1 and 6.1 us; but rounding at the edges acts the same way in every step, and dL/dw0 of small grids
+//     came out up to 3.8 times further from the 64-bit gradient.)  Along columns four lines are two packed
+//     operations.
+//   * cells within ADJ_BAND of a line's end: the ten products at that end once per line, then one thread per
+//     cell and line sums them with the corner tables; the units take all other cells by the central operators
+//     alone, so that no warp goes two ways.
+//   * the constant factors of the parameter sums are applied once, in double, to sums that are reduced over a
+//     warp once per 8 cells.
+constexpr int kLineMin = kEdgeMinLine;  // shorter lines (fewer than three quads or nine rows in a last tile)
+                                        // take the tile kernel above
 constexpr int LR = 2;         // rows per thread
 constexpr int LG = 8;         // most row groups of a tile
+constexpr int LROWS = LG * LR;
 constexpr int LNT = 256;      // threads of a block: two or four share a unit (see fk_adjoint_line_kernel)
+constexpr int LEND = 10;      // cells at a line's end that the band's sums take
 template <int SHARE>
 struct LineTile {
     static constexpr int LU = LNT / SHARE, LQ = LU / LG;  // units, most quads of a tile
     static constexpr int LSW = 4 * LQ + 12;  // staged row: 4 cells on either side, and 4 more so that 8 lanes
                                              // (2 quads of 4 groups) read from 8 different 16-byte banks
-    static constexpr int LSH = LG * LR + 8 + 1;  // 4 rows above and below; the first group of the last
-                                                 // tile row may reach one row further up
-    static constexpr int SMEM = (3 * LSH * LSW + 6 * LR * LU * 4) * 4;
+    static constexpr int LSH = LROWS + 8 + 1;  // 4 rows above and below; the first group of the last
+                                               // tile row may reach one row further up
+    static constexpr int LC = 4 * LQ;          // columns
+    static constexpr int SMEM = (3 * LSH * LSW + 8 * LR * LU * 4 +
+                                 4 * (LEND * LC + 2 * LEND * LROWS + 2 * ADJ_BAND * LROWS + LEND * ADJ_BAND)) * 4;
 };
 
-__constant__ float kHeadC[4] = {C_HEAD0, C_THREE, -C_3_2, C_1_3};
-__constant__ float kTailC[4] = {C_TAIL0, C_3_2, -C_THREE, C_TAIL3};
-
-struct V4 {
-    float x, y, z, w;
+// The corner tables by what a cell `pp` from the line's end takes of cell r: A[r][pp], B[r][pp], A[pp][r].
+struct alignas(16) EndTap {
+    float a, b, d, pad;
 };
-__device__ __forceinline__ V4 ld_v4(const float *p) {
-    const float4 v = *reinterpret_cast<const float4 *>(p);
-    return V4{v.x, v.y, v.z, v.w};
+struct EndTaps {
+    EndTap t[LEND][ADJ_BAND];
+};
+constexpr EndTaps make_end_taps() {
+    EndTaps x{};
+    for (int r = 0; r < LEND; ++r)
+        for (int p = 0; p < ADJ_BAND; ++p)
+            x.t[r][p] = EndTap{kEdgeHost.A[r][p], kEdgeHost.B[r][p], kEdgeHost.A[p][r], 0.0f};
+    return x;
 }
-__device__ __forceinline__ V4 vmul(V4 a, V4 b) { return V4{a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w}; }
-__device__ __forceinline__ V4 vscale(float c, V4 a) { return V4{c * a.x, c * a.y, c * a.z, c * a.w}; }
-__device__ __forceinline__ V4 vfma(V4 a, V4 b, V4 c) {
-    return V4{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y), fmaf(a.z, b.z, c.z), fmaf(a.w, b.w, c.w)};
-}
-__device__ __forceinline__ V4 vaxpy(float c, V4 a, V4 b) {  // c a + b
-    return V4{fmaf(c, a.x, b.x), fmaf(c, a.y, b.y), fmaf(c, a.z, b.z), fmaf(c, a.w, b.w)};
-}
-__device__ __forceinline__ float vmul(float a, float b) { return a * b; }
-__device__ __forceinline__ float vscale(float c, float a) { return c * a; }
-__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ float vaxpy(float c, float a, float b) { return fmaf(c, a, b); }
+__device__ const EndTaps kEndTaps = make_end_taps();
 
-template <class T>
-__device__ __forceinline__ T v_central(T m2, T m1, T p1, T p2) {
-    return vaxpy(-C_1_12, p2, vaxpy(C_2_3, p1, vaxpy(-C_2_3, m1, vscale(C_1_12, m2))));
-}
-template <class T>
-__device__ __forceinline__ T v_head(T a, T b, T c, T d) {
-    return vaxpy(C_1_3, d, vaxpy(-C_3_2, c, vaxpy(C_THREE, b, vscale(C_HEAD0, a))));
-}
-template <class T>
-__device__ __forceinline__ T v_tail(T a, T b, T c, T d) {
-    return vaxpy(C_TAIL3, d, vaxpy(-C_THREE, c, vaxpy(C_3_2, b, vscale(C_TAIL0, a))));
+// D mu, (B D) mu, u and mu u' at the cell at place b of the staged fields, s floats from one cell of the line to
+// the next; at: 0 at the line's first cell, 1 at its last one, 2 between.
+__device__ __forceinline__ float4 end_products(const float *su, const float *sd, const float *sl, int b, int s, int at,
+                                               float dt, float rdx) {
+    auto d1 = [&](const float *f) {
+        if (at == 0) return g_head(f[b], f[b + s], f[b + 2 * s], f[b + 3 * s]) * rdx;
+        if (at == 1) return g_tail(f[b - 3 * s], f[b - 2 * s], f[b - s], f[b]) * rdx;
+        return g_central(f[b - 2 * s], f[b - s], f[b + s], f[b + 2 * s]) * rdx;
+    };
+    const float mu = dt * sl[b], dq = d1(sd), uq = d1(su);
+    return make_float4(sd[b] * mu, dq * mu, su[b], mu * uq);
 }
 
-// One axis at R neighbouring cells x0 .. x0+R-1 of a line of N cells, in two halves so that few
-// values are live at a time; derivatives unscaled (results times 1/dx^2).  EDGE: a cell of the warp
-// lies within reach of one of the line's ends.  cell(f, d) is cell x0 + d of field f (0: u, 1: D, both
-// edge-padded; 2: lambda_u, zero outside the grid); of(f, t) the same at d = t - 4 for the t known at
-// compile time.  v_central with its arguments reversed is -G.
+// The four terms of a cell `pp` from its line's end, from the products of the ten cells there (`stride` apart), as
+// axis_edge sums them.
+__device__ __forceinline__ float4 end_sums(const float4 *L, int stride, const float4 *taps, int pp, float sgn,
+                                           float rdx) {
+    float AT = 0.f, BT = 0.f, d2 = 0.f, g = 0.f;
+#pragma unroll
+    for (int r = 0; r < LEND; ++r) {
+        const float4 l = L[r * stride], c = taps[r * ADJ_BAND + pp];
+        AT = fmaf(c.x, l.x, AT);
+        BT = fmaf(c.y, l.y, BT);
+        d2 = fmaf(c.z, l.z, d2);
+        g = fmaf(c.y, l.w, g);
+    }
+    return make_float4(AT * (rdx * rdx), sgn * BT * rdx, d2 * (rdx * rdx), sgn * g * rdx);
+}
+
+// Constants of the packed operations, each twice (in the constant bank).  (No packed product goes into a packed
+// addition: see fk_pack.cuh.)
+struct LineConsts {
+    float2 c_1_12, c_m2_3, c_2_3, c_m1_12, rdx, neg_rdx, dt;
+};
+__device__ __forceinline__ float2 pair_central(const LineConsts &k, float2 m2, float2 m1, float2 p1, float2 p2) {
+    return p_fma(k.c_m1_12, p2, p_fma(k.c_2_3, p1, p_fma(k.c_m2_3, m1, p_mul(k.c_1_12, m2))));
+}
+__device__ __forceinline__ Quad quad_central(const LineConsts &k, const Quad &m2, const Quad &m1, const Quad &p1,
+                                             const Quad &p2) {
+    return Quad{pair_central(k, m2.lo, m1.lo, p1.lo, p2.lo), pair_central(k, m2.hi, m1.hi, p1.hi, p2.hi)};
+}
+__device__ __forceinline__ Quad q_mul(const Quad &a, const Quad &b) {
+    return Quad{p_mul(a.lo, b.lo), p_mul(a.hi, b.hi)};
+}
+
+// The x direction (along the four columns of a quad) at R cells that are at least ADJ_BAND from the columns' ends
+// (others get values nobody reads), in two halves so that few values are live at a time.  of(f, t) is the cell
+// t - 4 from the first one of field f (0: u, 1: D, 2: lambda_u).
 //
-// gd: lambda u'' + B^T (lambda u').
-template <int R, bool EDGE, class T, class Of, class At>
-__device__ __forceinline__ void axis_gd(int x0, int N, Of of, At cell, T (&gd)[R]) {
-    T U[R + 8], ux[R + 4];
+// d2: u''; g: B^T (mu u').
+template <int R, class Of>
+__device__ __forceinline__ void cols_gd(const LineConsts &kc, Of of, Quad (&d2)[R], Quad (&g)[R]) {
+    Quad U[R + 8], ux[R + 4], m[R + 4];
 #pragma unroll
     for (int t = 0; t < 4; ++t) U[t] = of(0, t);
 #pragma unroll
     for (int t = 0; t < R + 4; ++t) {
         U[t + 4] = of(0, t + 4);
-        ux[t] = v_central(U[t], U[t + 1], U[t + 3], U[t + 4]);
-        if (EDGE) {
-            const int x = x0 - 2 + t;
-            if (t <= 2 && x <= 0) ux[t] = v_head(cell(0, t - 2), cell(0, t - 1), cell(0, t), cell(0, t + 1));
-            if (t >= 1 && x >= N - 1) ux[t] = v_tail(cell(0, t - 5), cell(0, t - 4), cell(0, t - 3), cell(0, t - 2));
-        }
+        ux[t] = q_scale(quad_central(kc, U[t], U[t + 1], U[t + 3], U[t + 4]), kc.rdx);
+        m[t] = q_mul(q_scale(of(2, t + 2), kc.dt), ux[t]);
     }
 #pragma unroll
     for (int k = 0; k < R; ++k) {
-        T d = v_central(ux[k], ux[k + 1], ux[k + 3], ux[k + 4]);
-        if (EDGE) {
-            const int x = x0 + k;
-            if (k == 0 && x == 0) d = v_head(ux[2], ux[3], ux[4], ux[5]);
-            if (x == N - 1) {
-                T far = ux[k >= 1 ? k - 1 : 0];
-                if (k == 0) far = v_central(cell(0, -5), cell(0, -4), cell(0, -2), cell(0, -1));
-                d = v_tail(far, ux[k], ux[k + 1], ux[k + 2]);
-            }
-        }
-        gd[k] = vmul(of(2, k + 4), d);
+        d2[k] = q_scale(quad_central(kc, ux[k], ux[k + 1], ux[k + 3], ux[k + 4]), kc.rdx);
+        g[k] = q_scale(quad_central(kc, m[k], m[k + 1], m[k + 3], m[k + 4]), kc.neg_rdx);
     }
-    // lambda u', with the one-sided rows 0 and N-1 taken out of the central sums
-    T (&m)[R + 4] = ux;
-#pragma unroll
-    for (int t = 0; t < R + 4; ++t) m[t] = vmul(of(2, t + 2), ux[t]);
-    if (EDGE) {
-        const T zero = vscale(0.0f, T{}), m1 = m[3];
-        const int dn = N - 1 - x0;
-        T m0 = zero, mn = zero;
-        if (x0 <= 4) m0 = vmul(cell(2, -x0), v_head(cell(0, -x0), cell(0, 1 - x0), cell(0, 2 - x0), cell(0, 3 - x0)));
-        if (dn <= R + 4) mn = vmul(cell(2, dn), v_tail(cell(0, dn - 3), cell(0, dn - 2), cell(0, dn - 1), cell(0, dn)));
-#pragma unroll
-        for (int t = 0; t < R + 4; ++t) {
-            if (t < 3 && x0 - 2 + t <= 0) m[t] = zero;
-            if (t >= 2 && x0 - 2 + t >= N - 1) m[t] = zero;
-        }
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const int x = x0 + k;
-            gd[k] = vaxpy((unsigned)x < 4u ? kHeadC[x & 3] : 0.0f, m0, gd[k]);
-            gd[k] = vaxpy(x >= N - 4 && x < N ? kTailC[(x - N) & 3] : 0.0f, mn, gd[k]);
-            // the pad rows fold onto the first and the last cell
-            if (k == 0 && x == 0) gd[k] = vaxpy(C_1_12, m1, gd[k]);
-            if (x == N - 1) gd[k] = vaxpy(-C_1_12, m[k + 1], gd[k]);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < R; ++k) gd[k] = vaxpy(1.0f, v_central(m[k + 4], m[k + 3], m[k + 1], m[k]), gd[k]);
 }
 
-// at: A^T (D lambda) + B^T ((B D) lambda).
-template <int R, bool EDGE, class T, class Of, class At>
-__device__ __forceinline__ void axis_at(int x0, int N, Of of, At cell, T (&at)[R]) {
-    const T zero = vscale(0.0f, T{});
-    // D lambda at the one-sided rows (q0, qn), and what these rows and the pad rows carry into the
-    // second operator (b0, bm and bn, bp)
-    T q0 = zero, b0 = zero, bm = zero, qn = zero, bn = zero, bp = zero;
-    if (EDGE) {
-        if (x0 <= 4) {
-            const int d = -x0;
-            auto Q = [&](int k) { return vmul(cell(1, d + k), cell(2, d + k)); };
-            q0 = Q(0);
-            const T q1 = Q(1);
-            bm = vscale(C_1_12, q1);
-            const T g = v_head(cell(1, d), cell(1, d + 1), cell(1, d + 2), cell(1, d + 3));
-            b0 = vfma(g, cell(2, d), vaxpy(C_HEAD0, q0, vaxpy(-C_2_3, q1, vscale(C_1_12, Q(2)))));
-        }
-        if (N - 1 - x0 <= R + 4) {
-            const int d = N - 1 - x0;
-            auto Q = [&](int k) { return vmul(cell(1, d - k), cell(2, d - k)); };
-            qn = Q(0);
-            const T q1 = Q(1);
-            bp = vscale(-C_1_12, q1);
-            const T g = v_tail(cell(1, d - 3), cell(1, d - 2), cell(1, d - 1), cell(1, d));
-            bn = vfma(g, cell(2, d), vaxpy(C_TAIL3, qn, vaxpy(C_2_3, q1, vscale(-C_1_12, Q(2)))));
-        }
-    }
-    T D[R + 8], q[R + 8], s[R + 4];
+// at: A^T (D mu); bt: B^T ((B D) mu).
+template <int R, class Of>
+__device__ __forceinline__ void cols_at(const LineConsts &kc, Of of, Quad (&at)[R], Quad (&bt)[R]) {
+    Quad D[R + 8], M[R + 8], q[R + 8], qx[R + 4], bx[R + 4];
     auto take = [&](int t) {
         D[t] = of(1, t);
-        q[t] = vmul(D[t], of(2, t));
-        if (EDGE) {
-            const int x = x0 - 4 + t;
-            if ((t <= 4 && x == 0) || (t >= 4 && x == N - 1)) q[t] = zero;
-        }
+        M[t] = q_scale(of(2, t), kc.dt);
+        q[t] = q_mul(D[t], M[t]);
     };
 #pragma unroll
     for (int t = 0; t < 4; ++t) take(t);
 #pragma unroll
     for (int t = 0; t < R + 4; ++t) {
         take(t + 4);
-        T g = v_central(D[t], D[t + 1], D[t + 3], D[t + 4]);
-        T y = v_central(q[t + 4], q[t + 3], q[t + 1], q[t]);
-        if (EDGE) {
-            const int x = x0 - 2 + t;
-            if (t <= 2 && x == 0) g = v_head(cell(1, t - 2), cell(1, t - 1), cell(1, t), cell(1, t + 1));
-            if (t >= 1 && x == N - 1) g = v_tail(cell(1, t - 5), cell(1, t - 4), cell(1, t - 3), cell(1, t - 2));
-            y = vaxpy((unsigned)x < 4u ? kHeadC[x & 3] : 0.0f, q0, y);
-            y = vaxpy((unsigned)(x - N + 4) < 4u ? kTailC[(x - N) & 3] : 0.0f, qn, y);
-        }
-        s[t] = vfma(g, of(2, t + 2), y);
+        qx[t] = q_scale(quad_central(kc, q[t], q[t + 1], q[t + 3], q[t + 4]), kc.rdx);
+        bx[t] = q_mul(q_scale(quad_central(kc, D[t], D[t + 1], D[t + 3], D[t + 4]), kc.rdx), M[t + 2]);
     }
-    const T s1 = s[3];
-    if (EDGE)  // rows -1, 0 and N-1, N leave the central sums of the second operator
-#pragma unroll
-        for (int t = 0; t < R + 4; ++t) {
-            if (t < 3 && x0 - 2 + t <= 0) s[t] = zero;
-            if (t >= 2 && x0 - 2 + t >= N - 1) s[t] = zero;
-        }
 #pragma unroll
     for (int k = 0; k < R; ++k) {
-        T a = v_central(s[k + 4], s[k + 3], s[k + 1], s[k]);
-        if (EDGE) {
-            const int x = x0 + k;
-            a = vaxpy((unsigned)x < 4u ? kHeadC[x & 3] : 0.0f, b0, a);
-            a = vaxpy((unsigned)x < 3u ? kHeadC[(x + 1) & 3] : 0.0f, bm, a);
-            a = vaxpy(x >= N - 4 && x < N ? kTailC[(x - N) & 3] : 0.0f, bn, a);
-            a = vaxpy(x >= N - 3 && x < N ? kTailC[(x - N - 1) & 3] : 0.0f, bp, a);
-            if (k == 0 && x == 0) a = vaxpy(C_HEAD0, bm, vaxpy(C_1_12, s1, a));  // the pad rows fold
-            if (x == N - 1) a = vaxpy(C_TAIL3, bp, vaxpy(-C_1_12, s[k + 1], a));
-        }
-        at[k] = a;
+        at[k] = q_scale(quad_central(kc, qx[k], qx[k + 1], qx[k + 3], qx[k + 4]), kc.rdx);
+        bt[k] = q_scale(quad_central(kc, bx[k], bx[k + 1], bx[k + 3], bx[k + 4]), kc.neg_rdx);
     }
+}
+
+// The same of the y direction, at the four cells 4 .. 7 of twelve along a row.  Results of a row lie in aligned
+// pairs of registers: the outer taps as packed operations, the inner ones as scalar ones (see pg_central_row).
+template <int N>
+__device__ __forceinline__ void row_central(const LineConsts &k, const float (&a)[N + 4], float2 c, float (&d)[N]) {
+#pragma unroll
+    for (int t = 0; t < N; t += 2) {
+        float2 s = p_mul(k.c_1_12, mk2(a[t], a[t + 1]));
+        s.x = fmaf(-C_2_3, a[t + 1], s.x);
+        s.y = fmaf(-C_2_3, a[t + 2], s.y);
+        s.x = fmaf(C_2_3, a[t + 3], s.x);
+        s.y = fmaf(C_2_3, a[t + 4], s.y);
+        s = p_mul(p_fma(k.c_m1_12, mk2(a[t + 4], a[t + 5]), s), c);
+        d[t] = s.x;
+        d[t + 1] = s.y;
+    }
+}
+template <int N, int M>
+__device__ __forceinline__ void row_mul(const float (&a)[M], const float (&b)[N], float (&d)[N]) {
+    constexpr int off = (M - N) / 2;
+#pragma unroll
+    for (int t = 0; t < N; t += 2) {
+        const float2 s = p_mul(mk2(a[t + off], a[t + off + 1]), mk2(b[t], b[t + 1]));
+        d[t] = s.x;
+        d[t + 1] = s.y;
+    }
+}
+__device__ __forceinline__ void row_gd(const LineConsts &kc, const float (&U)[12], const float (&mu)[12],
+                                       float (&d2)[4], float (&g)[4]) {
+    float uy[8], m[8];
+    row_central<8>(kc, U, kc.rdx, uy);
+    row_mul<8, 12>(mu, uy, m);
+    row_central<4>(kc, uy, kc.rdx, d2);
+    row_central<4>(kc, m, kc.neg_rdx, g);
+}
+__device__ __forceinline__ void row_at(const LineConsts &kc, const float (&D)[12], const float (&mu)[12],
+                                       float (&at)[4], float (&bt)[4]) {
+    float q[12], qy[8], by[8];
+    row_mul<12, 12>(D, mu, q);
+    row_central<8>(kc, q, kc.rdx, qy);
+    row_central<8>(kc, D, kc.rdx, by);
+    row_mul<8, 12>(mu, by, by);
+    row_central<4>(kc, qy, kc.rdx, at);
+    row_central<4>(kc, by, kc.neg_rdx, bt);
 }
 
 // Sums 16 values over a warp: lane i < 16 returns the sum of v[i] (lanes 16..31 the same).  Each
@@ -768,6 +752,7 @@ struct LineRun {
     int g_each, g_small, q_each, q_small;  // groups (quads) of a tile, and tiles that have one less
     int inv[2], inv_q[2];                  // 2^16 / groups of a tile (/ its quads + 2), rounded up: for the
                                            // tiles that have one less, and for the others
+    LineConsts kc;
 };
 
 // The arguments stay in the constant bank, for many experiments those of the first one and the distance to
@@ -787,12 +772,17 @@ __global__ void __launch_bounds__(LNT, 2)
     fk_adjoint_line_kernel(const __grid_constant__ AdjointArgs a, const __grid_constant__ LineRun b) {
     using T_ = LineTile<SHARE>;
     constexpr int LU = T_::LU, LSW = T_::LSW, LSH = T_::LSH;
-    // u, D, lambda_u with 4 cells around; a unit's own v, w, lambda_v, lambda_w, the first then its lambda_u
-    // through the currents; the x direction's part of lambda_u and of dL/dD
+    constexpr int LC = T_::LC;
+    // u, D and lambda_u with 4 cells around; a unit's own v, w, lambda_v, lambda_w, the first then its lambda_u
+    // through the currents; the x direction's A^T, B^T, u'', B^T (mu u'); the products at the
+    // ends of the columns ([r][column]) and of the rows ([end][r][row]), the four terms of the rows' bands
+    // ([end][pp][row]) and the corner tables
     extern __shared__ __align__(16) float line_smem[];
     float *const su = line_smem, *const sd = su + LSH * LSW, *const sl = sd + LSH * LSW;
     float4(*const sp)[LR][LU] = reinterpret_cast<float4(*)[LR][LU]>(sl + LSH * LSW);
     float4(*const sr)[LR][LU] = sp + 4;
+    float4 *const ex = reinterpret_cast<float4 *>(sr + 4);
+    float4 *const ey = ex + LEND * LC, *const yr = ey + 2 * LEND * LROWS, *const taps = yr + 2 * ADJ_BAND * LROWS;
     constexpr int PT_WARPS = SHARE == 4 ? 2 * LU / 32 : LU / 32;
     __shared__ float red[PT_WARPS][16];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -857,6 +847,10 @@ __global__ void __launch_bounds__(LNT, 2)
         }
     };
     if (b.early) load(true, false);
+    const bool left = bx == 0, right = bx == (int)gridDim.x - 1, top = by == 0, bottom = by == (int)gridDim.y - 1;
+    if (left || right || top || bottom)
+        for (int x = tid; x < LEND * ADJ_BAND; x += LNT)
+            taps[x] = __ldg(reinterpret_cast<const float4 *>(&kEndTaps) + x);
     grid_dependency_wait();
     grid_launch_dependents();
     load(!b.early, true);
@@ -872,17 +866,17 @@ __global__ void __launch_bounds__(LNT, 2)
     asm volatile("cp.async.wait_all;" ::: "memory");
     // A thread's own loads have arrived: at the grid's left and right sides the nearest cell takes the place
     // of those of u and D outside, zero that of lambda.
-    if (bx == 0 || bx == (int)gridDim.x - 1) {
+    if (left || right) {
         const int n = W - 1 - (j0 + 4 * (tq - 1));  // the last cell's place in the last quad
         each_quad([&](int r, int c) {
-            const bool left = bx == 0 && c == 1, right = bx == (int)gridDim.x - 1 && c == tq;
-            if (!left && !right) return;
+            const bool first = left && c == 1, last = right && c == tq;
+            if (!first && !last) return;
 #pragma unroll
             for (int f = 0; f < 3; ++f) {
                 float4 *const q = reinterpret_cast<float4 *>(line_smem + f * LSH * LSW + r * LSW) + c;
                 float4 y = *q;
-                if (f < 2 && left) q[-1] = make_float4(y.x, y.x, y.x, y.x);
-                if (right) {
+                if (f < 2 && first) q[-1] = make_float4(y.x, y.x, y.x, y.x);
+                if (last) {
                     if (n < 1) y.y = f < 2 ? y.x : 0.0f;
                     if (n < 2) y.z = f < 2 ? y.y : 0.0f;
                     if (n < 3) y.w = f < 2 ? y.z : 0.0f;
@@ -894,8 +888,47 @@ __global__ void __launch_bounds__(LNT, 2)
     }
     __syncthreads();
 
-    // Four threads of a unit: 0 and 1 take the pointwise part of its two rows, 2 and 3 the two sums of the
-    // x direction (along rows); then each one of the two sums of the y direction of one of the rows.  Two
+    // ---- the bands: products at the ends of the tile's lines, then the sums of the cells there ------------
+    if (left || right || top || bottom) {
+        const int rows = G * LR, first = 4 * LSW + 4;  // the tile's rows; its first cell's place
+        if (top || bottom)
+            for (int x = tid; x < LEND * LC; x += LNT) {
+                const int r = x / LC, c = x % LC;
+                if (c < 4 * tq)
+                    ex[x] = end_products(su, sd, sl, first + (top ? r : rows - 1 - r) * LSW + c, LSW,
+                                         r > 0 ? 2 : top ? 0 : 1, dt, rdx);
+            }
+        for (int x = tid; x < 2 * LEND * LROWS; x += LNT) {
+            const int end = x / (LEND * LROWS), r = x / LROWS % LEND, row = x % LROWS;
+            if (row < rows && (end ? right : left))
+                ey[x] = end_products(su, sd, sl, first + row * LSW + (end ? W - 1 - j0 - r : r), 1, r > 0 ? 2 : end, dt,
+                                     rdx);
+        }
+        __syncthreads();
+        if (top || bottom)
+            for (int x = tid; x < ADJ_BAND * LC; x += LNT) {
+                const int pp = x / LC, c = x % LC;
+                if (c >= 4 * tq) continue;
+                const float4 y = end_sums(ex + c, LC, taps, pp, top ? 1.0f : -1.0f, rdx);
+                // the cell's unit (see `pair`), its row there and its place in the quad
+                const int row = top ? pp : rows - 1 - pp, q = c >> 2;
+                const int un = 2 * ((q >> 1) * G + (row >> 1)) + (q & 1);
+                float *const to = reinterpret_cast<float *>(&sr[0][row & 1][un]) + (c & 3);
+                constexpr int plane = 4 * LR * LU;
+                to[0] = y.x;
+                to[plane] = y.y;
+                to[2 * plane] = y.z;
+                to[3 * plane] = y.w;
+            }
+        for (int x = tid; x < 2 * ADJ_BAND * LROWS; x += LNT) {
+            const int end = x / (ADJ_BAND * LROWS), pp = x / LROWS % ADJ_BAND, row = x % LROWS;
+            if (row < rows && (end ? right : left))
+                yr[x] = end_sums(ey + end * LEND * LROWS + row, LROWS, taps, pp, end ? -1.0f : 1.0f, rdx);
+        }
+    }
+
+    // Four threads of a unit: 0 and 1 take the pointwise part of its two rows, 2 and 3 the two halves of the
+    // x direction (along rows); then each one half of the y direction of one of the rows.  Two
     // threads: 0 the pointwise part, 1 the x direction; then each the y direction of one row.
     const int base = (lg * LR + 4) * LSW + 4 * lq + 4;  // the unit's first cell
     if (role < SHARE / 2) {
@@ -911,15 +944,14 @@ __global__ void __launch_bounds__(LNT, 2)
             float4 lv4 = sp[2][k][unit], lw4 = sp[3][k][unit];
             const float4 u4 = *reinterpret_cast<const float4 *>(su + base + k * LSW);
             const float4 l4 = *reinterpret_cast<const float4 *>(sl + base + k * LSW);
-            float4 lj4 = l4;  // lambda_u where the current is the model's
             const int i = i0 + k;
-            if (!stored) lj4 = make_float4(0.f, 0.f, 0.f, 0.f);
             if (j + 3 >= W) {  // columns beyond W: whatever lies in the padding (lambda_u is zero there)
                 if (j + 1 >= W) v4.y = w4.y = lv4.y = lw4.y = 0.f;
                 if (j + 2 >= W) v4.z = w4.z = lv4.z = lw4.z = 0.f;
                 if (j + 3 >= W) v4.w = w4.w = lv4.w = lw4.w = 0.f;
             }
-            if (active && stored)  // cells whose current a stimulus replaces
+            unsigned replaced = 0;  // cells whose current a stimulus replaces
+            if (active && stored)
                 for (unsigned x = active; x; x &= x - 1) {
                     const Stim &st = stims[__ffs(x) - 1];
                     float4 f;
@@ -932,35 +964,36 @@ __global__ void __launch_bounds__(LNT, 2)
                         f.z = in && j + 2 >= st.c0 && j + 2 < st.c1 ? st.amplitude : 0.0f;
                         f.w = in && j + 3 >= st.c0 && j + 3 < st.c1 ? st.amplitude : 0.0f;
                     }
-                    if (f.x != 0.0f) lj4.x = 0.0f;
-                    if (f.y != 0.0f) lj4.y = 0.0f;
-                    if (f.z != 0.0f) lj4.z = 0.0f;
-                    if (f.w != 0.0f) lj4.w = 0.0f;
+                    replaced |= (f.x != 0.0f ? 1u : 0u) | (f.y != 0.0f ? 2u : 0u) | (f.z != 0.0f ? 4u : 0u) |
+                                (f.w != 0.0f ? 8u : 0u);
                 }
             const float uu[4] = {u4.x, u4.y, u4.z, u4.w}, ll[4] = {l4.x, l4.y, l4.z, l4.w};
             const float vv[4] = {v4.x, v4.y, v4.z, v4.w}, ww[4] = {w4.x, w4.y, w4.z, w4.w};
             const float lvv[4] = {lv4.x, lv4.y, lv4.z, lv4.w}, lww[4] = {lw4.x, lw4.y, lw4.z, lw4.w};
-            const float ljj[4] = {lj4.x, lj4.y, lj4.z, lj4.w};
             float ov[4], ow[4], pu[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const float u = uu[c], v = vv[c], w = ww[c], lv = lvv[c], lw = lww[c], lj = ljj[c];
+                const float u = uu[c], v = vv[c], w = ww[c], lv = lvv[c], lw = lww[c], lu = ll[c];
+                const bool stim = (replaced >> c & 1u) != 0;
                 const bool p = u >= md.V_c, q = u >= md.V_v;
                 const float uk = u - md.V_csi;
                 const float S = one_plus_tanh(md.k * uk);  // 1 + tanh
                 const float sech2 = S * (2.0f - S);        // 1 - tanh^2
                 const float uc = u - md.V_c, u1 = 1.0f - u;
-                // (as one product with 1 + dt x, its rounding would act the same way in every step: dL/dv0
-                // off by up to 6e-8 per step)
-                ov[c] = fmaf(lv, dt * (p ? -md.r_tau_vp : (q ? -md.r_tau_v2m : -md.r_tau_v1m)), lv);
-                ow[c] = fmaf(lw, dt * (p ? -md.r_tau_wp : -md.r_tau_wm), lw);
+                // the cotangents: adjoint_pointwise's operations
+                const float mu = dt * lu;
+                const float dvdv = 1.0f + dt * (p ? -md.r_tau_vp : -(q ? md.r_tau_v2m : md.r_tau_v1m));
+                const float dwdw = 1.0f + dt * (p ? -md.r_tau_wp : -md.r_tau_wm);
                 const float dfi = p ? -v * (1.0f + md.V_c - 2.0f * u) * md.r_tau_d : 0.0f;
                 const float dso = p ? 0.0f : md.r_tau_0;
                 const float dsi = -w * md.k * sech2 * md.r_2tau_si;
-                const float mu = dt * lj;
-                ov[c] = fmaf(mu, p ? uc * u1 * md.r_tau_d * md.r_Cm : 0.0f, ov[c]);
-                ow[c] = fmaf(mu, S * md.r_2tau_si * md.r_Cm, ow[c]);
-                pu[c] = fmaf(mu, -(dfi + dso + dsi) * md.r_Cm, ll[c]);
+                const float dJdu = stim ? 0.0f : -(dfi + dso + dsi) * md.r_Cm;
+                const float dJdv = stim || !p ? 0.0f : uc * u1 * md.r_tau_d * md.r_Cm;
+                const float dJdw = stim ? 0.0f : S * md.r_2tau_si * md.r_Cm;
+                ov[c] = lv * dvdv + mu * dJdv;
+                ow[c] = lw * dwdw + mu * dJdw;
+                pu[c] = lu * (1.0f + dt * dJdu);
+                const float lj = stim || !stored ? 0.0f : lu;  // lambda_u where the current is the model's
                 // parameter sums without their constant factors (cardiax/params.py fields 0..11)
                 const float lvp = p ? lv : 0.0f, lvo = (lv - lvp) * (1.0f - v), lvq = q ? lvo : 0.0f;
                 const float lwp = p ? lw : 0.0f;
@@ -998,25 +1031,24 @@ __global__ void __launch_bounds__(LNT, 2)
             if (lane < 16) red[tid / 32][lane] = x;
         }
     } else {
-        V4 x[LR];
-        auto cell = [&](int f, int d) {
-            return ld_v4((f == 0 ? su : f == 1 ? sd : sl) + base + d * LSW);
-        };
-        auto of = [&](int f, int t) { return cell(f, t - 4); };
-        const bool edge = __any_sync(0xffffffffu, mine && (i0 <= 5 || i0 + LR + 1 >= H - 4)) != 0;
-        auto keep = [&](int f) {
+        Quad x[LR], y[LR];
+        auto of = [&](int f, int t) { return ld_quad((f == 0 ? su : f == 1 ? sd : sl) + base + (t - 4) * LSW); };
+        // (units in the band have their sums already)
+        const bool band = mine && (i0 < ADJ_BAND || i0 >= H - ADJ_BAND);
+        auto keep = [&](int f, Quad (&z)[LR]) {
 #pragma unroll
-            for (int k = 0; k < LR; ++k) sr[f][k][unit] = make_float4(x[k].x, x[k].y, x[k].z, x[k].w);
+            for (int k = 0; k < LR; ++k)
+                if (!band) sr[f][k][unit] = make_float4(z[k].lo.x, z[k].lo.y, z[k].hi.x, z[k].hi.y);
         };
         if (SHARE == 2 || role == 2) {
-            if (edge) axis_gd<LR, true, V4>(i0, H, of, cell, x);
-            else axis_gd<LR, false, V4>(i0, H, of, cell, x);
-            keep(1);
+            cols_gd<LR>(b.kc, of, x, y);
+            keep(2, x);
+            keep(3, y);
         }
         if (SHARE == 2 || role == 3) {
-            if (edge) axis_at<LR, true, V4>(i0, H, of, cell, x);
-            else axis_at<LR, false, V4>(i0, H, of, cell, x);
-            keep(0);
+            cols_at<LR>(b.kc, of, x, y);
+            keep(0, x);
+            keep(1, y);
         }
     }
     const int k = role & 1;
@@ -1025,11 +1057,10 @@ __global__ void __launch_bounds__(LNT, 2)
     const int64_t o = off0 + (int64_t)k * pitch;
     float4 gd4 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (takes_gd && a.gD && stored) gd4 = __ldcg(reinterpret_cast<const float4 *>(a.gD + e_plane + o));
-    float ay[4], gy[4];
+    float yt[4][4], mu[4];  // A^T, B^T, u'' and B^T (mu u') of the y direction
     {
         const int c0 = base + k * LSW;
-        auto cell = [&](int f, int d) { return (f == 0 ? su : f == 1 ? sd : sl)[c0 + d]; };
-        float L[12], F[12];
+        float M[12], F[12];
         auto row = [&](const float *p, float (&x)[12]) {
 #pragma unroll
             for (int t = 0; t < 3; ++t) {
@@ -1037,38 +1068,63 @@ __global__ void __launch_bounds__(LNT, 2)
                 x[4 * t] = q.x, x[4 * t + 1] = q.y, x[4 * t + 2] = q.z, x[4 * t + 3] = q.w;
             }
         };
-        const bool edge = __any_sync(0xffffffffu, mine && (j <= 5 || j + 5 >= W - 4)) != 0;
-        row(sl, L);
-        row(takes_gd ? su : sd, F);
-        auto of = [&](int f, int t) { return f == 2 ? L[t] : F[t]; };
-        if (takes_gd) {
-            if (edge) axis_gd<4, true, float>(j, W, of, cell, gy);
-            else axis_gd<4, false, float>(j, W, of, cell, gy);
+        row(sl, M);
+#pragma unroll
+        for (int t = 0; t < 12; t += 2) {
+            const float2 x = p_mul(mk2(M[t], M[t + 1]), b.kc.dt);
+            M[t] = x.x, M[t + 1] = x.y;
         }
+        row(takes_gd ? su : sd, F);
+        if (takes_gd) row_gd(b.kc, F, M, yt[2], yt[3]);
         if (takes_at) {
             if (takes_gd) row(sd, F);
-            if (edge) axis_at<4, true, float>(j, W, of, cell, ay);
-            else axis_at<4, false, float>(j, W, of, cell, ay);
+            row_at(b.kc, F, M, yt[0], yt[1]);
         }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) mu[c] = M[c + 4];
     }
     __syncthreads();
-    // (rdx^2 and dt apart: their product rounds, the same way in every step)
-    const float r2 = rdx * rdx;
-    // r2 dt (x + y) onto z, stored to `out`
-    auto put = [&](float4 x, const float (&y)[4], float4 z, float *out) {
-        z = make_float4(fmaf(r2, dt * (x.x + y[0]), z.x), fmaf(r2, dt * (x.y + y[1]), z.y),
-                        fmaf(r2, dt * (x.z + y[2]), z.z), fmaf(r2, dt * (x.w + y[3]), z.w));
+    // the row's cells in a band
+    if ((left && j < ADJ_BAND) || (right && j + 3 >= W - ADJ_BAND)) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int far = W - 1 - j - c;
+            const bool near0 = left && j + c < ADJ_BAND;
+            if (!near0 && !(right && far >= 0 && far < ADJ_BAND)) continue;
+            const float4 y = yr[((near0 ? 0 : ADJ_BAND) + (near0 ? j + c : far)) * LROWS + lg * LR + k];
+            yt[0][c] = y.x;
+            yt[1][c] = y.y;
+            yt[2][c] = y.z;
+            yt[3][c] = y.w;
+        }
+    }
+    auto put = [&](const float (&z)[4], float *out) {
         if (j + 3 < W) {
-            __stcg(reinterpret_cast<float4 *>(out), z);
+            __stcg(reinterpret_cast<float4 *>(out), make_float4(z[0], z[1], z[2], z[3]));
         } else {
-            const float zz[4] = {z.x, z.y, z.z, z.w};
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                if (j + c < W) __stcg(out + c, zz[c]);
+                if (j + c < W) __stcg(out + c, z[c]);
         }
     };
-    if (stored && takes_at) put(sr[0][k][unit], ay, sp[0][k][unit], a.olu + e_lam + o);
-    if (stored && takes_gd && a.gD) put(sr[1][k][unit], gy, gd4, a.gD + e_plane + o);
+    auto four = [](float4 q, float (&x)[4]) { x[0] = q.x, x[1] = q.y, x[2] = q.z, x[3] = q.w; };
+    float z[4], x0[4], x1[4];
+    if (stored && takes_at) {
+        four(sp[0][k][unit], z);
+        four(sr[0][k][unit], x0);
+        four(sr[1][k][unit], x1);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) z[c] = z[c] + ((x0[c] + yt[0][c]) + (x1[c] + yt[1][c]));
+        put(z, a.olu + e_lam + o);
+    }
+    if (stored && takes_gd && a.gD) {
+        four(gd4, z);
+        four(sr[2][k][unit], x0);
+        four(sr[3][k][unit], x1);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) z[c] = z[c] + (mu[c] * (x0[c] + yt[2][c]) + (x1[c] + yt[3][c]));
+        put(z, a.gD + e_plane + o);
+    }
     if (a.gtheta && tid < 12) {
         double x = 0.0;
 #pragma unroll
@@ -1175,6 +1231,9 @@ cudaError_t launch_line_as(const AdjointArgs &a, LineRun b, int n_exp, cudaStrea
         b.inv[q] = (65536 + b.g_each - 2 + q) / (b.g_each - 1 + q);
         b.inv_q[q] = (65536 + b.q_each + q) / (b.q_each + 1 + q);
     }
+    auto twice = [](float x) { return float2{x, x}; };
+    b.kc = LineConsts{twice(C_1_12), twice(-C_2_3), twice(C_2_3), twice(-C_1_12), twice(a.rdx), twice(-a.rdx),
+                      twice(a.dt)};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nbx, nby, n_exp);
     cfg.blockDim = dim3(LNT);
