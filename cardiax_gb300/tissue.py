@@ -68,10 +68,23 @@ def params_struct(params) -> N.Params:
 
 
 def analyse_fields(fields: Sequence[torch.Tensor]) -> list:
-    """Classifies stimulus fields of one (H, W) shape on one CUDA device: ``("empty",)`` (all
-    zero), ``("rect", r0, r1, c0, c1, a)`` (a constant ``a`` on a rectangle, zero elsewhere) or
-    ``("dense",)``.  One launch and one synchronisation for all of them (set-up cost, once per
-    tissue or batch)."""
+    """Classifies stimulus fields of one (H, W) shape: ``("empty",)`` (all zero), ``("rect", r0, r1,
+    c0, c1, a)`` (a constant ``a`` on a rectangle, zero elsewhere) or ``("dense",)``.  One launch and
+    one synchronisation for all float32 fields of a CUDA device (set-up cost, once per tissue or
+    batch); fields of another type or device are taken as they are, one by one."""
+    if not fields:
+        return []
+    if any(f.shape != fields[0].shape for f in fields):
+        raise ValueError(f"fields of different shapes: {sorted({tuple(f.shape) for f in fields})}")
+    on = [k for k, f in enumerate(fields) if f.dtype == torch.float32 and f.is_cuda and f.numel()]
+    dev = fields[on[0]].device if on else None
+    on = [k for k in on if fields[k].device == dev]
+    kinds = dict(zip(on, _analyse_on_device([fields[k] for k in on])))
+    return [kinds[k] if k in kinds else _analyse_any(f) for k, f in enumerate(fields)]
+
+
+def _analyse_on_device(fields: Sequence[torch.Tensor]) -> list:
+    """Float32 fields of one shape, at least one cell, on one CUDA device."""
     if not fields:
         return []
     H, W = (int(x) for x in fields[0].shape)
@@ -85,6 +98,22 @@ def analyse_fields(fields: Sequence[torch.Tensor]) -> list:
                W, work.data_ptr(), nbytes, out, stream_handle())
     return [("empty",) if k.kind == 0 else ("dense",) if k.kind == 2 else
             ("rect", k.r0, k.r1, k.c0, k.c1, float(k.amplitude)) for k in out]
+
+
+def _analyse_any(field: torch.Tensor):
+    """A field of any type on any device, by reductions."""
+    nz = field != 0
+    rows = torch.nonzero(nz.any(1)).flatten()
+    if rows.numel() == 0:
+        return ("empty",)
+    cols = torch.nonzero(nz.any(0)).flatten()
+    r0, r1 = int(rows[0]), int(rows[-1]) + 1
+    c0, c1 = int(cols[0]), int(cols[-1]) + 1
+    box = field[r0:r1, c0:c1]
+    a = box[0, 0]
+    if bool((box == a).all()):
+        return ("rect", r0, r1, c0, c1, float(a))
+    return ("dense",)
 
 
 def analyse_field(field: torch.Tensor):
