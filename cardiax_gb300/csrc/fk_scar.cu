@@ -32,6 +32,7 @@
 #include <cstdint>
 
 #include "../../include/cardiax_gb300.h"
+#include "fk_capi_internal.h"
 
 namespace fk {
 
@@ -295,6 +296,25 @@ __global__ void __launch_bounds__(CTH)
     }
 }
 
+size_t conv_cols_smem_bytes(int K) {
+    const size_t Kp = (size_t)((K + CR - 1) / CR * CR);
+    return sizeof(float) * ((CY + Kp) * CX + Kp);
+}
+
+// The kernels' shared-memory limits, once per thread and context, for the most taps each takes: the limit is the
+// function's, so one set to a call's own size could be lowered by another thread's call before the launch.
+bool conv_configured() {
+    static thread_local uint64_t configured_ctx = 0;
+    if (!context_changed(configured_ctx)) return true;
+    if (cudaFuncSetAttribute(fk_conv2d_tiled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)conv_smem_bytes(CONV_TILED_MAX_K)) == cudaSuccess &&
+        cudaFuncSetAttribute(fk_conv_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)conv_cols_smem_bytes(SEP_MAX_K)) == cudaSuccess)
+        return true;
+    configured_ctx = 0;
+    return false;
+}
+
 }  // namespace
 
 }  // namespace fk
@@ -329,10 +349,7 @@ extern "C" int fk_conv2d_same(const float *in, int64_t H, int64_t W, int64_t in_
     if (in == out) return FK_ERR_ARGUMENT;
     if (K <= fk::CONV_TILED_MAX_K) {
         const size_t smem = fk::conv_smem_bytes((int)K);
-        if (cudaFuncSetAttribute(fk::fk_conv2d_tiled_kernel,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess)
-            return FK_ERR_CUDA;
+        if (!fk::conv_configured()) return FK_ERR_CUDA;
         const dim3 grid((unsigned)((W + fk::CT - 1) / fk::CT), (unsigned)((H + fk::CT - 1) / fk::CT));
         if (grid.y > 65535) return FK_ERR_SHAPE;
         fk::fk_conv2d_tiled_kernel<<<grid, 256, smem, (cudaStream_t)stream>>>(
@@ -356,11 +373,8 @@ extern "C" int fk_conv2d_separable(const float *in, int64_t H, int64_t W, int64_
         H > (1 << 22) || W > (1 << 30))
         return FK_ERR_SHAPE;
     if (tmp == in || tmp == out) return FK_ERR_ARGUMENT;
-    const size_t Kp = (size_t)((K + fk::CR - 1) / fk::CR * fk::CR);
-    const size_t smem = sizeof(float) * ((fk::CY + Kp) * fk::CX + Kp);
-    if (cudaFuncSetAttribute(fk::fk_conv_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return FK_ERR_CUDA;
+    const size_t smem = fk::conv_cols_smem_bytes((int)K);
+    if (!fk::conv_configured()) return FK_ERR_CUDA;
     const dim3 rows((unsigned)((W + fk::RX - 1) / fk::RX), (unsigned)(H < 32768 ? H : 32768));
     fk::fk_conv_rows_kernel<<<rows, fk::RXT, 0, (cudaStream_t)stream>>>(in, (int)H, (int)W, in_pitch, kx, (int)K,
                                                                        tmp, tmp_pitch);
