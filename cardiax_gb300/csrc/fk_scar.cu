@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(CTH)
         acc[i] = 0.0f;
         v[i] = p[i * CX];
     }
-    for (int m = 0; m < Kp; m += CR) {
+    const int whole = K / CR * CR;
+    for (int m = 0; m < whole; m += CR) {
 #pragma unroll
         for (int i = 0; i < CR; ++i) v[CR + i] = p[(m + CR + i) * CX];
 #pragma unroll
@@ -288,6 +289,18 @@ __global__ void __launch_bounds__(CTH)
         }
 #pragma unroll
         for (int i = 0; i < CR; ++i) v[i] = v[CR + i];
+    }
+    // the last taps: rows beyond an output's window must not be touched (zero times an infinity there is not zero)
+    if (whole < K) {
+#pragma unroll
+        for (int i = 0; i < CR; ++i) v[CR + i] = p[(whole + CR + i) * CX];
+#pragma unroll
+        for (int t = 0; t < CR - 1; ++t) {
+            if (whole + t >= K) break;
+            const float w = ks[whole + t];
+#pragma unroll
+            for (int i = 0; i < CR; ++i) acc[i] = fmaf(w, v[i + t], acc[i]);
+        }
     }
 #pragma unroll
     for (int i = 0; i < CR; ++i) {
