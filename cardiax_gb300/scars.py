@@ -168,18 +168,27 @@ def outer_factors(weights: np.ndarray):
     return (ky, kx) if off <= 2.0 ** -22 * np.abs(w).sum() else None
 
 
+def _worth_factoring(H: int, W: int, K: int) -> bool:
+    """Whether two one-dimensional passes repay the test of the weights, the second launch and the
+    larger upload, some 70 us of a call: the direct sum takes 0.045 us K^2 for each round of its
+    64 x 64 tiles over the SMs.  us per call, direct | separable: 400^2, K = 40 114 | 126 and 50
+    165 | 129; 800^2, 25 93 | 120 and 40 168 | 120; 1200^2, 20 88 | 117 and 32 153 | 118; 2000^2,
+    12 85 | 114 and 20 161 | 117."""
+    tiles = -(-H // 64) * -(-W // 64)
+    return 8 <= K <= SEPARABLE_MAX_TAPS and H <= 1 << 22 and K * K * max(tiles, 152) > 250_000
+
+
 def blur_same(plane: torch.Tensor, weights: np.ndarray, one_minus: bool = False) -> torch.Tensor:
     """scipy.signal.convolve2d(plane, weights, "same") in float32, or 1 minus it:
     ``fk_conv2d_same``, or two one-dimensional passes (``fk_conv2d_separable``) for weights that
-    are an outer product, as a Gaussian's are."""
+    are an outer product, as a Gaussian's are, where there are enough of them."""
     H, W = int(plane.shape[0]), int(plane.shape[1])
     K = int(weights.shape[0])
     if weights.shape != (K, K):
         raise ValueError("the weights must be square")
     src = plane.to(torch.float32).contiguous()
     out = torch.empty((H, W), dtype=torch.float32, device=src.device)
-    # below about 8 taps the direct sum reads its inputs once and is the faster one
-    factors = outer_factors(weights) if 8 <= K <= SEPARABLE_MAX_TAPS and H <= 1 << 22 else None
+    factors = outer_factors(weights) if _worth_factoring(H, W, K) else None
     if factors is not None:
         k = torch.as_tensor(np.stack(factors), device=src.device)
         tmp = torch.empty_like(out)
