@@ -115,6 +115,7 @@ _SIGNATURES = {
     "fk_batch_set_options": [_P, _INT, _INT],
     "fk_batch_set_depth": [_P, _INT],
     "fk_batch_set_resident": [_P, _INT],
+    "fk_batch_takes_resident": [_P, _I64],
     "fk_batch_destroy": [_P],
 }
 

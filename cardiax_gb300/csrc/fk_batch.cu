@@ -63,7 +63,7 @@ struct fk_batch {
     // the resident kernel in place of one launch per step (fk_batch_set_resident; turned off by the
     // knobs of the stepping kernel)
     ResWaves res;
-    bool resident = false;
+    int resident = 0;  // 2: whatever the estimate says
     ResTissue *d_res = nullptr;
     uint64_t *d_xchg = nullptr;
     std::vector<ResTissue> h_res;
@@ -306,6 +306,12 @@ ResWaves plan_waves(const fk_tissue *ts, int n) {
 // step (4.4 us at least, about 140 GCUPS on mixed tissues).
 double res_time(const ResWaves &r, int64_t n) { return (double)r.w.size() * 30.0 + r.cost * (double)n; }
 double step_time(int64_t cells, int64_t n) { return std::max(4.4, (double)cells / 140e3) * (double)n; }
+// Whether n steps take the resident launches; stepping them takes `more` us more than step_time, they
+// `also` more than res_time.
+bool takes_resident(const fk_batch *b, int64_t n, double more = 0.0, double also = 0.0) {
+    return b->resident == 2 ||
+           (b->resident && res_time(b->res, n) + also < step_time(b->cells, n) + more);
+}
 
 // Relative cost of an edge tile (clamped halo, one-sided rows, bounds checks) against an
 // interior one, for balancing the CTAs' runs of the work list.
@@ -546,7 +552,7 @@ int fk_batch_create(const fk_tissue *tissues, int n, void *workspace, size_t byt
     for (int k = 0; k < n; ++k) b->tb_ok &= tb_batchable(tissues[k].g.H, tissues[k].g.W);
     b->d_t = reinterpret_cast<int *>(ws + L.t);
     b->res = std::move(res);
-    b->resident = b->res.ok();
+    b->resident = b->res.ok() ? 1 : 0;
     b->d_res = reinterpret_cast<ResTissue *>(ws + L.res);
     b->d_xchg = reinterpret_cast<uint64_t *>(ws + L.xchg);
     for (int k = 0; k < n; ++k) b->cells += tissues[k].g.H * tissues[k].g.W;
@@ -678,14 +684,18 @@ int fk_batch_create(const fk_tissue *tissues, int n, void *workspace, size_t byt
 int fk_batch_set_resident(fk_batch *b, int on) {
     if (!b) return FK_ERR_NULL;
     if (on && !b->res.ok()) return FK_ERR_ARGUMENT;
-    b->resident = on != 0;
+    b->resident = on == 2 ? 2 : on != 0;
     return FK_OK;
+}
+
+int fk_batch_takes_resident(const fk_batch *b, int64_t steps) {
+    return b && steps >= 2 && takes_resident(b, steps) ? 1 : 0;
 }
 
 int fk_batch_set_grid(fk_batch *b, int ctas) {
     if (!b) return FK_ERR_NULL;
     if (ctas < 1 || ctas > kBatchMaxGrid) return FK_ERR_ARGUMENT;
-    b->resident = false;
+    b->resident = 0;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev != b->device) return FK_ERR_CUDA;
     // ordered after the plan's earlier work; the host copies stay alive in the plan
@@ -715,7 +725,7 @@ int fk_batch_set_options(fk_batch *b, int interleave, int packed) {
     if (interleave != 0 && interleave != 1 && interleave != 2 && interleave != 4 &&
         interleave != 8)
         return FK_ERR_ARGUMENT;
-    b->resident = false;
+    b->resident = 0;
     const int il = interleave, pk = packed ? 1 : 0;
     if (il != b->interleave || pk != b->packed) release_graph(b);
     b->packed = pk;
@@ -741,7 +751,7 @@ int fk_batch_set_depth(fk_batch *b, int depth) {
     if (!b) return FK_ERR_NULL;
     if (depth != 1 && depth != kBatchTbDepth) return FK_ERR_ARGUMENT;
     if (depth != 1 && !b->tb_ok) return FK_ERR_ARGUMENT;
-    b->resident = false;
+    b->resident = 0;
     if (depth != b->depth) release_graph(b);
     b->depth = depth;
     return FK_OK;
@@ -752,7 +762,7 @@ int fk_batch_set_tile_rows(fk_batch *b, int rows) {
     for (int q = 0; q < kShapes; ++q)
         if (kShape[q].rows == rows) {
             if (b->shape != q) release_graph(b);
-            b->resident = false;
+            b->resident = 0;
             b->shape = q;
             return FK_OK;
         }
@@ -836,7 +846,7 @@ int fk_batch_forward_euler(fk_batch *b, int64_t t0, int64_t t1, int graph_steps,
     int64_t n = t1 - t0;
     if (n == 0) return FK_OK;
     // (two steps at least: in place, a block may write its cells only after its neighbours' first loads)
-    if (b->resident && n >= 2 && res_time(b->res, n) < step_time(b->cells, n))
+    if (n >= 2 && takes_resident(b, n))
         return run_resident(b, t0, n, ResOut{}, s);
     set_int_kernel<<<1, 1, 0, s>>>(b->d_t, (int)t0);
     if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
@@ -920,7 +930,7 @@ int fk_batch_forward_states(fk_batch *b, int64_t t0, const int64_t *steps, float
         const int64_t n = m ? steps[k + m - 1] - t : 0;
         // (a stepped state is also copied out, and one more resident launch copies the last one back)
         const double copy = 2.0 + (double)b->cells / 170e3;
-        if (m && res_time(b->res, n) + copy < step_time(b->cells, n) + m * copy) {
+        if (m && takes_resident(b, n, m * copy, copy)) {
             int rc = run_resident(b, t, n, ResOut{outs[k], exp_stride, 0, steps + k, outs + k, m}, s);
             if (rc) return rc;
             k += m;
@@ -952,8 +962,8 @@ int fk_batch_recompute(fk_batch *b, int64_t s, int64_t n, float *bufs, int64_t e
     const dim3 cgrid(64, b->n);
     // (a step outside the resident kernel also copies its states out: 12 bytes per cell read and
     // written, at about 4 TB/s from L2)
-    if (b->resident && n - 1 >= 2 && n - 1 <= kResMaxSteps &&
-        res_time(b->res, n - 1) < step_time(b->cells, n - 1) + (double)(n - 1) * (2.0 + (double)b->cells / 170e3)) {
+    if (n - 1 >= 2 && n - 1 <= kResMaxSteps &&
+        takes_resident(b, n - 1, (double)(n - 1) * (2.0 + (double)b->cells / 170e3))) {
         batch_state_out_kernel<<<cgrid, 256, 0, cs>>>(b->d_tissues, 0, bufs, exp_stride, ns);
         if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
         return run_resident(b, s, n - 1, ResOut{bufs, exp_stride, ns, nullptr, nullptr, 0}, cs);

@@ -349,8 +349,11 @@ int fk_batch_set_depth(fk_batch *plan, int depth);
  * plan's tissues that fit on chip together, one set after the other: on by default where every tissue
  * can take it (16 x 16 to about 1240 x 1240, no activation tracking) and a call has steps enough to
  * gain; the results do not change.  The other knobs tune the stepping kernel and turn it off.  Turning
- * it on where it does not apply is FK_ERR_ARGUMENT. */
+ * it on where it does not apply is FK_ERR_ARGUMENT.  `on` = 2: for every call of two steps or more,
+ * whether it gains or not. */
 int fk_batch_set_resident(fk_batch *plan, int on);
+/* Whether a call of `steps` steps would take the resident kernel as the plan stands (1 or 0). */
+int fk_batch_takes_resident(const fk_batch *plan, int64_t steps);
 
 int fk_batch_destroy(fk_batch *plan);
 
