@@ -18,7 +18,9 @@ from .tissue import Tissue, stream_handle
 
 class TissueBatch:
     """A batch of :class:`Tissue` objects on one device (shapes, parameters, D maps, stimuli and
-    dt/dx may all differ).  ``advance(t0, t1)`` steps every tissue in place."""
+    dt/dx may all differ).  ``advance(t0, t1)`` steps every tissue in place: many steps of tissues
+    that fit on chip by the resident kernel (:meth:`set_resident`), else by the batched kernel, whose
+    items have ``tile_rows`` rows (:meth:`set_tile_rows`, with 32 too, has it take every call)."""
 
     def __init__(self, tissues: Sequence[Tissue], graph_steps: int = 64, ctas: int = None,
                  tile_rows: int = 32):

@@ -255,7 +255,8 @@ class Tissue:
         from .batch import TissueBatch
         b = self._batches.get(tile_rows)
         if b is None:
-            b = TissueBatch([self], tile_rows=tile_rows)
+            # (set, not left at the default: the batched kernel, not the resident one)
+            b = TissueBatch([self]).set_tile_rows(tile_rows)
             self._batches[tile_rows] = b
         return b
 
