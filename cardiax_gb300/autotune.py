@@ -15,8 +15,8 @@ temporally blocked kernel at depth k in {2, 4, 8} (k steps per launch), and the 
 schedule -- on the tissue's own grid, and keeps the fastest.  All of them produce the same bits,
 so the choice changes only the speed (``Tissue.advance(..., schedule="auto")``).
 
-Both restore the timed state afterwards and cache their choice per (device name, shapes) for the
-process.
+Both restore the timed state afterwards and cache their choice for the process: per device name and
+shapes, ``tune_batch`` also per number of different (parameters, dt, dx) and activation tracking.
 """
 from __future__ import annotations
 
@@ -42,8 +42,11 @@ OPTION_CANDIDATES = ((1, False), (2, False), (4, False), (0, False), (1, True), 
 
 
 def _signature(batch: TissueBatch):
+    # the sets of constants and activation tracking decide whether and how the tissues run resident
     shapes = tuple(sorted((t.H, t.W) for t in batch.tissues))
-    return (torch.cuda.get_device_name(batch.device), shapes)
+    constants = len({(bytes(t.params), t.dt, t.dx) for t in batch.tissues})
+    tracking = any(t.activation is not None for t in batch.tissues)
+    return (torch.cuda.get_device_name(batch.device), shapes, constants, tracking)
 
 
 DEPTH_CANDIDATES = (1, 2)
@@ -73,8 +76,7 @@ def tune_batch(batch: TissueBatch, trial_steps: int = 256, candidates=GRAPH_CAND
     if key in _CACHE:
         res = _CACHE[key]
         _set_batch(batch, res["choice"])
-        batch.set_resident(res["resident"])
-        return res
+        return {**res, "resident": batch.set_resident(res["resident"])}
     saved = [(t.state.clone(), None if t.activation is None else
               (t.act_first.clone(), t.act_last.clone(), t.act_count.clone()))
              for t in batch.tissues]
@@ -106,7 +108,8 @@ def tune_batch(batch: TissueBatch, trial_steps: int = 256, candidates=GRAPH_CAND
     best = min(timings, key=timings.get)
     _set_batch(batch, best)
     resident_ms = None
-    if batch.set_resident(True):
+    # (a call that the plan would step all the same says nothing about the resident path)
+    if batch.set_resident(True) and N.lib().fk_batch_takes_resident(batch._plan, trial_steps):
         batch.advance(0, trial_steps)  # warm-up: the kernel's attributes
         resident_ms = timed(0)
         if verbose:

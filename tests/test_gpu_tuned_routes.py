@@ -33,3 +33,24 @@ def test_the_batch_schedule_is_the_batched_kernel(rows):
     u.advance(0, 64)
     for a, b in zip(t.view(), u.view()):
         assert torch.equal(a, b)
+
+
+KNOBS = dict(trial_steps=64, candidates=(0,), tile_rows=(32,), options=((1, False),), depths=(1,))
+
+
+def test_batches_of_the_same_shapes_are_tuned_apart():
+    """37 sets of constants are three resident launches, which the plan never takes; one set is one launch.
+    Tracked tissues cannot take it.  Whichever is tuned first must not decide for the others."""
+    from cardiax_gb300.autotune import tune_batch
+    for turn in range(2):  # measured, then from the cache
+        many = TissueBatch([_tissue(48, 52, k) for k in range(37)])
+        res = tune_batch(many, **KNOBS)
+        assert res["resident"] is False and res["resident_ms_per_step"] is None
+        one = TissueBatch([_tissue(48, 52) for _ in range(37)])
+        res = tune_batch(one, **KNOBS)
+        assert res["resident_ms_per_step"] > 0
+        assert res["resident"] == (res["resident_ms_per_step"] < min(res["ms_per_step"].values()))
+        assert _takes_resident(one._plan) == res["resident"]
+        tracked = TissueBatch([_tissue(48, 52).track_activation(0.5) for _ in range(37)])
+        res = tune_batch(tracked, **KNOBS)
+        assert res["resident"] is False and res["resident_ms_per_step"] is None
