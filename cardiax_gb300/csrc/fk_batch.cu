@@ -299,7 +299,10 @@ ResWaves plan_waves(const fk_tissue *ts, int n) {
             rows = R;
         }
     }
-    return best.w.size() > 1 ? plan_waves_rows(ts, n, plans, rows, true) : best;
+    if (best.w.size() > 1) best = plan_waves_rows(ts, n, plans, rows, true);
+    // the most blocks first: where the device refuses a launch, nothing has run yet (see run_resident)
+    std::stable_sort(best.w.begin(), best.w.end(), [](const ResWave &x, const ResWave &y) { return x.ctas > y.ctas; });
+    return best;
 }
 
 // us of n steps: the resident launches (a launch's fixed cost is 15 to 30 us), and one launch per
@@ -432,7 +435,7 @@ void fill_resident(fk_batch *b) {
 // n steps from t0 of every tissue through the resident launches: in place; or, n at most kResMaxSteps,
 // leaving the tissues' own states as they were and writing those of tissue k to base + k * stride + an
 // offset: every x_{t0+s}, s = 1 .. n, at offset s * every, or those of the steps steps[i] (n_outs of
-// them, the last one t0 + n) at offset outs[i] - base.
+// them, the last one t0 + n) at offset outs[i] - base.  kRefused: the first launch was, nothing ran.
 struct ResOut {
     float *base = nullptr;
     int64_t stride = 0, every = 0;
@@ -467,9 +470,11 @@ int run_resident(const fk_batch *b, int64_t t0, int64_t n, const ResOut &out, cu
                     ra.out_off[k] = out.outs[k] - out.base;
                 }
             }
-            if (cudaMemsetAsync(b->d_xchg, 0, (size_t)(w.ctas * 2 * ra.slot) * 8, s) != cudaSuccess ||
-                launch_resident(w.rows, w.ctas, w.threads, w.smem, false, ra, a, s) != cudaSuccess)
+            if (cudaMemsetAsync(b->d_xchg, 0, (size_t)(w.ctas * 2 * ra.slot) * 8, s) != cudaSuccess)
                 return FK_ERR_CUDA;
+            const cudaError_t e = launch_resident(w.rows, w.ctas, w.threads, w.smem, false, ra, a, s);
+            if (e != cudaSuccess)
+                return e == kResRefused && &w == b->res.w.data() && done == 0 ? kRefused : FK_ERR_CUDA;
             done += c;
         }
     }
@@ -846,8 +851,10 @@ int fk_batch_forward_euler(fk_batch *b, int64_t t0, int64_t t1, int graph_steps,
     int64_t n = t1 - t0;
     if (n == 0) return FK_OK;
     // (two steps at least: in place, a block may write its cells only after its neighbours' first loads)
-    if (n >= 2 && takes_resident(b, n))
-        return run_resident(b, t0, n, ResOut{}, s);
+    if (n >= 2 && takes_resident(b, n)) {
+        const int rc = run_resident(b, t0, n, ResOut{}, s);
+        if (rc != kRefused) return rc;
+    }
     set_int_kernel<<<1, 1, 0, s>>>(b->d_t, (int)t0);
     if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
     // the smem attribute must be set outside any capture: one plain (empty-range) call does it
@@ -920,10 +927,11 @@ int fk_batch_forward_states(fk_batch *b, int64_t t0, const int64_t *steps, float
     cudaStream_t s = (cudaStream_t)stream;
     const dim3 cgrid(64, b->n);
     int64_t t = t0;
+    bool refused = false;
     for (int k = 0; k < n_steps;) {
         // as many states, of distinct steps, as one resident launch writes
         int m = 0;
-        if (b->resident)
+        if (b->resident && !refused)
             while (k + m < n_steps && m < kResMaxOut && steps[k + m] > (m ? steps[k + m - 1] : t) &&
                    steps[k + m] - t <= kResMaxSteps)
                 ++m;
@@ -932,6 +940,10 @@ int fk_batch_forward_states(fk_batch *b, int64_t t0, const int64_t *steps, float
         const double copy = 2.0 + (double)b->cells / 170e3;
         if (m && takes_resident(b, n, m * copy, copy)) {
             int rc = run_resident(b, t, n, ResOut{outs[k], exp_stride, 0, steps + k, outs + k, m}, s);
+            if (rc == kRefused) {
+                refused = true;
+                continue;
+            }
             if (rc) return rc;
             k += m;
             batch_state_in_kernel<<<cgrid, 256, 0, s>>>(b->d_tissues, outs[k - 1], exp_stride, ns);
@@ -966,7 +978,8 @@ int fk_batch_recompute(fk_batch *b, int64_t s, int64_t n, float *bufs, int64_t e
         takes_resident(b, n - 1, (double)(n - 1) * (2.0 + (double)b->cells / 170e3))) {
         batch_state_out_kernel<<<cgrid, 256, 0, cs>>>(b->d_tissues, 0, bufs, exp_stride, ns);
         if (cudaGetLastError() != cudaSuccess) return FK_ERR_CUDA;
-        return run_resident(b, s, n - 1, ResOut{bufs, exp_stride, ns, nullptr, nullptr, 0}, cs);
+        const int rc = run_resident(b, s, n - 1, ResOut{bufs, exp_stride, ns, nullptr, nullptr, 0}, cs);
+        if (rc != kRefused) return rc;
     }
     set_int_kernel<<<1, 1, 0, cs>>>(b->d_t, (int)s);
     batch_state_out_kernel<<<cgrid, 256, 0, cs>>>(b->d_tissues, 0, bufs, exp_stride, ns);

@@ -467,7 +467,7 @@ static cudaError_t launch_plan(const ResPlan &plan, void *workspace, const Resid
 
 // Steps t0 .. t0+n-1 from `in` through the resident kernel, states written to `base` + offset after the
 // steps listed in `outs` ((step, offset) pairs in step order, the last one at step n); `tmp` (one state)
-// holds the state between launches that end at no listed step.
+// holds the state between launches that end at no listed step.  kRefused: the first launch was, nothing ran.
 static int resident_run(const ResPlan &plan, const fk_grid &g, const float *in, float *base,
                         const std::vector<std::pair<int64_t, int64_t>> &outs, float *tmp, const float *D,
                         const Model &m, const Stim *st, int ns, int64_t t0, int64_t n, float dt, float rdx,
@@ -497,8 +497,8 @@ static int resident_run(const ResPlan &plan, const fk_grid &g, const float *in, 
             in = tmp;
         }
         ra.n = (int)c;
-        if (launch_plan(plan, workspace, ra, a, s) != cudaSuccess)
-            return FK_ERR_CUDA;
+        const cudaError_t e = launch_plan(plan, workspace, ra, a, s);
+        if (e != cudaSuccess) return e == kResRefused && done == 0 ? kRefused : FK_ERR_CUDA;
         done += c;
     }
     return FK_OK;
@@ -575,6 +575,12 @@ int fk_selftest_wait_timeout(int64_t limit_ns, void *stream) {
     if (!st) return FK_ERR_CUDA;
     fk::selftest_wait_kernel<<<1, 32, 0, (cudaStream_t)stream>>>((uint64_t)limit_ns, st);
     return cudaGetLastError() == cudaSuccess ? FK_OK : FK_ERR_CUDA;
+}
+
+int fk_selftest_refuse_resident(int launches) {
+    if (launches < 0) return FK_ERR_ARGUMENT;
+    refuse_resident_launches(launches);
+    return FK_OK;
 }
 
 int fk_init(fk_grid g, float *state, void *stream) {
@@ -696,10 +702,11 @@ int fk_forward_euler_resident(fk_grid g, float *state, float *scratch, const flo
     int rc = common_checks(g, state, scratch, D, p, dx);
     if (rc) return rc;
     if (t1 < t0 || !std::isfinite(dt)) return FK_ERR_ARGUMENT;
+    auto stepped = [&] {
+        return fk_forward_euler_tracked(g, state, scratch, D, p, stimuli, n_stimuli, t0, t1, dt, dx, act, stream);
+    };
     ResPlan plan;
-    if (!takes_resident(g, t1 - t0, n_stimuli, workspace, workspace_bytes, plan))
-        return fk_forward_euler_tracked(g, state, scratch, D, p, stimuli, n_stimuli, t0, t1, dt, dx,
-                                        act, stream);
+    if (!takes_resident(g, t1 - t0, n_stimuli, workspace, workspace_bytes, plan)) return stepped();
     if (act) {
         if (!act->first || !act->last || !act->count) return FK_ERR_NULL;
         if (!std::isfinite(act->threshold)) return FK_ERR_ARGUMENT;
@@ -709,9 +716,10 @@ int fk_forward_euler_resident(fk_grid g, float *state, float *scratch, const flo
     int *status = status_ptr();
     if (!status) return FK_ERR_CUDA;
     const int64_t n = t1 - t0;
-    return resident_run(plan, g, state, state, {{n, 0}}, scratch, D, make_model(*p), st,
-                        n_stimuli, t0, n, (float)dt, 1.0f / (float)dx, act, workspace,
-                        status, (cudaStream_t)stream);
+    rc = resident_run(plan, g, state, state, {{n, 0}}, scratch, D, make_model(*p), st,
+                      n_stimuli, t0, n, (float)dt, 1.0f / (float)dx, act, workspace,
+                      status, (cudaStream_t)stream);
+    return rc == kRefused ? stepped() : rc;
 }
 
 int64_t fk_flow_flag_words(fk_grid g) {
@@ -985,10 +993,12 @@ int fk_forward_resident(fk_grid g, const float *state0, float *scratch, const fl
     for (int i = 0; i + 1 < n_checkpoints; ++i)
         if (checkpoints[i + 1] < checkpoints[i]) return FK_ERR_ARGUMENT;
     const int64_t t0 = checkpoints[0], n = checkpoints[n_checkpoints - 1] - t0;
+    auto stepped = [&] {
+        return fk_forward(g, state0, scratch, D, p, stimuli, n_stimuli, checkpoints, n_checkpoints, dt, dx, out,
+                          stream);
+    };
     ResPlan plan;
-    if (!takes_resident(g, n, n_stimuli, workspace, workspace_bytes, plan))
-        return fk_forward(g, state0, scratch, D, p, stimuli, n_stimuli, checkpoints, n_checkpoints,
-                          dt, dx, out, stream);
+    if (!takes_resident(g, n, n_stimuli, workspace, workspace_bytes, plan)) return stepped();
     Stim st[kMaxStim];
     if ((rc = make_stims(stimuli, n_stimuli, g, st))) return rc;
     int *status = status_ptr();
@@ -1002,7 +1012,7 @@ int fk_forward_resident(fk_grid g, const float *state0, float *scratch, const fl
     if ((rc = resident_run(plan, g, state0, out, outs, scratch, D, make_model(*p), st, n_stimuli,
                            t0, n, (float)dt, 1.0f / (float)dx, nullptr, workspace, status,
                            s)))
-        return rc;
+        return rc == kRefused ? stepped() : rc;
     const float *cur = state0;
     for (int i = 0; i + 1 < n_checkpoints; ++i) {  // intervals of no steps repeat the state before
         float *dst = out + i * n_state;
@@ -1032,17 +1042,18 @@ int fk_forward_states(fk_grid g, float *state, float *scratch, const float *D, c
     const size_t bytes = sizeof(float) * 3 * g.H * g.pitch;
     const int64_t n = steps[n_steps - 1] - t0;
     cudaStream_t s = (cudaStream_t)stream;
-    ResPlan plan;
-    if (!takes_resident(g, n, n_stimuli, workspace, workspace_bytes, plan)) {
+    auto stepped = [&]() -> int {
         for (int k = 0; k < n_steps; ++k) {
-            if ((rc = fk_forward_euler_tracked(g, state, scratch, D, p, stimuli, n_stimuli,
-                                               k ? steps[k - 1] : t0, steps[k], dt, dx, nullptr, stream)))
-                return rc;
+            if (int e = fk_forward_euler_tracked(g, state, scratch, D, p, stimuli, n_stimuli,
+                                                 k ? steps[k - 1] : t0, steps[k], dt, dx, nullptr, stream))
+                return e;
             if (cudaMemcpyAsync(outs[k], state, bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
                 return FK_ERR_CUDA;
         }
         return FK_OK;
-    }
+    };
+    ResPlan plan;
+    if (!takes_resident(g, n, n_stimuli, workspace, workspace_bytes, plan)) return stepped();
     Stim st[kMaxStim];
     if ((rc = make_stims(stimuli, n_stimuli, g, st))) return rc;
     int *status = status_ptr();
@@ -1052,7 +1063,7 @@ int fk_forward_states(fk_grid g, float *state, float *scratch, const float *D, c
         if (steps[k] > (k ? steps[k - 1] : t0)) at.push_back({steps[k] - t0, outs[k] - state});
     if ((rc = resident_run(plan, g, state, state, at, scratch, D, make_model(*p), st, n_stimuli, t0, n,
                            (float)dt, 1.0f / (float)dx, nullptr, workspace, status, s)))
-        return rc;
+        return rc == kRefused ? stepped() : rc;
     for (int k = 0; k <= n_steps; ++k) {  // steps listed twice; then the state itself
         const float *src = k ? outs[k - 1] : state;
         if ((k == n_steps || steps[k] == (k ? steps[k - 1] : t0)) &&
@@ -1234,9 +1245,10 @@ int fk_recompute_resident(fk_grid g, const float *state, int64_t s, int64_t n, c
                           const fk_params *p, const fk_stimulus *stimuli, int n_stimuli, double dt,
                           double dx, float *buf, void *workspace, size_t workspace_bytes, void *stream) {
     ResPlan plan;
+    auto stepped = [&] { return fk_recompute(g, state, s, n, D, p, stimuli, n_stimuli, dt, dx, buf, stream); };
     if (check_grid(g) || n - 1 > kResMaxSteps ||  // (one launch writes every state)
         !takes_resident(g, n - 1, n_stimuli, workspace, workspace_bytes, plan))
-        return fk_recompute(g, state, s, n, D, p, stimuli, n_stimuli, dt, dx, buf, stream);
+        return stepped();
     int rc = common_checks(g, state, buf, D, p, dx);
     if (rc) return rc;
     if (!std::isfinite(dt)) return FK_ERR_ARGUMENT;
@@ -1256,9 +1268,8 @@ int fk_recompute_resident(fk_grid g, const float *state, int64_t s, int64_t n, c
     ra.t0 = s;
     ra.n = (int)(n - 1);
     ra.every = ns;
-    if (launch_plan(plan, workspace, ra, a, cs) != cudaSuccess)
-        return FK_ERR_CUDA;
-    return FK_OK;
+    const cudaError_t e = launch_plan(plan, workspace, ra, a, cs);
+    return e == cudaSuccess ? FK_OK : e == kResRefused ? stepped() : FK_ERR_CUDA;
 }
 
 int fk_adjoint_range(fk_grid g, const float *buf, int64_t s, int64_t n, const float *D,

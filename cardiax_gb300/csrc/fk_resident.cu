@@ -831,8 +831,8 @@ static cudaError_t launch_rows(const cudaLaunchConfig_t &cfg, const ResidentArgs
     return a.act_last ? launch_one<R, true, false>(cfg, ra, a, k) : launch_one<R, false, false>(cfg, ra, a, k);
 }
 
-cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, bool cluster, const ResidentArgs &ra,
-                            const StepArgs &a, cudaStream_t stream) {
+static cudaError_t launch_any(int rows, int ctas, int threads, size_t smem, bool cluster, const ResidentArgs &ra,
+                              const StepArgs &a, cudaStream_t stream) {
     const ResLaunch l(ctas, threads, smem, cluster, stream);
     const PackConsts k = make_pack_consts(a.m, a.rdx, a.dt);
     if (cluster) {
@@ -846,6 +846,26 @@ cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, bool c
         case 4: return launch_rows<4>(l.cfg, ra, a, k);
         case 5: return launch_rows<5>(l.cfg, ra, a, k);
         default: return cudaErrorInvalidValue;
+    }
+}
+
+static thread_local int refusals = 0;
+void refuse_resident_launches(int n) { refusals = n; }
+
+cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, bool cluster, const ResidentArgs &ra,
+                            const StepArgs &a, cudaStream_t stream) {
+    if (refusals > 0) {
+        --refusals;
+        return kResRefused;
+    }
+    const cudaError_t e = launch_any(rows, ctas, threads, smem, cluster, ra, a, stream);
+    switch (e) {
+        case cudaErrorCooperativeLaunchTooLarge:
+        case cudaErrorInvalidClusterSize:
+        case cudaErrorLaunchOutOfResources:
+            cudaGetLastError();  // (not the next call's error)
+            return kResRefused;
+        default: return e;
     }
 }
 

@@ -47,6 +47,8 @@ void resident_plans(int64_t H, int64_t W, int most, int rows, std::vector<ResPla
 // The fastest plan on a device of n_sm SMs that takes clusters of up to max_cluster blocks, and on the current device (not ok() without one).
 ResPlan resident_plan(int64_t H, int64_t W, int n_sm, int max_cluster);
 ResPlan resident_plan(int64_t H, int64_t W);
+// The calling thread's next n resident launches are refused (self-test).
+void refuse_resident_launches(int n);
 // The most blocks a launch may use on the current device (0: no cooperative launches, no device).
 int resident_ctas();
 
@@ -87,6 +89,10 @@ struct ResidentArgs {
 // Launches ra.n steps with `rows` rows per thread; `a` describes the one tissue (several: only its
 // dt and dx constants are read, by the launch-wide stencil coefficients).  The words of the strips
 // must be zero.
+// kResRefused: the device does not run that many blocks at once at present (a context with fewer SMs than the
+// device); nothing was launched, and one launch per step still runs.
+constexpr cudaError_t kResRefused = cudaErrorCooperativeLaunchTooLarge;
+constexpr int kRefused = -1;  // the same as a return code of the functions that call it (never of an entry point)
 cudaError_t launch_resident(int rows, int ctas, int threads, size_t smem, bool cluster, const ResidentArgs &ra,
                             const StepArgs &a, cudaStream_t stream);
 

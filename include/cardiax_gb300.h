@@ -90,6 +90,10 @@ int fk_device_status(int reset, int *value);
  * usable.  No counterpart in the reference. */
 int fk_selftest_wait_timeout(int64_t limit_ns, void *stream);
 
+/* Self-test: the calling thread's next `launches` launches of the resident kernel are refused, as on a
+ * context that runs fewer blocks at once than the device; their calls then take one launch per step. */
+int fk_selftest_refuse_resident(int launches);
+
 /* Which kernel takes the Euler steps of every single-tissue entry point (process-wide):
  * 0 = the tiled kernel (32 x 64-cell tiles, two passes) -- the default; 1 = the strip kernel
  * (128-column strips walked row by row with register windows) wherever it applies (W % 128 != 1),
