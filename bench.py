@@ -624,16 +624,18 @@ def run_next_rows(dev, reps: int = 2):
     e1.record()
     torch.cuda.synchronize()
     t_blur = e0.elapsed_time(e1) / 5 / 1e3
+    two = scars._worth_factoring(Hs, Hs, K) and scars.outer_factors(wts) is not None
     scar_r = {"size": f"{Hs}x{Hs}", "blobs": d.n_blobs, "taps": K,
               "ms_per_map": t_sc * 1e3, "blur_ms": t_blur * 1e3,
-              "blur_tflops": 2.0 * K * K * Hs * Hs / t_blur / 1e12}
+              "blur_passes": 2 if two else 1,
+              "blur_tflops": (4.0 * K if two else 2.0 * K * K) * Hs * Hs / t_blur / 1e12}
     return {"heun": heun_r, "sequence": seq_r, "hdf5": h5_r, "scar": scar_r}
 
 
 def run_schedules(dev, sizes=(256, 512, 1024, 2048), steps: int = 400):
     """GCUPS of each stepping schedule on the roofline workload (best of 2 runs of ``steps``
     steps, L2 flushed before each run), and of ``schedule="auto"`` with the choice the tissue
-    autotuner made."""
+    autotuner made.  "k1" is the default schedule: resident where the tissue fits on chip."""
     import torch
     from cardiax_gb300 import params
     from cardiax_gb300.stimulus import Protocol, Stimulus
@@ -670,7 +672,9 @@ def run_schedules(dev, sizes=(256, 512, 1024, 2048), steps: int = 400):
                 row[name]["choice"] = {"schedule": sched, "depth": depth,
                                        "kernel": (f"batched, {kernel}-row items"
                                                   if sched == "batch" else
-                                                  "strip" if kernel else "tiled")}
+                                                  "strip" if kernel else
+                                                  "resident" if sched == "step" and depth == 1
+                                                  and tis._resident_workspace()[1] else "tiled")}
         out[f"{size}x{size}"] = row
     return out
 

@@ -9,8 +9,8 @@ CUDA graph replays), over a short run with CUDA events, and keeps the fastest; t
 tissues fit on chip, whether sets of them run all steps in one launch instead.  Every
 combination gives the same bits.
 
-``tune_tissue``: for one tissue, times every way of taking its Euler steps -- the tiled step
-kernel (32 x 64-cell tiles), the strip kernel (128-column strips walked row by row), the
+``tune_tissue``: for one tissue, times every way of taking its Euler steps -- the default (the
+resident kernel where the tissue fits on chip, else the tiled step kernel), the strip kernel (128-column strips walked row by row), the
 temporally blocked kernel at depth k in {2, 4, 8} (k steps per launch), and the dataflow
 schedule -- on the tissue's own grid, and keeps the fastest.  All of them produce the same bits,
 so the choice changes only the speed (``Tissue.advance(..., schedule="auto")``).
@@ -28,9 +28,8 @@ from .batch import TissueBatch
 _CACHE: dict = {}
 _TISSUE_CACHE: dict = {}
 
-# (schedule, depth, step kernel) candidates of tune_tissue; step kernel 0 = tiled, 1 = strip
-# (schedule, depth, third): the step kernel (0 tiled, 1 strip) for "step" and "flow", the work
-# item rows for "batch" (the batched kernel on the one tissue)
+# candidates of tune_tissue, (schedule, depth, third): the step kernel for "step" and "flow" (0 the
+# default, resident or tiled; 1 strip), the work item rows for "batch" (the batched kernel on the one tissue)
 TISSUE_CANDIDATES = (("step", 1, 0), ("step", 1, 1), ("step", 2, 0), ("step", 4, 0),
                      ("step", 8, 0), ("flow", 1, 0), ("batch", 1, 16), ("batch", 1, 32))
 

@@ -757,16 +757,16 @@ struct LineRun {
 
 // The arguments stay in the constant bank, for many experiments those of the first one and the distance to
 // the others.  With programmatic dependent launch the state and D, which no reverse step writes, are fetched
-// before the step before has ended.  (us per step with the arguments copied from memory and all loads after
-// the step before: 28.4 for 16 experiments of 256^2, 7.1 for 151 x 203, against 24.2 and 5.0.  Blocks that
-// walk over tiles, the next one's loads in flight: 28.1; their shares are fixed, some take four tiles where
-// 3.4 are the mean.)
+// before the step before has ended.  (Measured with the regrouped operators, us per step: arguments copied from
+// memory and all loads after the step before 28.4 for 16 experiments of 256^2, 7.1 for 151 x 203, against 24.2 and
+// 5.0; blocks that walk over tiles, the next one's loads in flight, 28.1: their shares are fixed, some take four
+// tiles where 3.4 are the mean; three blocks per SM, at 80 registers, spill: 24.0, but 512^2 9.5 against 7.4.)
 //
 // SHARE: threads that share a unit.  What a thread does once per tile (places, addresses, loads, sums) costs
 // it as much as two cells, so many tiles take two threads per unit (tiles of 16 x 64 cells); where all tiles
 // run at once the chain of a thread counts, and four take it (16 x 32).  us per step with 2 | 4: 151 x 203
-// 6.0 | 5.0, 16 of 64^2 6.8 | 6.0, 512^2 (512 tiles of 16 x 32 on 304 places) 7.4 | 9.4, 16 of 256^2
-// 24.2 | 30.3.  (Three blocks per SM, at 80 registers, spill: 512^2 9.5, 16 of 256^2 24.0.)
+// 6.3 | 5.0, 16 of 64^2 6.9 | 5.2, 4 of 100 x 400 7.9 | 9.0, 512^2 (512 tiles of 16 x 32 on 304 places) 7.9 | 9.7,
+// 16 of 256^2 24.8 | 29.0.
 template <int SHARE>
 __global__ void __launch_bounds__(LNT, 2)
     fk_adjoint_line_kernel(const __grid_constant__ AdjointArgs a, const __grid_constant__ LineRun b) {

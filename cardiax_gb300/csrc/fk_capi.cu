@@ -437,10 +437,11 @@ int flow_run(const fk_grid &g, const float *src, float *dst, float *scratch, con
 }
 
 // ---- resident stepping --------------------------------------------------------------------------
-// Calls of fewer steps take one launch per step.  The resident kernel's fixed cost (clearing the
-// strips, loading the state, the cooperative launch) is 12 us at 64^2 and 26 at 1200^2, against
-// 4.4 and 9.7 us per single-step launch: at 6 steps 24.1 against 35.4 us (64^2), 28.0 against 33.1
-// (512^2), 64.9 against 82.2 (1200^2).
+// Calls of fewer steps take one launch per step.  The resident kernel's fixed cost on the device (clearing
+// the strips, loading the state, the cooperative launch) is 12 us at 64^2 and 26 at 1200^2, against 4.4 and
+// 9.7 us per single-step launch; the host searches the plan, up to some 20 us, in every call.  us of a whole
+// call of 6 steps that is waited for, launch by launch | resident: 64^2 53 | 36, 256^2 51 | 48, 512^2 52 | 53,
+// 1200^2 98 | 77 (20 steps: 123 | 58, 114 | 74, 115 | 85, 230 | 159).
 constexpr int64_t kResidentMinSteps = 6;
 
 // The plan's part of a launch's arguments.

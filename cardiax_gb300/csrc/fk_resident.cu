@@ -8,8 +8,8 @@
 // updates its cells; then the cells within 4 of a tile side go to the neighbour through global
 // memory.  Only u is exchanged, only with the 4 direct neighbours: no stencil is diagonal.
 //
-// What bounds it (us per step, GB300; one launch per step before): 256^2 1.88 (4.4), 512^2 2.36
-// (4.5), 1024^2 5.08 (8.2), 1200^2 5.98 (9.7).  One launch per step pays launch, load and store
+// What bounds it (us per step, GB300; one launch per step before): 256^2 1.84 (4.4), 512^2 2.36
+// (4.5), 1024^2 5.08 (8.2), 1200^2 5.97 (9.7).  One launch per step pays launch, load and store
 // latencies in a row whatever it computes.  Here a small grid's step is one dependent chain: about
 // 1000 cycles for a unit of 8 cells (1600 at the grid's edge), 1700 from a strip's store to its
 // neighbour's load of it through L2, and two barriers.  A large grid's step is bound by issue
@@ -18,7 +18,7 @@
 //
 // Rows per thread: more rows share u rows and u_x, and hold more cells (512 threads of 4 R cells
 // on each SM: 152 SMs hold 1247^2 cells at R = 5), but lengthen the chain: a 256^2 step takes
-// 2.1 / 2.7 / 3.6 / 4.3 us at R = 2 / 3 / 4 / 5, so resident_plan takes the fewest that fit.
+// 1.8 / 2.5 / 3.4 / 4.3 us at R = 2 / 3 / 4 / 5, so resident_plan takes the fewest that fit.
 //
 // The exchange.  A word of a strip is 8 bytes, (float, step tag), stored and loaded as one 64-bit
 // access, so a reader that sees the tag of the step it waits for has the value as well: no flag,
@@ -28,7 +28,7 @@
 //
 // A tissue of few cells per SM on 16 SMs runs as one cluster instead: the strips are stored straight into the
 // neighbours' u tiles (distributed shared memory) and the cluster's barrier takes the place of the tags; no
-// words in memory, no spinning, no cooperative launch.  64^2 1.88 -> 1.54 us per step, 128^2 1.87 -> 1.63.
+// words in memory, no spinning, no cooperative launch.  64^2 1.88 -> 1.57 us per step, 128^2 1.88 -> 1.62.
 //
 // Every wait on memory is bounded (1 s); a tile whose wait runs out reports it and leaves, its neighbours'
 // waits then run out as well.  The launch is cooperative, so all tiles run at the same time, and
@@ -658,14 +658,14 @@ static double step_cost(int R, int units, int items) {
 }
 
 // The same with the tiles in one cluster: the faster one up to some 140^2 cells (us per step in a cluster | in
-// blocks all over the device: 64^2 1.54 | 1.93, 128^2 1.61 | 2.02, 160^2 2.09 | 1.93, 200^2 2.30 | 2.03: 16 SMs
+// blocks all over the device: 64^2 1.57 | 1.88, 128^2 1.62 | 1.88, 160^2 2.09 | 1.88, 200^2 2.31 | 1.97: 16 SMs
 // have more units each).
 static double cluster_cost(int units, int items) { return 1.66 + 2.0e-3 * units + 7e-4 * items; }
 
 // Quads of a row of the u tile.  Of 8 lanes that load 16 bytes each, those beyond the end of a group of R rows
 // go on in the next one: with this many quads in a row in the 16-byte banks after the others' (where R and the
-// count allow it).  us per step without | with: 64^2 1.61 | 1.54, 128^2 1.75 | 1.63, 256^2 1.92 | 1.88, 1024^2
-// 5.30 | 5.08, 1200^2 6.03 | 5.98 (27 % of the wavefronts there were conflicts).
+// count allow it).  us per step without | with: 64^2 1.64 | 1.57, 128^2 1.76 | 1.62, 256^2 1.89 | 1.84, 1024^2
+// 5.30 | 5.08, 1200^2 6.03 | 5.97 (27 % of the wavefronts there were conflicts).
 static int tile_quads(int R, int max_q) {
     for (int x = max_q + 2; x < max_q + 10; ++x)
         if ((R * x - (max_q - 2)) % 8 == 0) return x;
